@@ -83,3 +83,33 @@ def test_device_hc_unsorted_pairs_take_the_host_loop(cuda):
     hperm, hoffs = hierarchical_clustering_v0_fast(rp, ci, 2000, (pi, pj, ps), 4)
     dperm, doffs = hierarchical_clustering_device(_csr(rp, ci, 2000), pairs_from_arrays(pi, pj, ps), 4)
     assert np.array_equal(dperm, hperm) and np.array_equal(doffs, hoffs)
+
+
+@pytest.mark.parametrize("sizes", [
+    [(2, 1), (3, 3), (32, 496), (33, 500), (64, 512), (64, 513), (65, 512)],       # one-warp blocks and just above
+    [(256, 8192), (256, 8193), (257, 300), (255, 1000), (2, 1), (64, 63)],         # 256-thread blocks and just above
+    [(1500, 4000), (700, 699), (64, 400), (20, 30), (2, 1)],                       # the rounds beside both
+])
+@pytest.mark.parametrize("cs", [2, 8, 40])
+def test_device_hc_component_sizes(cuda, sizes, cs):
+    """Connected components of given (rows, pairs) at the limits between the
+    block forms and the rounds, over rows in random order, with tied scores."""
+    from sparseops_b200.spgemm import hierarchical_clustering_device, hierarchical_clustering_v0_fast, pairs_from_arrays
+    rng = np.random.default_rng(sum(r + p for r, p in sizes) + cs)
+    n = sum(r for r, _ in sizes) + 37  # some rows in no pair
+    rows = rng.permutation(n)
+    key, at = [], 0
+    for r, p in sizes:
+        mine, at = rows[at:at + r], at + r
+        have = {(min(a, b), max(a, b)) for a, b in zip(mine[:-1], mine[1:])}  # a path connects them
+        while len(have) < p:
+            a, b = rng.choice(mine, 2, replace=False)
+            have.add((min(a, b), max(a, b)))
+        key += [int(a) * n + int(b) for a, b in have]
+    key = np.sort(np.array(key, np.int64))
+    pi, pj = key // n, key % n
+    ps = rng.integers(0, 17, len(key)) / 16.0
+    rp, ci, _ = synth.planted_communities(n, ncomm=max(1, n // 40), mean=6.0, seed=n)
+    hperm, hoffs = hierarchical_clustering_v0_fast(rp, ci, n, (pi, pj, ps), cs)
+    dperm, doffs = hierarchical_clustering_device(_csr(rp, ci, n), pairs_from_arrays(pi, pj, ps), cs)
+    assert np.array_equal(dperm, hperm) and np.array_equal(doffs, hoffs)
