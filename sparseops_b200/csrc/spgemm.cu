@@ -44,6 +44,7 @@
 #include <vector>
 
 #include "spops_internal.h"
+#include "spgemm_rows.cuh"
 #include "spgemm_sort.cuh"
 
 namespace spops {
@@ -761,15 +762,18 @@ __global__ void classify_kernel(const int64_t* __restrict__ cptr, const int64_t*
   drop[c] = (dense || sort_output) ? 1 : 0;
 }
 
+constexpr unsigned char kRowSettled = 2;  // settled[c] of the one-row clusters of row_sort_kernel
+
 // ------------------------------------------------------------ to CSR
 template <typename V>
 __global__ void row_count_kernel(const int64_t* __restrict__ soff_val, const int64_t* __restrict__ nz,
                                  const int64_t* __restrict__ offsets, const int64_t* __restrict__ perm, int64_t ncl,
-                                 const V* __restrict__ cval, bool keep_zeros, int64_t* __restrict__ rowcnt) {
+                                 const V* __restrict__ cval, bool keep_zeros,
+                                 const unsigned char* __restrict__ settled, int64_t* __restrict__ rowcnt) {
   // warp per cluster, lanes over its rows (csz <= 32 common) and columns
   const int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (c >= ncl) return;
+  if (c >= ncl || settled[c] == kRowSettled) return;  // its kernel counted the row
   const int64_t csz = offsets[c + 1] - offsets[c];
   const int64_t ncol = nz[c];
   for (int64_t l = 0; l < csz; ++l) {
@@ -814,7 +818,8 @@ __global__ void row_write_kernel(const int64_t* __restrict__ soff, const int64_t
 // cluster) so each bin lists its clusters in ascending order, and the bin
 // boundaries found by binary search in the sorted keys.  Only the
 // boundaries come back to the host.
-constexpr uint32_t kNoBin = 15;
+constexpr uint32_t kNoBin = 31;
+constexpr int kBinBits = 5;
 
 __device__ __forceinline__ int64_t pow2_ceil(int64_t v) {
   return v <= 1 ? 1 : (int64_t)1 << (64 - __clzll((unsigned long long)(v - 1)));
@@ -887,32 +892,50 @@ __global__ void num_bin_kernel(const int64_t* __restrict__ nz, const int64_t* __
   key[c] = bytes <= lim.wbytes[5] ? 5 : (bytes <= lim.wbytes[6] ? 6 : 7);
 }
 
-// sort path (spgemm_sort.cuh): bin q (R = 2^q keys per lane, q = 0..6)
-// for a cluster with at most 32 * 2^q products and kSortCols columns whose
-// output columns fit the key beside the product index; settled[c] = 1 then.
-// bins 0-4: one warp, 2^q keys per lane (sort_accum_kernel); bins 5-8: 2^(q-4)
-// warps of 16 keys per lane (sort_accum_multi_kernel); bin q holds P <= 32 << q
+// sort path: bin q holds the clusters with at most 32 << q products whose
+// output columns fit a 32-bit key beside the product index.  settled[c]:
+//   1            sort_accum kernels (spgemm_sort.cuh), at most kSortCols
+//                (kMultiCols) columns: bins 0-4 one warp, 2^q keys per lane;
+//                bins 5-8 2^(q-4) warps of 16 keys per lane
+//   kRowSettled  row_sort_kernel (spgemm_rows.cuh), clusters of one row with
+//                more than 32 << (kRowBin0 - 1) products: bin kSortBins + q -
+//                kRowBin0.  Smaller rows fit a few keys per lane, where four
+//                rows share a block of the one-warp kernel.
 constexpr int kSortBins = 9;
 constexpr int kSortOneWarpBins = 5;
+constexpr int kRowBin0 = 2;
+constexpr int kRowBins = kSortBins - kRowBin0;
+constexpr int kAllBins = kSortBins + kRowBins;
 
-__global__ void sort_bin_kernel(const int64_t* __restrict__ flops, const int64_t* __restrict__ cptr, int64_t ncl,
-                                int64_t bcols, unsigned char* __restrict__ settled, uint32_t* __restrict__ key,
+__global__ void sort_bin_kernel(const int64_t* __restrict__ flops, const int64_t* __restrict__ cptr,
+                                const int64_t* __restrict__ offsets, int64_t ncl, int64_t bcols,
+                                unsigned char* __restrict__ settled, uint32_t* __restrict__ key,
                                 int64_t* __restrict__ ids) {
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= ncl) return;
   ids[c] = c;
   const int64_t P = flops[c], nj = cptr[c + 1] - cptr[c];
   uint32_t b = kNoBin;
+  unsigned char how = 0;
   for (int q = 0; q < kSortBins; ++q) {
     if (P <= (32LL << q)) {
       const int tbits = 5 + q;
-      const int64_t max_cols = q < kSortOneWarpBins ? kSortCols : kMultiCols;
-      if (nj <= max_cols && bcols <= (1LL << (32 - tbits)) - 1) b = (uint32_t)q;
+      // a key of all ones marks an empty slot: the last column and the last
+      // product index may not both occur
+      const int64_t room = 1LL << (32 - tbits);
+      const bool fits = bcols < room || (bcols == room && P < (32LL << q));
+      if (fits && q >= kRowBin0 && offsets[c + 1] - offsets[c] == 1) {
+        b = (uint32_t)(kSortBins + q - kRowBin0);
+        how = kRowSettled;
+      } else if (fits && nj <= (q < kSortOneWarpBins ? kSortCols : kMultiCols)) {
+        b = (uint32_t)q;
+        how = 1;
+      }
       break;
     }
   }
   key[c] = b;
-  settled[c] = b != kNoBin ? 1 : 0;
+  settled[c] = how;
 }
 
 // room in each cluster's output slab: its product count on the sort path (at
@@ -1309,10 +1332,10 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
     if (ncl == 0) return SPOPS_OK;
     size_t cb2 = 0;
     SPOPS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, cb2, bkey.as<uint32_t>(), bkey_s.as<uint32_t>(),
-                                               bid.as<int64_t>(), bid_s.as<int64_t>(), ncl, 0, 4, st));
+                                               bid.as<int64_t>(), bid_s.as<int64_t>(), ncl, 0, kBinBits, st));
     SPOPS_TRY(tmp.alloc(cb2 + 256));
     SPOPS_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, cb2, bkey.as<uint32_t>(), bkey_s.as<uint32_t>(),
-                                               bid.as<int64_t>(), bid_s.as<int64_t>(), ncl, 0, 4, st));
+                                               bid.as<int64_t>(), bid_s.as<int64_t>(), ncl, 0, kBinBits, st));
     bin_bounds_kernel<<<1, 32, 0, st>>>(bkey_s.as<uint32_t>(), ncl, nb, bstart.as<int64_t>());
     SPOPS_LAUNCH_CHECK();
     SPOPS_CUDA(cudaMemcpyAsync(start.data(), bstart.p, ((size_t)nb + 1) * 8, cudaMemcpyDeviceToHost, st));
@@ -1336,21 +1359,21 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
   };
   tr.mark(st, "flops per cluster");
 
-  // --- sort path: which clusters the one-warp sort-accumulate kernels take
-  // (their list kept apart: the bin buffers are reused below)
+  // --- sort path: which clusters the sort-accumulate kernels take (their list
+  // kept apart: the bin buffers are reused below)
   const int64_t bcols = B->cols;
   PoolBuf settled(ctx), slist(ctx);
   SPOPS_TRY(settled.alloc(ncl1));
   SPOPS_CUDA(cudaMemsetAsync(settled.p, 0, ncl1, st));
-  std::vector<int64_t> tstart((size_t)kSortBins + 1, 0);
+  std::vector<int64_t> tstart((size_t)kAllBins + 1, 0);
   if (ncl > 0) {
-    sort_bin_kernel<<<grid_for(ncl), 256, 0, st>>>(flops.as<int64_t>(), cptr.as<int64_t>(), ncl, bcols,
-                                                  settled.as<unsigned char>(), bkey.as<uint32_t>(),
+    sort_bin_kernel<<<grid_for(ncl), 256, 0, st>>>(flops.as<int64_t>(), cptr.as<int64_t>(), offs.as<int64_t>(), ncl,
+                                                  bcols, settled.as<unsigned char>(), bkey.as<uint32_t>(),
                                                   bid.as<int64_t>());
     SPOPS_LAUNCH_CHECK();
-    SPOPS_TRY(sort_bins(kSortBins, tstart));
+    SPOPS_TRY(sort_bins(kAllBins, tstart));
   }
-  const int64_t nsorted = tstart[kSortBins];
+  const int64_t nsorted = tstart[kAllBins];
   SPOPS_TRY(slist.alloc((size_t)std::max<int64_t>(nsorted, 1) * 8));
   if (nsorted > 0)
     SPOPS_CUDA(cudaMemcpyAsync(slist.p, bid_s.p, (size_t)nsorted * 8, cudaMemcpyDeviceToDevice, st));
@@ -1481,6 +1504,36 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
 #undef SPOPS_SORT_LAUNCH
 #undef SPOPS_MULTI_LAUNCH
     SPOPS_LAUNCH_CHECK();
+  }
+  // the same for one-row clusters, their rows counted too; largest first
+  PoolBuf rowcnt(ctx);
+  SPOPS_TRY(rowcnt.alloc((nn + 1) * 8));
+  SPOPS_CUDA(cudaMemsetAsync(rowcnt.p, 0, (nn + 1) * 8, st));
+  for (int q = kRowBins - 1; q >= 0; --q) {
+    const int64_t m = tstart[kSortBins + q + 1] - tstart[kSortBins + q];
+    if (m <= 0) continue;
+    const int64_t* dl = slist.as<int64_t>() + tstart[kSortBins + q];
+    auto launch = [&](auto kern, size_t smem, int threads) -> spops_status_t {
+      SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+      kern<<<(unsigned)m, threads, smem, st>>>(
+          dl, cptr.as<int64_t>(), cptr_val.as<int64_t>(), colids.as<int32_t>(), avals.as<V>(), offs.as<int64_t>(),
+          perm.as<int64_t>(), B->row.as<I>(), B->col.as<I>(), B->val.as<V>(), b_rowdense, l2_budget, sort_output,
+          rowwise, soff.as<int64_t>(), soff_val.as<int64_t>(), nzd.as<int64_t>(), cmin.as<int64_t>(),
+          cmax.as<int64_t>(), drop.as<unsigned char>(), reinterpret_cast<unsigned long long*>(ndense.p),
+          ccol.as<int32_t>(), cval.as<V>(), rowcnt.as<int64_t>());
+      SPOPS_LAUNCH_CHECK();
+      return SPOPS_OK;
+    };
+    switch (q) {
+      case 0: SPOPS_TRY(launch(row_sort_kernel<I, V, 4, 1>, sizeof(RowSmem<V, 4, 1>), 32)); break;
+      case 1: SPOPS_TRY(launch(row_sort_kernel<I, V, 8, 1>, sizeof(RowSmem<V, 8, 1>), 32)); break;
+      case 2: SPOPS_TRY(launch(row_sort_kernel<I, V, 16, 1>, sizeof(RowSmem<V, 16, 1>), 32)); break;
+      case 3: SPOPS_TRY(launch(row_sort_kernel<I, V, 16, 2>, sizeof(RowSmem<V, 16, 2>), 64)); break;
+      case 4: SPOPS_TRY(launch(row_sort_kernel<I, V, 16, 4>, sizeof(RowSmem<V, 16, 4>), 128)); break;
+      case 5: SPOPS_TRY(launch(row_sort_kernel<I, V, 16, 8>, sizeof(RowSmem<V, 16, 8>), 256)); break;
+      default: SPOPS_TRY(launch(row_sort_kernel<I, V, 16, 16>, sizeof(RowSmem<V, 16, 16>), 512)); break;
+    }
   }
   tr.mark(st, "sort-path kernels");
 
@@ -1633,14 +1686,13 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
   }
 
   // --- back to CSR, original row order
-  PoolBuf rowcnt(ctx), crp(ctx);
-  SPOPS_TRY(rowcnt.alloc((nn + 1) * 8));
+  PoolBuf crp(ctx);
   SPOPS_TRY(crp.alloc((nn + 1) * 8));
-  SPOPS_CUDA(cudaMemsetAsync(rowcnt.p, 0, (nn + 1) * 8, st));
   if (ncl > 0) {
     row_count_kernel<V><<<grid_for(ncl * 32), 256, 0, st>>>(soff_val.as<int64_t>(), nzd.as<int64_t>(),
                                                             offs.as<int64_t>(), perm.as<int64_t>(), ncl, cval.as<V>(),
-                                                            rowwise, rowcnt.as<int64_t>());
+                                                            rowwise, settled.as<unsigned char>(),
+                                                            rowcnt.as<int64_t>());
     SPOPS_LAUNCH_CHECK();
   }
   SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, cb, rowcnt.as<int64_t>(), crp.as<int64_t>(), (int64_t)(n + 1), st));

@@ -26,7 +26,9 @@
 //
 // Limits (the caller bins clusters accordingly): P <= 32*R (R <= 16), the cluster has
 // at most kSortCols columns, and B's column count fits the key
-// (cols <= 2^(32 - tbits) - 1, tbits = log2(32*R)).
+// (cols < 2^(32 - tbits), tbits = log2(32*R), or equal with P < 32*R).
+// One-row clusters of more than 64 products take row_sort_kernel
+// (spgemm_rows.cuh) instead.
 #pragma once
 
 #include <cstdint>

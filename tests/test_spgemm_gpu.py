@@ -404,3 +404,56 @@ def test_vlength_refusals(cuda):
     fake._h, fake._codes = A.device(), Acl._codes
     with pytest.raises(SpOpsError):
         LeSpGEMM_VLength(fake, _csr(brp, bci, bv, m))
+
+
+@pytest.mark.parametrize("itype,vtype,sorted_b", [(np.int64, np.float64, True), (np.int32, np.float64, False),
+                                                  (np.int64, np.float32, True)])
+def test_rowwise_product_count_edges(cuda, itype, vtype, sorted_b):
+    """Rows of C with product counts at the limits between the kernel forms,
+    made of many one-entry and longer rows of B, their columns at both ends of
+    2^19 columns (where the largest key is one product short of full) and
+    often repeated; B's rows ascending, or in any order with repeats."""
+    from sparseops_b200.spgemm import LeSpGEMM
+    rng = np.random.default_rng(77)
+    ncols, ones, longer = 1 << 19, 1700, 500
+    hot = np.concatenate([np.arange(64), np.arange(ncols - 64, ncols)])
+    rows = []
+    for r in range(ones + longer):
+        m = 1 if r < ones else int(rng.integers(2, 41))
+        c = np.concatenate([rng.choice(hot, (m + 1) // 2, replace=not sorted_b), rng.integers(64, ncols - 64, m // 2)])
+        rows.append(np.unique(c) if sorted_b else c)
+    lens = np.array([len(r) for r in rows])
+    brp = np.concatenate([[0], np.cumsum(lens)])
+    bci, bv = np.concatenate(rows), rng.standard_normal(brp[-1])
+    counts = [64, 65, 128, 129, 256, 257, 512, 513, 1024, 1025, 1600, 2048, 2049, 4096, 4097, 8191, 8192, 8193]
+    acols = []
+    for i, P in enumerate(counts):
+        pick = [] if P == 1600 else list(rng.permutation(np.arange(ones, ones + longer)))
+        take, left = [], P
+        while pick and left > 60:
+            r = pick.pop()
+            if lens[r] <= left:
+                take.append(r)
+                left -= lens[r]
+        take += list(rng.choice(ones, left, replace=False)) if left <= ones else []
+        assert lens[take].sum() == P
+        acols.append(np.sort(np.array(take)))
+    arp = np.concatenate([[0], np.cumsum([len(c) for c in acols])])
+    aci, av = np.concatenate(acols), rng.standard_normal(arp[-1])
+    av, bv = av.astype(vtype), bv.astype(vtype)
+    C = LeSpGEMM(_csr(arp.astype(itype), aci.astype(itype), av, len(rows)),
+                 _csr(brp.astype(itype), bci.astype(itype), bv, ncols))
+    rp, ci, v = C.host()
+    tol = 1e-12 if vtype == np.float64 else 1e-5
+    for i in range(len(counts)):
+        val, mag = {}, {}
+        for k in range(arp[i], arp[i + 1]):
+            for e in range(brp[aci[k]], brp[aci[k] + 1]):
+                x = float(av[k]) * float(bv[e])
+                val[bci[e]] = val.get(bci[e], 0.0) + x
+                mag[bci[e]] = mag.get(bci[e], 0.0) + abs(x)
+        want = sorted(val)
+        assert np.array_equal(ci[rp[i]:rp[i + 1]], want), counts[i]
+        got = v[rp[i]:rp[i + 1]].astype(np.float64)
+        err = np.abs(got - [val[c] for c in want]) / np.array([mag[c] for c in want])
+        assert err.max() <= tol, counts[i]
