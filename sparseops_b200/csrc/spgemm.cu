@@ -8,11 +8,12 @@
 // vlength_cluster2csr (1777) and the inverse reorder.
 //
 // Pipeline (rows of A grouped by the clustering's permutation / offsets):
-//   1. clusters   entries of the reordered rows keyed by (cluster, column),
-//                 one stable radix sort, unique keys -> each cluster's column
-//                 list ASCENDING, values [columns x csz] column-major by row
-//                 in the cluster (the reference's CSR_VlengthCluster layout;
-//                 it orders a cluster's columns by hash-map iteration instead).
+//   1. clusters   each cluster's column list ASCENDING, values [columns x
+//                 csz] column-major by row in the cluster (the reference's
+//                 CSR_VlengthCluster layout; it orders a cluster's columns by
+//                 hash-map iteration instead): one-row clusters copied, small
+//                 ones sorted by a warp, the rest by one radix sort of
+//                 (cluster, column) keys (build_clusters).
 //   2. flops      per cluster sum of nnz(B row) over its columns; clusters
 //                 binned by the size of their accumulator.
 //   3. symbolic   per cluster (one thread block) a hash set of B columns in
@@ -55,12 +56,6 @@ inline unsigned grid_for(int64_t work, int threads = 256) {
   return (unsigned)(g < 1 ? 1 : g);
 }
 
-inline int64_t pow2_at_least(int64_t v) {
-  int64_t p = 1;
-  while (p < v) p <<= 1;
-  return p;
-}
-
 __device__ __forceinline__ uint32_t hslot(int32_t key, uint32_t mask) {
   return ((uint32_t)key * 2654435761u) & mask;
 }
@@ -94,29 +89,253 @@ inline int key_bits(int64_t m) {
   return b;
 }
 
-template <typename I, typename V>
-__global__ void cluster_keys_kernel(const I* __restrict__ rp, const I* __restrict__ ci, const int64_t* __restrict__ perm,
-                                    const int64_t* __restrict__ row_cluster, int64_t n, const int64_t* __restrict__ rpr,
-                                    int shift, uint64_t* __restrict__ keys, int64_t* __restrict__ src) {
-  // warp per reordered row: entries of original row perm[r] in order; key =
-  // cluster << shift | column (shift: the bits of A's column count)
-  const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+// Clusters by what building their column list takes.
+//   kClOne   one row, columns strictly increasing: the row as it is
+//   kClSort  at most 32 rows and 512 entries whose (column, entry) pairs fit a
+//            32-bit key: one warp sorts them in registers, twice (to count the
+//            distinct columns, then, the output places known, to write them)
+//   kClWide  the rest: one global radix sort of (cluster, column) keys
+// The global sort over all entries took 1.1 ms for 10M entries in 516,012
+// clusters (98 % of one row), bound by its passes over 16-byte records.
+constexpr unsigned char kClOne = 0, kClSort = 1, kClWide = 2;
+constexpr int kClRows = 32, kClR = 16;
+
+// A cluster's rows in the warp's lanes (csz <= 32): start of each row's
+// entries and the entries before it
+struct ClRows {
+  int64_t start;
+  int32_t off, total;
+};
+
+template <typename I>
+__device__ __forceinline__ ClRows cl_rows(const I* __restrict__ rp, const int64_t* __restrict__ perm, int64_t r0,
+                                          int csz, int lane) {
+  int64_t st = 0;
+  int32_t len = 0;
+  if (lane < csz) {
+    const int64_t r = perm[r0 + lane];
+    st = rp[r];
+    len = (int32_t)((int64_t)rp[r + 1] - st);
+  }
+  int32_t inc = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  return ClRows{st, inc - len, __shfl_sync(0xffffffffu, inc, 31)};
+}
+
+// the row (lane) holding entry t of the cluster; all lanes call
+__device__ __forceinline__ int cl_find(const ClRows& w, int csz, int t) {
+  int lo = 0;
+#pragma unroll
+  for (int step = 16; step > 0; step >>= 1) {
+    const int cand = lo + step;
+    const int32_t oc = __shfl_sync(0xffffffffu, w.off, cand & 31);
+    if (cand < csz && oc <= t) lo = cand;
+  }
+  return lo;
+}
+
+// Sorted keys (column << tbits | entry), blocked, and which of this lane's
+// start a column; returns their count before this lane (total: over all).
+template <int R, typename I>
+__device__ __forceinline__ int cl_sort(const ClRows& w, int csz, const I* __restrict__ ci, int lane, uint32_t (&key)[R],
+                                       uint32_t* first, int* total) {
+  constexpr int tbits = 5 + (R > 1) + (R > 2) + (R > 4) + (R > 8);
+#pragma unroll
+  for (int s = 0; s < R; ++s) {
+    const int t = s * 32 + lane;
+    const int l = cl_find(w, csz, t);
+    const int64_t st = __shfl_sync(0xffffffffu, w.start, l);
+    const int32_t of = __shfl_sync(0xffffffffu, w.off, l);
+    key[s] = t < w.total ? (uint32_t)ci[st + (t - of)] << tbits | (uint32_t)t : ~0u;
+  }
+  warp_bitonic_sort<R>(key, lane);
+  uint32_t before = __shfl_up_sync(0xffffffffu, key[R - 1], 1);
+  uint32_t f = 0;
+#pragma unroll
+  for (int s = 0; s < R; ++s) {
+    const uint32_t prev = s ? key[s - 1] : before;
+    if (lane * R + s < w.total && ((lane == 0 && s == 0) || prev >> tbits != key[s] >> tbits)) f |= 1u << s;
+  }
+  int inc = __popc(f);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  *first = f;
+  *total = __shfl_sync(0xffffffffu, inc, 31);
+  return inc - __popc(f);
+}
+
+template <int R, typename I>
+__device__ __forceinline__ int cl_count(const ClRows& w, int csz, const I* __restrict__ ci, int lane) {
+  uint32_t key[R], first;
+  int total;
+  cl_sort<R, I>(w, csz, ci, lane, key, &first, &total);
+  return total;
+}
+
+// Eight lanes per cluster: its kind, the column counts of kClOne clusters,
+// the list of kClSort clusters; count[0] += the entries of wide clusters,
+// count[1] = listed clusters.  (One warp per cluster, or this beside the
+// register sorts in one kernel, leaves half the lanes or the warps idle on
+// rows of 20 entries: 268 us against 60 us for the planted matrix.)
+constexpr int kClLanes = 8;
+
+template <typename I>
+__global__ void cluster_kind_kernel(const I* __restrict__ rp, const I* __restrict__ ci, int64_t acols,
+                                    const int64_t* __restrict__ perm, const int64_t* __restrict__ offsets,
+                                    int64_t ncl, unsigned char* __restrict__ kind, int64_t* __restrict__ ncols,
+                                    int64_t* __restrict__ list, unsigned long long* __restrict__ count) {
+  const int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kClLanes;
+  const int lane = threadIdx.x & 31, sub = lane & (kClLanes - 1);
+  const unsigned group = ((1u << kClLanes) - 1u) << (lane - sub);
+  if (c >= ncl) return;
+  const int64_t r0 = offsets[c], csz = offsets[c + 1] - r0;
+  int64_t entries = 0;
+  bool ascend = csz == 1;
+  if (csz == 1) {
+    const int64_t r = perm[r0], s = rp[r], e = rp[r + 1];
+    entries = e - s;
+    for (int64_t k = s + 1 + sub; k < e; k += kClLanes) ascend &= ci[k - 1] < ci[k];
+  } else {
+    for (int64_t l = sub; l < csz; l += kClLanes) {
+      const int64_t r = perm[r0 + l];
+      entries += (int64_t)rp[r + 1] - (int64_t)rp[r];
+    }
+#pragma unroll
+    for (int o = kClLanes / 2; o > 0; o >>= 1) entries += __shfl_xor_sync(group, entries, o);
+  }
+  ascend = __all_sync(group, ascend);
+  if (sub) return;
+  unsigned char how = kClWide;
+  if (ascend) {
+    how = kClOne;
+  } else if (csz <= kClRows && entries <= 32 * kClR) {
+    int q = 0;
+    while ((32 << q) < entries) ++q;
+    if (acols < (1LL << (27 - q))) how = kClSort;
+  }
+  kind[c] = how;
+  ncols[c] = how == kClOne ? entries : 0;
+  if (how == kClSort) list[atomicAdd(count + 1, 1ULL)] = c;
+  if (how == kClWide) atomicAdd(count, (unsigned long long)entries);
+}
+
+// One warp per listed (kClSort) cluster: its distinct columns.
+template <typename I>
+__global__ void cluster_count_kernel(const int64_t* __restrict__ list, int64_t m, const I* __restrict__ rp,
+                                     const I* __restrict__ ci, const int64_t* __restrict__ perm,
+                                     const int64_t* __restrict__ offsets, int64_t* __restrict__ ncols) {
+  const int64_t b = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (r >= n) return;
-  const int64_t orow = perm[r];
-  const int64_t s = rp[orow], e = rp[orow + 1], o = rpr[r];
-  const uint64_t c = (uint64_t)row_cluster[r];
-  for (int64_t k = lane; k < e - s; k += 32) {
-    keys[o + k] = (c << shift) | (uint64_t)(uint32_t)ci[s + k];
-    src[o + k] = s + k;  // entry of A
+  if (b >= m) return;
+  const int64_t c = list[b], r0 = offsets[c];
+  const int csz = (int)(offsets[c + 1] - r0);
+  const ClRows w = cl_rows(rp, perm, r0, csz, lane);
+  int n;
+  if (w.total <= 32) n = cl_count<1, I>(w, csz, ci, lane);
+  else if (w.total <= 64) n = cl_count<2, I>(w, csz, ci, lane);
+  else if (w.total <= 128) n = cl_count<4, I>(w, csz, ci, lane);
+  else if (w.total <= 256) n = cl_count<8, I>(w, csz, ci, lane);
+  else n = cl_count<16, I>(w, csz, ci, lane);
+  if (lane == 0) ncols[c] = n;
+}
+
+template <int R, typename I, typename V>
+__device__ __forceinline__ void cl_fill(const ClRows& w, int csz, const I* __restrict__ ci, const V* __restrict__ av,
+                                        int lane, int64_t cp, int64_t cpv, int32_t* __restrict__ colids,
+                                        V* __restrict__ cvals) {
+  constexpr int tbits = 5 + (R > 1) + (R > 2) + (R > 4) + (R > 8);
+  uint32_t key[R], first;
+  int total;
+  int u = cl_sort<R, I>(w, csz, ci, lane, key, &first, &total) - 1;
+#pragma unroll
+  for (int s = 0; s < R; ++s) {
+    const bool in = lane * R + s < w.total;
+    const int t = in ? (int)(key[s] & ((1u << tbits) - 1u)) : 0;
+    const int l = cl_find(w, csz, t);
+    const int64_t st = __shfl_sync(0xffffffffu, w.start, l);
+    const int32_t of = __shfl_sync(0xffffffffu, w.off, l);
+    if (in) {
+      if (first >> s & 1u) {
+        ++u;
+        colids[cp + u] = (int32_t)(key[s] >> tbits);
+      }
+      cvals[cpv + (int64_t)u * csz + l] = av[st + (t - of)];
+    }
   }
 }
 
+// Eight lanes per cluster: columns and values of the kClOne clusters.
+template <typename I, typename V>
+__global__ void cluster_copy_kernel(const I* __restrict__ rp, const I* __restrict__ ci, const V* __restrict__ av,
+                                    const int64_t* __restrict__ perm, const int64_t* __restrict__ offsets, int64_t ncl,
+                                    const unsigned char* __restrict__ kind, const int64_t* __restrict__ cptr,
+                                    const int64_t* __restrict__ cptr_val, int32_t* __restrict__ colids,
+                                    V* __restrict__ cvals) {
+  const int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kClLanes;
+  if (c >= ncl || kind[c] != kClOne) return;
+  const int64_t s = rp[perm[offsets[c]]], cp = cptr[c], cpv = cptr_val[c], n = cptr[c + 1] - cp;
+  for (int64_t k = threadIdx.x & (kClLanes - 1); k < n; k += kClLanes) {
+    colids[cp + k] = (int32_t)ci[s + k];
+    cvals[cpv + k] = av[s + k];
+  }
+}
+
+// One warp per listed (kClSort) cluster: columns and values (which start out
+// zero).
+template <typename I, typename V>
+__global__ void cluster_fill_kernel(const int64_t* __restrict__ list, int64_t m, const I* __restrict__ rp,
+                                    const I* __restrict__ ci, const V* __restrict__ av,
+                                    const int64_t* __restrict__ perm, const int64_t* __restrict__ offsets,
+                                    const int64_t* __restrict__ cptr, const int64_t* __restrict__ cptr_val,
+                                    int32_t* __restrict__ colids, V* __restrict__ cvals) {
+  const int64_t b = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (b >= m) return;
+  const int64_t c = list[b], r0 = offsets[c], cp = cptr[c], cpv = cptr_val[c];
+  const int csz = (int)(offsets[c + 1] - r0);
+  const ClRows w = cl_rows(rp, perm, r0, csz, lane);
+  if (w.total <= 32) cl_fill<1, I, V>(w, csz, ci, av, lane, cp, cpv, colids, cvals);
+  else if (w.total <= 64) cl_fill<2, I, V>(w, csz, ci, av, lane, cp, cpv, colids, cvals);
+  else if (w.total <= 128) cl_fill<4, I, V>(w, csz, ci, av, lane, cp, cpv, colids, cvals);
+  else if (w.total <= 256) cl_fill<8, I, V>(w, csz, ci, av, lane, cp, cpv, colids, cvals);
+  else cl_fill<16, I, V>(w, csz, ci, av, lane, cp, cpv, colids, cvals);
+}
+
+// ---- wide clusters: (cluster, column) keys, one radix sort
 template <typename I>
-__global__ void reordered_len_kernel(const I* __restrict__ rp, const int64_t* __restrict__ perm, int64_t n,
-                                     int64_t* __restrict__ len) {
+__global__ void wide_len_kernel(const I* __restrict__ rp, const int64_t* __restrict__ perm,
+                                const int64_t* __restrict__ row_cluster, const unsigned char* __restrict__ kind,
+                                int64_t n, int64_t* __restrict__ len) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r < n) len[r] = (int64_t)rp[perm[r] + 1] - (int64_t)rp[perm[r]];
+  if (r < n) len[r] = kind[row_cluster[r]] == kClWide ? (int64_t)rp[perm[r] + 1] - (int64_t)rp[perm[r]] : 0;
+}
+
+// warp per reordered row: entries of original row perm[r] in order; key =
+// cluster << shift | column (shift: the bits of A's column count); payload =
+// (entry of A, row within the cluster)
+template <typename I>
+__global__ void wide_keys_kernel(const I* __restrict__ rp, const I* __restrict__ ci, const int64_t* __restrict__ perm,
+                                 const int64_t* __restrict__ row_cluster, const int64_t* __restrict__ offsets,
+                                 const unsigned char* __restrict__ kind, int64_t n, const int64_t* __restrict__ rpr,
+                                 int shift, uint64_t* __restrict__ keys, longlong2* __restrict__ src) {
+  const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (r >= n) return;
+  const int64_t c = row_cluster[r];
+  if (kind[c] != kClWide) return;
+  const int64_t orow = perm[r];
+  const int64_t s = rp[orow], e = rp[orow + 1], o = rpr[r];
+  for (int64_t k = lane; k < e - s; k += 32) {
+    keys[o + k] = ((uint64_t)c << shift) | (uint64_t)(uint32_t)ci[s + k];
+    src[o + k] = longlong2{(long long)(s + k), (long long)(r - offsets[c])};
+  }
 }
 
 __global__ void row_cluster_kernel(const int64_t* __restrict__ offsets, int64_t ncl, int64_t* __restrict__ row_cluster) {
@@ -125,47 +344,163 @@ __global__ void row_cluster_kernel(const int64_t* __restrict__ offsets, int64_t 
   for (int64_t r = offsets[c]; r < offsets[c + 1]; ++r) row_cluster[r] = c;
 }
 
-__global__ void key_flag_kernel(const uint64_t* __restrict__ keys, int64_t m, int64_t* __restrict__ flag) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < m) flag[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1 : 0;
-}
-
-// per unique key: its cluster's column count, and the column itself
-__global__ void cluster_cols_kernel(const uint64_t* __restrict__ keys, const int64_t* __restrict__ flag,
-                                    const int64_t* __restrict__ uidx, int64_t m, int shift, int32_t* __restrict__ colids,
-                                    unsigned long long* __restrict__ ncols) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= m || !flag[i]) return;
-  const int64_t u = uidx[i] - 1;
-  colids[u] = (int32_t)(keys[i] & ((1ULL << shift) - 1ULL));
-  atomicAdd(ncols + (keys[i] >> shift), 1ULL);
-}
-
-template <typename I, typename V>
-__global__ void cluster_vals_kernel(const uint64_t* __restrict__ keys, const int64_t* __restrict__ src,
-                                    const int64_t* __restrict__ uidx, int64_t m, int shift, const V* __restrict__ av,
-                                    const I* __restrict__ rp, const int64_t* __restrict__ perm,
-                                    const int64_t* __restrict__ offsets, const int64_t* __restrict__ cptr,
-                                    const int64_t* __restrict__ cptr_val, const int64_t* __restrict__ row_of_entry,
-                                    V* __restrict__ cvals) {
+// distinct keys flagged and counted per cluster
+__global__ void wide_flag_kernel(const uint64_t* __restrict__ keys, int64_t m, int shift, int64_t* __restrict__ flag,
+                                 unsigned long long* __restrict__ ncols) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= m) return;
-  const int64_t c = (int64_t)(keys[i] >> shift);
-  const int64_t u = uidx[i] - 1;
-  const int64_t l = row_of_entry[src[i]] - offsets[c];  // row within the cluster
-  const int64_t csz = offsets[c + 1] - offsets[c];
-  cvals[cptr_val[c] + (u - cptr[c]) * csz + l] = av[src[i]];
+  const bool f = i == 0 || keys[i] != keys[i - 1];
+  flag[i] = f ? 1 : 0;
+  if (f) atomicAdd(ncols + (keys[i] >> shift), 1ULL);
 }
 
-// reordered position of each entry's row: entry e of original row perm[r] -> r
-template <typename I>
-__global__ void entry_row_kernel(const I* __restrict__ rp, const int64_t* __restrict__ perm, int64_t n,
-                                 int64_t* __restrict__ row_of_entry) {
-  const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (r >= n) return;
-  const int64_t orow = perm[r];
-  for (int64_t k = (int64_t)rp[orow] + lane; k < (int64_t)rp[orow + 1]; k += 32) row_of_entry[k] = r;
+// the distinct keys before each wide cluster
+__global__ void wide_base_kernel(const uint64_t* __restrict__ keys, const int64_t* __restrict__ uidx, int64_t m,
+                                 int shift, int64_t* __restrict__ base) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < m && (i == 0 || keys[i] >> shift != keys[i - 1] >> shift)) base[keys[i] >> shift] = uidx[i] - 1;
+}
+
+template <typename V>
+__global__ void wide_fill_kernel(const uint64_t* __restrict__ keys, const longlong2* __restrict__ src,
+                                 const int64_t* __restrict__ flag, const int64_t* __restrict__ uidx,
+                                 const int64_t* __restrict__ base, int64_t m, int shift, const V* __restrict__ av,
+                                 const int64_t* __restrict__ offsets, const int64_t* __restrict__ cptr,
+                                 const int64_t* __restrict__ cptr_val, int32_t* __restrict__ colids,
+                                 V* __restrict__ cvals) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  const int64_t c = (int64_t)(keys[i] >> shift), u = uidx[i] - 1 - base[c];
+  if (flag[i]) colids[cptr[c] + u] = (int32_t)(keys[i] & ((1ULL << shift) - 1ULL));
+  const longlong2 e = src[i];
+  cvals[cptr_val[c] + u * (offsets[c + 1] - offsets[c]) + e.y] = av[e.x];
+}
+
+__global__ void weight_kernel(const int64_t* __restrict__ cnt, const int64_t* __restrict__ offsets, int64_t ncl,
+                              int64_t* __restrict__ weighted) {
+  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (c < ncl) weighted[c] = cnt[c] * (offsets[c + 1] - offsets[c]);
+}
+
+// The clustered form of A's rows perm[offsets[c]] .. (device arrays): per
+// cluster its distinct columns ascending (ncols, cptr, colids) and values
+// [columns x rows of the cluster] (cptr_val, avals); refused above max_values.
+template <typename I, typename V>
+spops_status_t build_clusters(Context* ctx, const Matrix* A, const int64_t* perm, const int64_t* offs, int64_t ncl,
+                              PoolBuf& ncols, PoolBuf& cptr, PoolBuf& cptr_val, PoolBuf& colids, PoolBuf& avals,
+                              int64_t max_values, int64_t* nnzc, int64_t* nnzv) {
+  cudaStream_t st = ctx->stream;
+  const int64_t n = A->rows;
+  const size_t nn = (size_t)std::max<int64_t>(n, 1), nc1 = (size_t)(ncl + 1);
+  PoolBuf kind(ctx), cw(ctx), list(ctx), count(ctx), tmp(ctx);
+  SPOPS_TRY(ncols.alloc(nc1 * 8));
+  SPOPS_TRY(cptr.alloc(nc1 * 8));
+  SPOPS_TRY(cptr_val.alloc(nc1 * 8));
+  SPOPS_TRY(cw.alloc(nc1 * 8));
+  SPOPS_TRY(list.alloc(nc1 * 8));
+  SPOPS_TRY(kind.alloc(nc1));
+  SPOPS_TRY(count.alloc(16));
+  // ncols[ncl] and cw[ncl] stay zero: the scans' last slots
+  SPOPS_CUDA(cudaMemsetAsync(ncols.as<int64_t>() + ncl, 0, 8, st));
+  SPOPS_CUDA(cudaMemsetAsync(cw.as<int64_t>() + ncl, 0, 8, st));
+  SPOPS_CUDA(cudaMemsetAsync(count.p, 0, 16, st));
+  if (ncl > 0) {
+    cluster_kind_kernel<I><<<grid_for(ncl * kClLanes), 256, 0, st>>>(
+        A->row.as<I>(), A->col.as<I>(), A->cols, perm, offs, ncl, kind.as<unsigned char>(), ncols.as<int64_t>(),
+        list.as<int64_t>(), count.as<unsigned long long>());
+    SPOPS_LAUNCH_CHECK();
+  }
+  int64_t hc[2] = {0, 0};
+  SPOPS_CUDA(cudaMemcpyAsync(hc, count.p, 16, cudaMemcpyDeviceToHost, st));
+  SPOPS_CUDA(cudaStreamSynchronize(st));
+  const int64_t nw = hc[0], nlist = hc[1];  // entries of wide clusters, clusters to sort
+  if (nlist > 0) {
+    cluster_count_kernel<I><<<grid_for(nlist * 32), 256, 0, st>>>(list.as<int64_t>(), nlist, A->row.as<I>(),
+                                                                  A->col.as<I>(), perm, offs, ncols.as<int64_t>());
+    SPOPS_LAUNCH_CHECK();
+  }
+  // key = cluster << kshift | column: sort only the bits in use
+  const int kshift = key_bits(A->cols), kend = std::min(64, kshift + key_bits(ncl));
+  PoolBuf skeys(ctx), ssrc(ctx), flag(ctx), uidx(ctx), base(ctx);
+  if (nw > 0) {
+    PoolBuf rowcl(ctx), rlen(ctx), rpr(ctx), keys(ctx), src(ctx);
+    SPOPS_TRY(skeys.alloc((size_t)nw * 8));
+    SPOPS_TRY(ssrc.alloc((size_t)nw * 16));
+    SPOPS_TRY(flag.alloc((size_t)nw * 8));
+    SPOPS_TRY(uidx.alloc((size_t)nw * 8));
+    SPOPS_TRY(base.alloc(nc1 * 8));
+    SPOPS_TRY(rowcl.alloc(nn * 8));
+    SPOPS_TRY(rlen.alloc(nn * 8));
+    SPOPS_TRY(rpr.alloc(nn * 8));
+    SPOPS_TRY(keys.alloc((size_t)nw * 8));
+    SPOPS_TRY(src.alloc((size_t)nw * 16));
+    row_cluster_kernel<<<grid_for(ncl), 256, 0, st>>>(offs, ncl, rowcl.as<int64_t>());
+    wide_len_kernel<I><<<grid_for(n), 256, 0, st>>>(A->row.as<I>(), perm, rowcl.as<int64_t>(),
+                                                    kind.as<unsigned char>(), n, rlen.as<int64_t>());
+    SPOPS_LAUNCH_CHECK();
+    size_t c1 = 0, c2 = 0, c3 = 0;
+    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, c1, rlen.as<int64_t>(), rpr.as<int64_t>(), n, st));
+    SPOPS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, c2, keys.as<uint64_t>(), skeys.as<uint64_t>(),
+                                               src.as<longlong2>(), ssrc.as<longlong2>(), nw, 0, kend, st));
+    SPOPS_CUDA(cub::DeviceScan::InclusiveSum(nullptr, c3, flag.as<int64_t>(), uidx.as<int64_t>(), nw, st));
+    SPOPS_TRY(tmp.alloc(std::max(c1, std::max(c2, c3)) + 256));
+    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, c1, rlen.as<int64_t>(), rpr.as<int64_t>(), n, st));
+    wide_keys_kernel<I><<<grid_for(n * 32), 256, 0, st>>>(
+        A->row.as<I>(), A->col.as<I>(), perm, rowcl.as<int64_t>(), offs, kind.as<unsigned char>(), n,
+        rpr.as<int64_t>(), kshift, keys.as<uint64_t>(), src.as<longlong2>());
+    SPOPS_LAUNCH_CHECK();
+    SPOPS_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, c2, keys.as<uint64_t>(), skeys.as<uint64_t>(),
+                                               src.as<longlong2>(), ssrc.as<longlong2>(), nw, 0, kend, st));
+    wide_flag_kernel<<<grid_for(nw), 256, 0, st>>>(skeys.as<uint64_t>(), nw, kshift, flag.as<int64_t>(),
+                                                   ncols.as<unsigned long long>());
+    SPOPS_LAUNCH_CHECK();
+    SPOPS_CUDA(cub::DeviceScan::InclusiveSum(tmp.p, c3, flag.as<int64_t>(), uidx.as<int64_t>(), nw, st));
+    wide_base_kernel<<<grid_for(nw), 256, 0, st>>>(skeys.as<uint64_t>(), uidx.as<int64_t>(), nw, kshift,
+                                                   base.as<int64_t>());
+    SPOPS_LAUNCH_CHECK();
+  }
+  // column pointers: exclusive scans of the column counts, plain and weighted
+  // by the cluster size
+  if (ncl > 0) {
+    weight_kernel<<<grid_for(ncl), 256, 0, st>>>(ncols.as<int64_t>(), offs, ncl, cw.as<int64_t>());
+    SPOPS_LAUNCH_CHECK();
+  }
+  {
+    size_t c1 = 0, c2 = 0;
+    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, c1, ncols.as<int64_t>(), cptr.as<int64_t>(), ncl + 1, st));
+    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, c2, cw.as<int64_t>(), cptr_val.as<int64_t>(), ncl + 1, st));
+    SPOPS_TRY(tmp.alloc(std::max(c1, c2) + 256));
+    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, c1, ncols.as<int64_t>(), cptr.as<int64_t>(), ncl + 1, st));
+    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, c2, cw.as<int64_t>(), cptr_val.as<int64_t>(), ncl + 1, st));
+  }
+  SPOPS_CUDA(cudaMemcpyAsync(nnzc, cptr.as<int64_t>() + ncl, 8, cudaMemcpyDeviceToHost, st));
+  SPOPS_CUDA(cudaMemcpyAsync(nnzv, cptr_val.as<int64_t>() + ncl, 8, cudaMemcpyDeviceToHost, st));
+  SPOPS_CUDA(cudaStreamSynchronize(st));
+  if (*nnzv > max_values)
+    return fail(SPOPS_ERR_TOO_LARGE, "csr_to_vlength_cluster: %lld values exceed int32 indices", (long long)*nnzv);
+  SPOPS_TRY(colids.alloc((size_t)std::max<int64_t>(*nnzc, 1) * 4));
+  SPOPS_TRY(avals.alloc((size_t)std::max<int64_t>(*nnzv, 1) * sizeof(V)));
+  SPOPS_CUDA(cudaMemsetAsync(avals.p, 0, avals.bytes, st));
+  if (ncl > 0) {
+    cluster_copy_kernel<I, V><<<grid_for(ncl * kClLanes), 256, 0, st>>>(
+        A->row.as<I>(), A->col.as<I>(), A->val.as<V>(), perm, offs, ncl, kind.as<unsigned char>(), cptr.as<int64_t>(),
+        cptr_val.as<int64_t>(), colids.as<int32_t>(), avals.as<V>());
+    SPOPS_LAUNCH_CHECK();
+  }
+  if (nlist > 0) {
+    cluster_fill_kernel<I, V><<<grid_for(nlist * 32), 256, 0, st>>>(
+        list.as<int64_t>(), nlist, A->row.as<I>(), A->col.as<I>(), A->val.as<V>(), perm, offs, cptr.as<int64_t>(),
+        cptr_val.as<int64_t>(), colids.as<int32_t>(), avals.as<V>());
+    SPOPS_LAUNCH_CHECK();
+  }
+  if (nw > 0) {
+    wide_fill_kernel<V><<<grid_for(nw), 256, 0, st>>>(
+        skeys.as<uint64_t>(), ssrc.as<longlong2>(), flag.as<int64_t>(), uidx.as<int64_t>(), base.as<int64_t>(), nw,
+        kshift, A->val.as<V>(), offs, cptr.as<int64_t>(), cptr_val.as<int64_t>(), colids.as<int32_t>(),
+        avals.as<V>());
+    SPOPS_LAUNCH_CHECK();
+  }
+  return SPOPS_OK;
 }
 
 // ------------------------------------------------------------ flops
@@ -784,6 +1119,9 @@ __global__ void row_count_kernel(const int64_t* __restrict__ soff_val, const int
   }
 }
 
+// C's rows from the slabs, one warp per cluster.  Bound by HBM: 28 bytes per
+// entry of an int64 / FP64 C, 0.83 ms for 1.2e8 entries (4.1 TB/s; 1.26 ms with
+// 32 entries in flight and a ballot per step).
 template <typename I, typename V>
 __global__ void row_write_kernel(const int64_t* __restrict__ soff, const int64_t* __restrict__ soff_val,
                                  const int64_t* __restrict__ nz, const int64_t* __restrict__ offsets,
@@ -795,16 +1133,41 @@ __global__ void row_write_kernel(const int64_t* __restrict__ soff, const int64_t
   if (c >= ncl) return;
   const int64_t csz = offsets[c + 1] - offsets[c];
   const int64_t ncol = nz[c];
+  const int64_t co = soff[c], cvo = soff_val[c];
   for (int64_t l = 0; l < csz; ++l) {
-    int64_t o = crp[perm[offsets[c] + l]];
+    const int64_t row = perm[offsets[c] + l];
+    int64_t o = crp[row];
+    if (csz == 1 && crp[row + 1] - o == ncol) {  // every column kept: a plain copy, 4 x 32 entries in flight
+      for (int64_t p0 = 0; p0 < ncol; p0 += 128) {
+        int32_t k[4];
+        V v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int64_t p = p0 + 32 * u + lane;
+          if (p < ncol) {
+            k[u] = __ldcs(ccol + co + p);
+            v[u] = __ldcs(cval + cvo + p);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int64_t p = p0 + 32 * u + lane;
+          if (p < ncol) {
+            __stcs(oci + o + p, (I)k[u]);
+            __stcs(ov + o + p, v[u]);
+          }
+        }
+      }
+      continue;
+    }
     for (int64_t p0 = 0; p0 < ncol; p0 += 32) {
       const int64_t p = p0 + lane;
-      const V v = p < ncol ? cval[soff_val[c] + p * csz + l] : V(0);
+      const V v = p < ncol ? cval[cvo + p * csz + l] : V(0);
       const bool keep = p < ncol && (keep_zeros || v != V(0));
       const unsigned m = __ballot_sync(0xffffffffu, keep);
       if (keep) {
         const int64_t at = o + __popc(m & ((1u << lane) - 1));
-        oci[at] = (I)ccol[soff[c] + p];
+        oci[at] = (I)ccol[co + p];
         ov[at] = v;
       }
       o += __popc(m);
@@ -823,12 +1186,6 @@ constexpr int kBinBits = 5;
 
 __device__ __forceinline__ int64_t pow2_ceil(int64_t v) {
   return v <= 1 ? 1 : (int64_t)1 << (64 - __clzll((unsigned long long)(v - 1)));
-}
-
-__global__ void weight_kernel(const int64_t* __restrict__ cnt, const int64_t* __restrict__ offsets, int64_t ncl,
-                              int64_t* __restrict__ weighted) {
-  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c < ncl) weighted[c] = cnt[c] * (offsets[c + 1] - offsets[c]);
 }
 
 // symbolic: table >= 2 * min(flops, cols) slots; 0 warp, 1 / 2 block in
@@ -1184,112 +1541,22 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
   Trace tr("spgemm");
   // --- permutation, offsets, per-row cluster
   ArenaScope scope(ctx);  // this call's temporaries come from the arena
-  PoolBuf perm(ctx), offs(ctx), rowcl(ctx), rlen(ctx), rpr(ctx), keys(ctx), skeys(ctx), src(ctx), ssrc(ctx), flag(ctx), uidx(ctx), colids(ctx), ncols_u(ctx), cptr(ctx), cptr_val(ctx), avals(ctx), row_of_entry(ctx), tmp(ctx);
-  SPOPS_TRY(perm.alloc((size_t)std::max<int64_t>(n, 1) * 8));
+  PoolBuf perm(ctx), offs(ctx), ncols_u(ctx), cptr(ctx), cptr_val(ctx), colids(ctx), avals(ctx), tot(ctx), tmp(ctx);
+  const size_t nn = (size_t)std::max<int64_t>(n, 1);
+  SPOPS_TRY(perm.alloc(nn * 8));
   SPOPS_TRY(offs.alloc((size_t)(ncl + 1) * 8));
+  SPOPS_TRY(tot.alloc(64));
   // host or device arrays (the device clustering hands over device ones)
   SPOPS_CUDA(cudaMemcpyAsync(perm.p, perm_h, (size_t)n * 8, cudaMemcpyDefault, st));
   SPOPS_CUDA(cudaMemcpyAsync(offs.p, offs_h, (size_t)(ncl + 1) * 8, cudaMemcpyDefault, st));
-  const size_t nn = (size_t)std::max<int64_t>(n, 1), nz1 = (size_t)std::max<int64_t>(nnz, 1);
-  SPOPS_TRY(rowcl.alloc(nn * 8));
-  SPOPS_TRY(rlen.alloc(nn * 8));
-  SPOPS_TRY(rpr.alloc((nn + 1) * 8));
-  if (ncl > 0) row_cluster_kernel<<<grid_for(ncl), 256, 0, st>>>(offs.as<int64_t>(), ncl, rowcl.as<int64_t>());
-  if (n > 0) reordered_len_kernel<I><<<grid_for(n), 256, 0, st>>>(A->row.as<I>(), perm.as<int64_t>(), n, rlen.as<int64_t>());
-  SPOPS_LAUNCH_CHECK();
+  // --- the clustered form of A
+  int64_t nnzc = 0, nnzv = 0;
+  SPOPS_TRY((build_clusters<I, V>(ctx, A, perm.as<int64_t>(), offs.as<int64_t>(), ncl, ncols_u, cptr, cptr_val,
+                                  colids, avals, INT64_MAX, &nnzc, &nnzv)));
+  const int64_t* cnt_d = ncols_u.as<int64_t>();
   size_t cb = 0;
-  SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, cb, rlen.as<int64_t>(), rpr.as<int64_t>(), (int64_t)nn, st));
-  SPOPS_TRY(tmp.alloc(cb + 256));
-  SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, cb, rlen.as<int64_t>(), rpr.as<int64_t>(), (int64_t)n, st));
-  tr.mark(st, "setup + reordered row scan");
-  // --- cluster keys, sort, unique
-  SPOPS_TRY(keys.alloc(nz1 * 8));
-  SPOPS_TRY(skeys.alloc(nz1 * 8));
-  SPOPS_TRY(src.alloc(nz1 * 8));
-  SPOPS_TRY(ssrc.alloc(nz1 * 8));
-  SPOPS_TRY(flag.alloc(nz1 * 8));
-  SPOPS_TRY(uidx.alloc(nz1 * 8));
-  SPOPS_TRY(row_of_entry.alloc(nz1 * 8));
-  tr.mark(st, "alloc key arrays");
-  if (tr.on && ctx->pool) {  // the pool's reserved and used bytes, for the trace
-    unsigned long long rsv = 0, used = 0;
-    cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &rsv);
-    cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used);
-    std::fprintf(stderr, "[spgemm] pool reserved %.1f MB, used %.1f MB\n", rsv / 1e6, used / 1e6);
-  }
-  // key = cluster << kshift | column: sort only the bits in use
-  const int kshift = key_bits(A->cols), kend = std::min(64, kshift + key_bits(ncl));
-  if (n > 0) {
-    cluster_keys_kernel<I, V><<<grid_for(n * 32), 256, 0, st>>>(A->row.as<I>(), A->col.as<I>(), perm.as<int64_t>(),
-                                                                rowcl.as<int64_t>(), n, rpr.as<int64_t>(), kshift,
-                                                                keys.as<uint64_t>(), src.as<int64_t>());
-    entry_row_kernel<I><<<grid_for(n * 32), 256, 0, st>>>(A->row.as<I>(), perm.as<int64_t>(), n,
-                                                          row_of_entry.as<int64_t>());
-    SPOPS_LAUNCH_CHECK();
-  }
-  int64_t nnzc = 0;
-  SPOPS_TRY(ncols_u.alloc((size_t)(ncl + 1) * 8));
-  SPOPS_CUDA(cudaMemsetAsync(ncols_u.p, 0, (size_t)(ncl + 1) * 8, st));
-  if (nnz > 0) {
-    size_t c1 = 0, c2 = 0;
-    SPOPS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, c1, keys.as<uint64_t>(), skeys.as<uint64_t>(), src.as<int64_t>(),
-                                               ssrc.as<int64_t>(), nnz, 0, kend, st));
-    SPOPS_CUDA(cub::DeviceScan::InclusiveSum(nullptr, c2, flag.as<int64_t>(), uidx.as<int64_t>(), nnz, st));
-    SPOPS_TRY(tmp.alloc(std::max(c1, c2) + 256));
-    SPOPS_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, c1, keys.as<uint64_t>(), skeys.as<uint64_t>(), src.as<int64_t>(),
-                                               ssrc.as<int64_t>(), nnz, 0, kend, st));
-    key_flag_kernel<<<grid_for(nnz), 256, 0, st>>>(skeys.as<uint64_t>(), nnz, flag.as<int64_t>());
-    SPOPS_LAUNCH_CHECK();
-    SPOPS_CUDA(cub::DeviceScan::InclusiveSum(tmp.p, c2, flag.as<int64_t>(), uidx.as<int64_t>(), nnz, st));
-    SPOPS_CUDA(cudaMemcpyAsync(&nnzc, uidx.as<int64_t>() + nnz - 1, 8, cudaMemcpyDeviceToHost, st));
-    SPOPS_CUDA(cudaStreamSynchronize(st));
-  }
-  tr.mark(st, "keys + sort + unique");
-  SPOPS_TRY(colids.alloc((size_t)std::max<int64_t>(nnzc, 1) * 4));
-  if (nnz > 0) {
-    cluster_cols_kernel<<<grid_for(nnz), 256, 0, st>>>(skeys.as<uint64_t>(), flag.as<int64_t>(), uidx.as<int64_t>(),
-                                                       nnz, kshift, colids.as<int32_t>(),
-                                                       reinterpret_cast<unsigned long long*>(ncols_u.p));
-    SPOPS_LAUNCH_CHECK();
-  }
-  // cluster column pointers: exclusive scans of the column counts, plain and
-  // weighted by the cluster size (ncols_u[ncl] and cw[ncl] are zero)
-  PoolBuf cw(ctx), tot(ctx);
-  SPOPS_TRY(cptr.alloc((size_t)(ncl + 1) * 8));
-  SPOPS_TRY(cptr_val.alloc((size_t)(ncl + 1) * 8));
-  SPOPS_TRY(cw.alloc((size_t)(ncl + 1) * 8));
-  SPOPS_TRY(tot.alloc(64));
-  SPOPS_CUDA(cudaMemsetAsync(cw.p, 0, (size_t)(ncl + 1) * 8, st));
-  const int64_t* cnt_d = reinterpret_cast<const int64_t*>(ncols_u.p);
-  if (ncl > 0) {
-    weight_kernel<<<grid_for(ncl), 256, 0, st>>>(cnt_d, offs.as<int64_t>(), ncl, cw.as<int64_t>());
-    SPOPS_LAUNCH_CHECK();
-  }
-  {
-    size_t c1 = 0, c2 = 0;
-    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, c1, cnt_d, cptr.as<int64_t>(), ncl + 1, st));
-    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, c2, cw.as<int64_t>(), cptr_val.as<int64_t>(), ncl + 1, st));
-    SPOPS_TRY(tmp.alloc(std::max(c1, c2) + 256));
-    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, c1, cnt_d, cptr.as<int64_t>(), ncl + 1, st));
-    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, c2, cw.as<int64_t>(), cptr_val.as<int64_t>(), ncl + 1, st));
-  }
-  int64_t nnzv = 0;
-  SPOPS_CUDA(cudaMemcpyAsync(&nnzv, cptr_val.as<int64_t>() + ncl, 8, cudaMemcpyDeviceToHost, st));
-  SPOPS_CUDA(cudaStreamSynchronize(st));
-  tr.mark(st, "cluster pointers");
-  SPOPS_TRY(avals.alloc((size_t)std::max<int64_t>(nnzv, 1) * sizeof(V)));
-  SPOPS_CUDA(cudaMemsetAsync(avals.p, 0, avals.bytes, st));
-  if (nnz > 0) {
-    cluster_vals_kernel<I, V><<<grid_for(nnz), 256, 0, st>>>(
-        skeys.as<uint64_t>(), ssrc.as<int64_t>(), uidx.as<int64_t>(), nnz, kshift, A->val.as<V>(), A->row.as<I>(),
-        perm.as<int64_t>(), offs.as<int64_t>(), cptr.as<int64_t>(), cptr_val.as<int64_t>(),
-        row_of_entry.as<int64_t>(), avals.as<V>());
-    SPOPS_LAUNCH_CHECK();
-  }
-  keys.release(); skeys.release(); src.release(); ssrc.release(); flag.release(); uidx.release();
-  row_of_entry.release(); rlen.release(); rpr.release(); rowcl.release();
   if (stats) stats->cluster_ms = tm.lap(st);
-  tr.mark(st, "cluster values + frees");
+  tr.mark(st, "clusters");
 
   // --- flops per cluster
   PoolBuf flops(ctx), nzd(ctx), cmin(ctx), cmax(ctx);
@@ -1795,97 +2062,18 @@ namespace {
 template <typename I, typename V>
 spops_status_t vl_from_csr_t(Context* ctx, Matrix* A, const int64_t* offs_h, int64_t ncl, Matrix** out) {
   cudaStream_t st = ctx->stream;
-  const int64_t n = A->rows, nnz = A->nnz;
-  const size_t nn = (size_t)std::max<int64_t>(n, 1), nz1 = (size_t)std::max<int64_t>(nnz, 1);
+  const int64_t n = A->rows;
+  const size_t nn = (size_t)std::max<int64_t>(n, 1);
   ArenaScope scope(ctx);  // this call's temporaries come from the arena
-  PoolBuf perm(ctx), offs(ctx), rowcl(ctx), rlen(ctx), rpr(ctx), keys(ctx), skeys(ctx), src(ctx), ssrc(ctx),
-      flag(ctx), uidx(ctx), colids(ctx), ncols_u(ctx), cptr(ctx), cptr_val(ctx), cw(ctx), avals(ctx), roe(ctx),
-      tmp(ctx);
+  PoolBuf perm(ctx), offs(ctx), ncols(ctx), cptr(ctx), cptr_val(ctx), colids(ctx), avals(ctx);
   SPOPS_TRY(perm.alloc(nn * 8));
   SPOPS_TRY(offs.alloc((size_t)(ncl + 1) * 8));
-  SPOPS_TRY(rowcl.alloc(nn * 8));
-  SPOPS_TRY(rlen.alloc(nn * 8));
-  SPOPS_TRY(rpr.alloc((nn + 1) * 8));
   SPOPS_CUDA(cudaMemcpyAsync(offs.p, offs_h, (size_t)(ncl + 1) * 8, cudaMemcpyHostToDevice, st));
   if (n > 0) iota_kernel<<<grid_for(n), 256, 0, st>>>(perm.as<int64_t>(), n);
-  if (ncl > 0) row_cluster_kernel<<<grid_for(ncl), 256, 0, st>>>(offs.as<int64_t>(), ncl, rowcl.as<int64_t>());
-  if (n > 0) reordered_len_kernel<I><<<grid_for(n), 256, 0, st>>>(A->row.as<I>(), perm.as<int64_t>(), n, rlen.as<int64_t>());
   SPOPS_LAUNCH_CHECK();
-  size_t cb = 0;
-  SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, cb, rlen.as<int64_t>(), rpr.as<int64_t>(), (int64_t)nn, st));
-  SPOPS_TRY(tmp.alloc(cb + 256));
-  if (n > 0) SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, cb, rlen.as<int64_t>(), rpr.as<int64_t>(), n, st));
-  SPOPS_TRY(keys.alloc(nz1 * 8));
-  SPOPS_TRY(skeys.alloc(nz1 * 8));
-  SPOPS_TRY(src.alloc(nz1 * 8));
-  SPOPS_TRY(ssrc.alloc(nz1 * 8));
-  SPOPS_TRY(flag.alloc(nz1 * 8));
-  SPOPS_TRY(uidx.alloc(nz1 * 8));
-  SPOPS_TRY(roe.alloc(nz1 * 8));
-  // key = cluster << kshift | column: sort only the bits in use
-  const int kshift = key_bits(A->cols), kend = std::min(64, kshift + key_bits(ncl));
-  if (n > 0) {
-    cluster_keys_kernel<I, V><<<grid_for(n * 32), 256, 0, st>>>(A->row.as<I>(), A->col.as<I>(), perm.as<int64_t>(),
-                                                                rowcl.as<int64_t>(), n, rpr.as<int64_t>(), kshift,
-                                                                keys.as<uint64_t>(), src.as<int64_t>());
-    entry_row_kernel<I><<<grid_for(n * 32), 256, 0, st>>>(A->row.as<I>(), perm.as<int64_t>(), n, roe.as<int64_t>());
-    SPOPS_LAUNCH_CHECK();
-  }
-  int64_t nnzc = 0;
-  SPOPS_TRY(ncols_u.alloc((size_t)(ncl + 1) * 8));
-  SPOPS_CUDA(cudaMemsetAsync(ncols_u.p, 0, (size_t)(ncl + 1) * 8, st));
-  if (nnz > 0) {
-    size_t c1 = 0, c2 = 0;
-    SPOPS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, c1, keys.as<uint64_t>(), skeys.as<uint64_t>(), src.as<int64_t>(),
-                                               ssrc.as<int64_t>(), nnz, 0, kend, st));
-    SPOPS_CUDA(cub::DeviceScan::InclusiveSum(nullptr, c2, flag.as<int64_t>(), uidx.as<int64_t>(), nnz, st));
-    SPOPS_TRY(tmp.alloc(std::max(c1, c2) + 256));
-    SPOPS_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, c1, keys.as<uint64_t>(), skeys.as<uint64_t>(), src.as<int64_t>(),
-                                               ssrc.as<int64_t>(), nnz, 0, kend, st));
-    key_flag_kernel<<<grid_for(nnz), 256, 0, st>>>(skeys.as<uint64_t>(), nnz, flag.as<int64_t>());
-    SPOPS_LAUNCH_CHECK();
-    SPOPS_CUDA(cub::DeviceScan::InclusiveSum(tmp.p, c2, flag.as<int64_t>(), uidx.as<int64_t>(), nnz, st));
-    SPOPS_CUDA(cudaMemcpyAsync(&nnzc, uidx.as<int64_t>() + nnz - 1, 8, cudaMemcpyDeviceToHost, st));
-    SPOPS_CUDA(cudaStreamSynchronize(st));
-  }
-  SPOPS_TRY(colids.alloc((size_t)std::max<int64_t>(nnzc, 1) * 4));
-  if (nnz > 0) {
-    cluster_cols_kernel<<<grid_for(nnz), 256, 0, st>>>(skeys.as<uint64_t>(), flag.as<int64_t>(), uidx.as<int64_t>(),
-                                                       nnz, kshift, colids.as<int32_t>(),
-                                                       reinterpret_cast<unsigned long long*>(ncols_u.p));
-    SPOPS_LAUNCH_CHECK();
-  }
-  SPOPS_TRY(cptr.alloc((size_t)(ncl + 1) * 8));
-  SPOPS_TRY(cptr_val.alloc((size_t)(ncl + 1) * 8));
-  SPOPS_TRY(cw.alloc((size_t)(ncl + 1) * 8));
-  SPOPS_CUDA(cudaMemsetAsync(cw.p, 0, (size_t)(ncl + 1) * 8, st));
-  const int64_t* cnt_d = reinterpret_cast<const int64_t*>(ncols_u.p);
-  if (ncl > 0) {
-    weight_kernel<<<grid_for(ncl), 256, 0, st>>>(cnt_d, offs.as<int64_t>(), ncl, cw.as<int64_t>());
-    SPOPS_LAUNCH_CHECK();
-  }
-  {
-    size_t c1 = 0, c2 = 0;
-    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, c1, cnt_d, cptr.as<int64_t>(), ncl + 1, st));
-    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, c2, cw.as<int64_t>(), cptr_val.as<int64_t>(), ncl + 1, st));
-    SPOPS_TRY(tmp.alloc(std::max(c1, c2) + 256));
-    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, c1, cnt_d, cptr.as<int64_t>(), ncl + 1, st));
-    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, c2, cw.as<int64_t>(), cptr_val.as<int64_t>(), ncl + 1, st));
-  }
-  int64_t nnzv = 0;
-  SPOPS_CUDA(cudaMemcpyAsync(&nnzv, cptr_val.as<int64_t>() + ncl, 8, cudaMemcpyDeviceToHost, st));
-  SPOPS_CUDA(cudaStreamSynchronize(st));
-  if (sizeof(I) == 4 && nnzv > INT32_MAX)
-    return fail(SPOPS_ERR_TOO_LARGE, "csr_to_vlength_cluster: %lld values exceed int32 indices", (long long)nnzv);
-  SPOPS_TRY(avals.alloc((size_t)std::max<int64_t>(nnzv, 1) * sizeof(V)));
-  SPOPS_CUDA(cudaMemsetAsync(avals.p, 0, avals.bytes, st));
-  if (nnz > 0) {
-    cluster_vals_kernel<I, V><<<grid_for(nnz), 256, 0, st>>>(
-        skeys.as<uint64_t>(), ssrc.as<int64_t>(), uidx.as<int64_t>(), nnz, kshift, A->val.as<V>(), A->row.as<I>(),
-        perm.as<int64_t>(), offs.as<int64_t>(), cptr.as<int64_t>(), cptr_val.as<int64_t>(), roe.as<int64_t>(),
-        avals.as<V>());
-    SPOPS_LAUNCH_CHECK();
-  }
+  int64_t nnzc = 0, nnzv = 0;
+  SPOPS_TRY((build_clusters<I, V>(ctx, A, perm.as<int64_t>(), offs.as<int64_t>(), ncl, ncols, cptr, cptr_val, colids,
+                                  avals, sizeof(I) == 4 ? INT32_MAX : INT64_MAX, &nnzc, &nnzv)));
   return make_vlcluster<I, V>(ctx, n, A->cols, ncl, offs.as<int64_t>(), cptr.as<int64_t>(), colids.as<int32_t>(),
                               nnzc, cptr_val.as<int64_t>(), avals.as<V>(), nnzv, A->itype, out);
 }

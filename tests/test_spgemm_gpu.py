@@ -457,3 +457,37 @@ def test_rowwise_product_count_edges(cuda, itype, vtype, sorted_b):
         got = v[rp[i]:rp[i + 1]].astype(np.float64)
         err = np.abs(got - [val[c] for c in want]) / np.array([mag[c] for c in want])
         assert err.max() <= tol, counts[i]
+
+
+@pytest.mark.parametrize("itype", [np.int32, np.int64])
+def test_cluster_build_kinds(cuda, orc, itype):
+    """Clusters at the limits between the ways their column lists are built:
+    one row (ascending, or in another order), up to 32 rows and 512 entries
+    (33, 64, 65, 128, 129, 256, 257, 512), one entry or one row more, none."""
+    from sparseops_b200.spgemm import LeSpGEMM_clustered
+    rng = np.random.default_rng(31)
+    ncols = 700
+    shapes = [(1, 40), (1, 9), (1, 0), (0, 0), (32, 33), (5, 64), (32, 65), (3, 128), (9, 129), (32, 256), (2, 257),
+              (32, 512), (32, 513), (33, 60), (1, 600), (40, 2000), (7, 0), (1, 1)]
+    lens, offs = [], [0]
+    for rows, entries in shapes:
+        cut = np.sort(rng.integers(0, entries + 1, max(rows - 1, 0)))
+        part = np.diff(np.concatenate([[0], cut, [entries]])) if rows else np.zeros(0, int)
+        while rows and part.max() > ncols:  # a row holds each column once
+            part[part.argmax()] -= 100
+            part[part.argmin()] += 100
+        lens += list(part)
+        offs.append(offs[-1] + rows)
+    n = len(lens)
+    perm = rng.permutation(n)  # cluster position r holds original row perm[r]
+    cols = [None] * n
+    for r, m in enumerate(lens):
+        c = rng.choice(ncols, m, replace=False)
+        cols[perm[r]] = c if r == 1 else np.sort(c)  # position 1: a one-row cluster in another order
+    arp = np.concatenate([[0], np.cumsum([len(c) for c in cols])])
+    aci, av = np.concatenate(cols), rng.standard_normal(arp[-1])
+    brp, bci, bv = synth.powerlaw(ncols, hi=60, seed=6)
+    a, b = (arp.astype(itype), aci.astype(itype), av), (brp.astype(itype), bci.astype(itype), bv)
+    C = LeSpGEMM_clustered(_csr(*a, ncols), _csr(*b, ncols), perm, offs)
+    a64, b64 = (arp.astype(np.int64), aci.astype(np.int64), av), (brp.astype(np.int64), bci.astype(np.int64), bv)
+    _check_c(C, orc.spgemm(a64, b64, perm.astype(np.int64), np.array(offs, np.int64)))
