@@ -322,7 +322,9 @@ spops_status_t spops_matrix_download(spops_context_t ctx, spops_matrix_t A, spop
 spops_status_t spops_matrix_destroy(spops_matrix_t A) {
   if (!A) return SPOPS_OK;
   DeviceGuard g(A->ctx->device);
-  cudaStreamSynchronize(A->ctx->stream);
+  // every stream that may still read the arrays: blocks that go to the
+  // context's cache are handed out again without cudaFree's own wait
+  cudaDeviceSynchronize();
   A->release_all();
   delete A;
   return SPOPS_OK;

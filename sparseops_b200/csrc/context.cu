@@ -55,32 +55,36 @@ spops_status_t DevBuf::alloc(size_t n) {
 
 void DevBuf::release() {
   if (own && p) {
-    if (home) home->cache_block(p, bytes);
+    if (home) home->cache_block(p, span, keep);
     else cudaFree(p);
   }
   p = nullptr;
-  bytes = 0;
+  bytes = span = 0;
   own = false;
   home = nullptr;
 }
 
-constexpr size_t kCacheMin = size_t(1) << 20;   // blocks below this go back to the driver
-constexpr size_t kCacheMax = size_t(24) << 30;  // bytes the cache may hold
+constexpr size_t kCacheMin = size_t(1) << 20;  // blocks below this go back to the driver, ...
+constexpr size_t kBuildMin = 16;               // ... except what building makes (plans, windows)
+constexpr size_t kBuildBlocks = 512;           // of which the cache holds at most this many
+inline size_t cache_min(size_t keep_max) { return keep_max == kBuildCacheMax ? kBuildMin : kCacheMin; }
 
-spops_status_t DevBuf::alloc_cached(Context* ctx, size_t n) {
+spops_status_t DevBuf::alloc_cached(Context* ctx, size_t n, size_t keep_max) {
   release();
   if (n == 0) n = 16;
   static const bool trace = [] {
     const char* e = std::getenv("SPOPS_TRACE");
     return e && (e[0] == '1' || e[0] == '2');
   }();
-  if (n >= kCacheMin) {
+  if (n >= cache_min(keep_max)) {
     void* q = nullptr;
     size_t b = 0;
     if (ctx->take_block(n, &q, &b)) {
       if (trace) std::fprintf(stderr, "[cache] %zu bytes from a cached block of %zu\n", n, b);
       p = q;
-      bytes = b;
+      bytes = n;
+      span = b;
+      keep = keep_max;
       own = true;
       home = ctx;
       return SPOPS_OK;
@@ -89,15 +93,35 @@ spops_status_t DevBuf::alloc_cached(Context* ctx, size_t n) {
       std::fprintf(stderr, "[cache] %zu bytes: no cached block (%zu blocks, %zu bytes held)\n", n,
                    ctx->block_cache.size(), ctx->block_cache_bytes);
   }
-  SPOPS_TRY(alloc(n));
-  if (n >= kCacheMin) home = ctx;
+  spops_status_t s = alloc(n);
+  if (s == SPOPS_ERR_ALLOC && ctx->block_cache_bytes > 0) {  // what the cache holds may be what is missing
+    ctx->drop_block_cache();
+    s = alloc(n);
+  }
+  SPOPS_TRY(s);
+  if (n >= cache_min(keep_max)) {
+    home = ctx;
+    span = n;
+    keep = keep_max;
+  }
   return SPOPS_OK;
 }
 
-void Context::cache_block(void* q, size_t b) {
-  if (b < kCacheMin || block_cache_bytes + b > kCacheMax) {
+// The cache is locked: a handle may be destroyed by one thread while another
+// is inside a call on the same context.  What building makes has its own
+// limits, and its oldest blocks make room for new ones.
+void Context::cache_block(void* q, size_t b, size_t keep_max) {
+  std::lock_guard<std::mutex> lock(block_mutex);
+  const bool build = keep_max == kBuildCacheMax;
+  if (build ? b > keep_max / 2 : (b < kCacheMin || block_cache_bytes + b > keep_max)) {
     cudaFree(q);
     return;
+  }
+  while (build && (build_bytes + b > keep_max || build_blocks >= kBuildBlocks)) {
+    size_t i = 0;  // the oldest of them
+    while (!block_cache[i].build) ++i;
+    cudaEventSynchronize(block_cache[i].done);
+    drop_block(i, true);
   }
   cudaEvent_t e = nullptr;
   if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess ||
@@ -107,13 +131,32 @@ void Context::cache_block(void* q, size_t b) {
     cudaFree(q);
     return;
   }
-  block_cache.push_back(CachedBlock{q, b, e});
+  block_cache.push_back(CachedBlock{q, b, e, build});
   block_cache_bytes += b;
+  if (build) {
+    build_bytes += b;
+    ++build_blocks;
+  }
+}
+
+// take block i off the list (and free it); the caller has waited for it
+void Context::drop_block(size_t i, bool free_it) {
+  const CachedBlock c = block_cache[i];
+  block_cache.erase(block_cache.begin() + (ptrdiff_t)i);
+  block_cache_bytes -= c.bytes;
+  if (c.build) {
+    build_bytes -= c.bytes;
+    --build_blocks;
+  }
+  cudaEventDestroy(c.done);
+  if (free_it) cudaFree(c.p);
 }
 
 bool Context::take_block(size_t n, void** q, size_t* b) {
-  // the smallest block of at least n bytes and at most n + n / 8 + 2 MB
-  const size_t hi = n + n / 8 + (size_t(2) << 20);
+  // the smallest block of at least n bytes and at most n + n / 8 + 2 MB (4 KB
+  // for the small ones)
+  const size_t hi = n + n / 8 + (n >= kCacheMin ? size_t(2) << 20 : size_t(4) << 10);
+  std::lock_guard<std::mutex> lock(block_mutex);
   int best = -1;
   for (int i = 0; i < (int)block_cache.size(); ++i) {
     const size_t s = block_cache[i].bytes;
@@ -121,23 +164,19 @@ bool Context::take_block(size_t n, void** q, size_t* b) {
   }
   if (best < 0) return false;
   const CachedBlock c = block_cache[best];
-  block_cache.erase(block_cache.begin() + best);
-  block_cache_bytes -= c.bytes;
   cudaStreamWaitEvent(stream, c.done, 0);  // work queued before the release may still use it
-  cudaEventDestroy(c.done);
+  drop_block((size_t)best, false);
   *q = c.p;
   *b = c.bytes;
   return true;
 }
 
 void Context::drop_block_cache() {
-  for (const CachedBlock& c : block_cache) {
-    cudaEventSynchronize(c.done);
-    cudaEventDestroy(c.done);
-    cudaFree(c.p);
+  std::lock_guard<std::mutex> lock(block_mutex);
+  while (!block_cache.empty()) {
+    cudaEventSynchronize(block_cache.back().done);
+    drop_block(block_cache.size() - 1, true);
   }
-  block_cache.clear();
-  block_cache_bytes = 0;
 }
 
 spops_status_t Context::pool_alloc(void** out, size_t bytes) {

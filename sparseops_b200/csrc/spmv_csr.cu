@@ -58,9 +58,13 @@ __global__ void validate_kernel(const I* __restrict__ rp, const I* __restrict__ 
   }
 }
 
+// blocks starting at each row (nblk[n] = 0 for the scan's last slot), and the
+// number of long rows
 template <typename I>
-__global__ void plan_count_kernel(const I* __restrict__ rp, int64_t n, int64_t* __restrict__ nblk) {
+__global__ void plan_count_kernel(const I* __restrict__ rp, int64_t n, int64_t* __restrict__ nblk,
+                                  unsigned long long* __restrict__ nlong) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (r == n) nblk[n] = 0;
   if (r >= n) return;
   const int64_t s = rp[r], e = rp[r + 1];
   const int64_t len = e - s;
@@ -72,6 +76,7 @@ __global__ void plan_count_kernel(const I* __restrict__ rp, int64_t n, int64_t* 
     flag = is_long || prev_long || (s / kCap) != (sp / kCap) || (r % kRowCap) == 0;
   }
   nblk[r] = flag ? (is_long ? (len + kCap - 1) / kCap : 1) : 0;
+  if (is_long) atomicAdd(nlong, 1ULL);
 }
 
 template <typename I>
@@ -89,12 +94,6 @@ __global__ void plan_fill_kernel(const I* __restrict__ rp, int64_t n, const int6
     blk_row[o + c] = r;
     blk_chunk[o + c] = is_long ? (int)c : -1;
   }
-}
-
-__global__ void count_long_kernel(const int* __restrict__ blk_chunk, int64_t nblocks,
-                                  unsigned long long* __restrict__ nlong) {
-  const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (b < nblocks && blk_chunk[b] == 0) atomicAdd(nlong, 1ULL);
 }
 
 template <typename I>
@@ -151,17 +150,21 @@ spops_status_t analyse_t(Context* ctx, Matrix* A) {
   cudaStream_t st = ctx->stream;
   size_t cub_bytes = 0;
   int64_t* dummy = nullptr;
-  SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, dummy, dummy, (int64_t)(n > 0 ? n : 1), st));
-  const size_t arr = ((size_t)(n > 0 ? n : 1) * sizeof(int64_t) + 255) & ~(size_t)255;
-  SPOPS_TRY(ctx->scratch_reserve(2 * arr + 256 + cub_bytes));
+  SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, dummy, dummy, n + 1, st));
+  // nblk [n + 1] | boff [n + 1], followed by the pattern flag and the number of
+  // long rows, read back with boff's last entry | the scan's temporaries
+  const size_t n1 = (size_t)n + 1, arr = (n1 * sizeof(int64_t) + 255) & ~(size_t)255;
+  const size_t arr2 = ((n1 + 2) * sizeof(int64_t) + 255) & ~(size_t)255;
+  SPOPS_TRY(ctx->scratch_reserve(arr + arr2 + cub_bytes));
   char* base = ctx->scratch.as<char>();
   int64_t* nblk = reinterpret_cast<int64_t*>(base);
   int64_t* boff = reinterpret_cast<int64_t*>(base + arr);
-  int* bad = reinterpret_cast<int*>(base + 2 * arr);
-  void* cub_tmp = base + 2 * arr + 256;
+  int* bad = reinterpret_cast<int*>(boff + n1);
+  unsigned long long* nlong = reinterpret_cast<unsigned long long*>(boff + n1 + 1);
+  void* cub_tmp = base + arr + arr2;
 
   // validate the pattern once: the kernels index x with these columns
-  SPOPS_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), st));
+  SPOPS_CUDA(cudaMemsetAsync(bad, 0, 2 * sizeof(int64_t), st));
   {
     const int64_t work = (n + 1 > A->nnz ? n + 1 : A->nnz);
     int64_t grid = (work + 255) / 256;
@@ -170,24 +173,14 @@ spops_status_t analyse_t(Context* ctx, Matrix* A) {
     validate_kernel<I><<<(unsigned)grid, 256, 0, st>>>(rp, A->col.as<I>(), n, A->nnz, A->cols, bad);
     SPOPS_LAUNCH_CHECK();
   }
-  int hbad = 0;
-  SPOPS_CUDA(cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
-
-  int64_t nblocks = 0;
-  if (n > 0) {
-    const int threads = 256;
-    const int64_t grid = (n + threads - 1) / threads;
-    plan_count_kernel<I><<<(unsigned)grid, threads, 0, st>>>(rp, n, nblk);
-    SPOPS_LAUNCH_CHECK();
-    SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, nblk, boff, n, st));
-    int64_t last_off = 0, last_cnt = 0;
-    SPOPS_CUDA(cudaMemcpyAsync(&last_off, boff + n - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    SPOPS_CUDA(cudaMemcpyAsync(&last_cnt, nblk + n - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    SPOPS_CUDA(cudaStreamSynchronize(st));
-    nblocks = last_off + last_cnt;
-  } else {
-    SPOPS_CUDA(cudaStreamSynchronize(st));
-  }
+  plan_count_kernel<I><<<(unsigned)((n + 256) / 256), 256, 0, st>>>(rp, n, nblk, nlong);
+  SPOPS_LAUNCH_CHECK();
+  SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, nblk, boff, n + 1, st));
+  int64_t h[3] = {0, 0, 0};  // blocks, flag, long rows
+  SPOPS_CUDA(cudaMemcpyAsync(h, boff + n, sizeof(h), cudaMemcpyDeviceToHost, st));
+  SPOPS_CUDA(cudaStreamSynchronize(st));
+  const int64_t nblocks = h[0];
+  const int hbad = (int)h[1];
   if (hbad) {
     return fail(SPOPS_ERR_INVALID, "CSR pattern invalid: %s%s", (hbad & 1) ? "row offsets not monotone in [0,nnz] " : "",
                 (hbad & 2) ? "column index outside [0,cols)" : "");
@@ -196,11 +189,11 @@ spops_status_t analyse_t(Context* ctx, Matrix* A) {
   P.cap = kCap;
   P.nblocks = nblocks;
   const size_t nb1 = (size_t)(nblocks > 0 ? nblocks : 1);
-  SPOPS_TRY(P.blk_row.alloc((size_t)(nblocks + 1) * sizeof(int64_t)));
-  SPOPS_TRY(P.blk_chunk.alloc(nb1 * sizeof(int)));
-  SPOPS_TRY(P.seg.alloc(nb1 * sizeof(CsrSeg)));
-  SPOPS_TRY(P.partial.alloc(nb1 * sizeof(double)));
-  SPOPS_TRY(P.counter.alloc(nb1 * sizeof(int)));
+  SPOPS_TRY(P.blk_row.alloc_cached(ctx, (size_t)(nblocks + 1) * sizeof(int64_t), kBuildCacheMax));
+  SPOPS_TRY(P.blk_chunk.alloc_cached(ctx, nb1 * sizeof(int), kBuildCacheMax));
+  SPOPS_TRY(P.seg.alloc_cached(ctx, nb1 * sizeof(CsrSeg), kBuildCacheMax));
+  SPOPS_TRY(P.partial.alloc_cached(ctx, nb1 * sizeof(double), kBuildCacheMax));
+  SPOPS_TRY(P.counter.alloc_cached(ctx, nb1 * sizeof(int), kBuildCacheMax));
   SPOPS_CUDA(cudaMemsetAsync(P.counter.p, 0, P.counter.bytes, st));
   if (n > 0) {
     const int threads = 256;
@@ -211,18 +204,13 @@ spops_status_t analyse_t(Context* ctx, Matrix* A) {
     if (nblocks > 0) {
       plan_seg_kernel<I><<<(unsigned)((nblocks + 255) / 256), 256, 0, st>>>(
           rp, P.blk_row.as<int64_t>(), P.blk_chunk.as<int>(), nblocks, P.seg.as<CsrSeg>());
-      unsigned long long* nl = reinterpret_cast<unsigned long long*>(nblk);  // scratch reuse
-      SPOPS_CUDA(cudaMemsetAsync(nl, 0, 8, st));
-      count_long_kernel<<<(unsigned)((nblocks + 255) / 256), 256, 0, st>>>(P.blk_chunk.as<int>(), nblocks, nl);
       SPOPS_LAUNCH_CHECK();
-      unsigned long long hl = 0;
-      SPOPS_CUDA(cudaMemcpyAsync(&hl, nl, 8, cudaMemcpyDeviceToHost, st));
-      SPOPS_CUDA(cudaStreamSynchronize(st));
-      P.nlong = (int64_t)hl;
     }
   } else {
     SPOPS_CUDA(cudaMemsetAsync(P.blk_row.p, 0, sizeof(int64_t), st));
   }
+  SPOPS_CUDA(cudaStreamSynchronize(st));  // the plan may be used on another stream
+  P.nlong = h[2];
   P.ready = true;
   return SPOPS_OK;
 }

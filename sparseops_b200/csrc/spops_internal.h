@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <string>
 #include <functional>
+#include <mutex>
 #include <utility>
 #include <vector>
 
@@ -40,15 +41,25 @@ spops_status_t cuda_fail(cudaError_t e, const char* what, const char* file, int 
 // ---------------------------------------------------------------- buffers
 // Device allocation owned by a handle (or borrowed when own == false).
 struct Context;
+constexpr size_t kBlockCacheMax = size_t(24) << 30;  // bytes a context's block cache may hold
+// for what conversions and assembly make (COO views, CSR, padded formats):
+// blocks of a few tens to hundreds of MB, whose cudaMalloc and cudaFree cost
+// more than filling them
+constexpr size_t kBuildCacheMax = size_t(2) << 30;
+
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
   bool own = false;
   Context* home = nullptr;  // set by alloc_cached: released into home's block cache
+  size_t span = 0;          // alloc_cached: the block's size (bytes: what was asked for)
+  size_t keep = 0;          // alloc_cached: its keep_max
   spops_status_t alloc(size_t n);
   // n bytes, reusing a block of about that size that an earlier result of
-  // this context released (large results only; see Context::block_cache)
-  spops_status_t alloc_cached(Context* ctx, size_t n);
+  // this context released (large results only; see Context::block_cache).
+  // keep_max: the block is kept on release only while the cache then holds no
+  // more than this (kBuildCacheMax: of the blocks allocated with it).
+  spops_status_t alloc_cached(Context* ctx, size_t n, size_t keep_max = kBlockCacheMax);
   void release();
   void borrow(const void* q, size_t n) { release(); p = const_cast<void*>(q); bytes = n; own = false; }
   template <typename T> T* as() const { return static_cast<T*>(p); }
@@ -124,10 +135,14 @@ struct Context {
     void* p;
     size_t bytes;
     cudaEvent_t done;
+    bool build;  // made by a conversion or assembly: kBuildCacheMax bytes of these at most
   };
   std::vector<CachedBlock> block_cache;
   size_t block_cache_bytes = 0;
-  void cache_block(void* p, size_t bytes);
+  size_t build_bytes = 0, build_blocks = 0;
+  void drop_block(size_t i, bool free_it);
+  std::mutex block_mutex;
+  void cache_block(void* p, size_t bytes, size_t keep_max);
   bool take_block(size_t n, void** p, size_t* bytes);
   void drop_block_cache();
   size_t arena_top = 0;       // bytes handed out

@@ -396,3 +396,61 @@ def test_csr_reorder_rows(cuda, itype, vtype):
     bad[0] = n  # out of range
     with pytest.raises(SpOpsError):
         csr_reorder_rows(A, bad)
+
+
+@pytest.mark.parametrize("itype,vtype", [(np.int32, np.float64), (np.int64, np.float32)])
+@pytest.mark.parametrize("lens,cols", [
+    ([1, 31, 32, 33, 64, 65, 128, 129, 256, 257, 511, 512, 0, 7], 90),      # rows summed in registers
+    ([1, 31, 0, 513, 64], 90),                                              # one row too long: the global sorts
+    ([20, 512, 3], (1 << 23) - 1), ([20, 512, 3], 1 << 23), ([5], 1 << 27)  # columns that just fit a key, and not
+])
+def test_coo_to_csr_compact_row_lengths(cuda, itype, vtype, lens, cols):
+    """Duplicate sums at the row lengths and column counts where the summation
+    changes its form: bit-exact against the sequential definition (values
+    added in file order from zero, columns in reverse order of first
+    appearance, exact-zero sums dropped)."""
+    import torch
+    from sparseops_b200 import COO_Matrix, coo_to_csr
+    rng = np.random.default_rng(len(lens) * 1000 + cols % 997)
+    rows = np.repeat(np.arange(len(lens)), lens)
+    few = np.concatenate([rng.integers(0, cols, 60), [0, cols - 1]])
+    ci = rng.choice(few, len(rows))
+    v = rng.integers(-2, 3, len(rows)) * 0.25 + rng.choice([0.0, 0.1], len(rows))  # sums that cancel exactly, too
+    order = rng.permutation(len(rows))
+    rows, ci, v = rows[order].astype(itype), ci[order].astype(itype), v[order].astype(vtype)
+    C = coo_to_csr(COO_Matrix(len(lens), cols, *(torch.from_numpy(a).to("cuda") for a in (rows, ci, v))), compact=True)
+    rp, oc, ov = C.host()
+    want_c, want_v, want_p = [], [], [0]
+    for r in range(len(lens)):
+        sums = {}
+        for k in np.flatnonzero(rows == r):
+            sums[ci[k]] = vtype(sums.get(ci[k], vtype(0)) + v[k])
+        kept = [(c, s) for c, s in reversed(sums.items()) if s != 0]
+        want_c += [c for c, _ in kept]
+        want_v += [s for _, s in kept]
+        want_p.append(len(want_c))
+    assert np.array_equal(rp, want_p) and np.array_equal(oc, want_c)
+    assert np.array_equal(ov, np.array(want_v, vtype))
+
+
+@pytest.mark.parametrize("lens", [[5] * 70, [0] * 33 + [1], [40, 0, 3] * 30, [1] * 31, [300] + [2] * 63])
+def test_sell_c32_chunk_fill(cuda, lens):
+    """Column-major chunks of 32 rows, padding included: ragged last chunk,
+    empty rows, rows over several 32-slot strips."""
+    import torch
+    from sparseops_b200 import CSR_Matrix, convert_to
+    rng = np.random.default_rng(len(lens))
+    n, cols = len(lens), 400
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = np.concatenate([np.sort(rng.choice(cols, m, replace=False)) for m in lens]).astype(np.int32)
+    v = rng.standard_normal(len(ci))
+    A = CSR_Matrix(n, cols, *(torch.from_numpy(a).to("cuda") for a in (rp, ci, v)))
+    S = convert_to(A, "sell_c_sigma", sigma=64, chunk=32, layout=1)
+    ro, cl, off = S.reorder, S.chunk_len, S._arr("chunk_off")
+    col, val = S._arr("col"), S._arr("val", "f")
+    wc, wv = np.full(off[-1], -1, np.int32), np.zeros(off[-1])
+    for i, r in enumerate(ro):
+        c, l = divmod(i, 32)
+        for k in range(lens[r]):
+            wc[off[c] + k * 32 + l], wv[off[c] + k * 32 + l] = ci[rp[r] + k], v[rp[r] + k]
+    assert len(cl) == (n + 31) // 32 and np.array_equal(col, wc) and np.array_equal(val, wv)
