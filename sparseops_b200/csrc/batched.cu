@@ -157,36 +157,73 @@ __global__ void __launch_bounds__(kBatchBlock, KT == 1 ? 4 : 3) batch_kernel(con
 }
 
 // Tile items (k = 8, 16, 32): item idx covers tiles [idx, idx + kTilesPerItem) of its
-// matrix, taken from the queue as in batch_kernel.
+// matrix, taken from the queue as in batch_kernel, but by whole blocks: a
+// block takes kBlockItems neighbouring items and its warps their tiles in
+// turn, so the warps running together hold neighbouring rows and find the
+// X rows that a banded pattern shares in L1, while the window of matrices in
+// flight stays small enough for L2.  256 matrices, FP64: k = 32 6.03 ms with
+// items taken by single warps, 5.27 ms so, 4.43 ms with the entries staged, a
+// lane per column (csr_tile.cuh) and grabs of 4 items (8: 4.57, 16: 5.22 ms);
+// k = 16 3.06 -> 2.70 ms, k = 8 1.75 -> 1.72 ms.  Still bound by the latency of
+// the X gathers (nothing above half its rate).
 constexpr int64_t kTilesPerItem = 4;
+template <int G>
+constexpr int kBlockItems = G == 8 ? 4 : 8;
 
-template <typename I, typename V, int G>
+template <typename I, typename V, int G, bool kVec, bool kStage>
 __global__ void __launch_bounds__(kBatchBlock, 2) batch_tile_kernel(const BatchItem* __restrict__ items,
                                                                    int64_t nitems, const BatchMat* __restrict__ mats,
                                                                    V alpha, V beta, bool bz,
                                                                    unsigned long long* __restrict__ next_item) {
-  const int lane = threadIdx.x & 31;
-  unsigned long long grab = 0, ahead = 0;
-  if (lane == 0) {
-    grab = atomicAdd(next_item, (unsigned long long)kGrab);
-    ahead = atomicAdd(next_item, (unsigned long long)kGrab);
-  }
-  grab = __shfl_sync(0xffffffffu, grab, 0);
-  for (;;) {
-    if ((int64_t)grab >= nitems) break;
-    const int64_t jend = (int64_t)grab + kGrab < nitems ? (int64_t)grab + kGrab : nitems;
-    for (int64_t j = (int64_t)grab; j < jend; ++j) {
+  constexpr int kWarps = kBatchBlock / 32, kItems = kBlockItems<G>;
+  extern __shared__ __align__(16) unsigned char batch_tile_smem[];
+  using Tile = SpmmTile<I, V, G>;
+  __shared__ unsigned long long s_grab[2];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  Tile* S = reinterpret_cast<Tile*>(batch_tile_smem) + 2 * w;
+  if (threadIdx.x == 0) s_grab[0] = atomicAdd(next_item, (unsigned long long)kItems);
+  __syncthreads();
+  for (int turn = 0;; turn ^= 1) {
+    const int64_t grab = (int64_t)s_grab[turn];
+    if (grab >= nitems) break;
+    if (threadIdx.x == 0) s_grab[turn ^ 1] = atomicAdd(next_item, (unsigned long long)kItems);
+    // tile q of the grab: its matrix (null past the end) and number
+    auto tile_of = [&](int q, int64_t* t) -> const BatchMat* {
+      const int64_t j = grab + q / (int)kTilesPerItem;
+      if (q >= kItems * (int)kTilesPerItem || j >= nitems) return nullptr;
       const BatchItem it = items[j];
-      const BatchMat& M = mats[it.mat];
-      const int64_t t1 = it.idx + kTilesPerItem < M.tiles ? it.idx + kTilesPerItem : M.tiles;
-      for (int64_t t = it.idx; t < t1; ++t)
-        spmm_tile_groups<I, V, G>(static_cast<const I*>(M.rp), M.rows, M.nnz, static_cast<const I*>(M.ci),
-                                  static_cast<const V*>(M.val), M.tile_row, M.tflags, t, static_cast<const V*>(M.x),
-                                  M.ldx, static_cast<V*>(M.y), M.ldy, alpha, beta, bz, static_cast<V*>(M.tcin),
-                                  static_cast<V*>(M.tosum), M.topen, lane);
+      *t = it.idx + q % (int)kTilesPerItem;
+      return *t < mats[it.mat].tiles ? mats + it.mat : nullptr;
+    };
+    int64_t t = 0, tn = 0;
+    const BatchMat* M = tile_of(w, &t);
+    if constexpr (kStage) {
+      if (M) S[0].fetch(static_cast<const I*>(M->ci), static_cast<const V*>(M->val), M->nnz, t, lane);
+      cp_async_commit();
     }
-    grab = __shfl_sync(0xffffffffu, ahead, 0);
-    if (lane == 0 && (int64_t)grab < nitems) ahead = atomicAdd(next_item, (unsigned long long)kGrab);
+    for (int q = w, b = 0; q < kItems * (int)kTilesPerItem; q += kWarps, b ^= 1) {
+      const BatchMat* N = tile_of(q + kWarps, &tn);
+      if constexpr (kStage) {
+        if (N) S[b ^ 1].fetch(static_cast<const I*>(N->ci), static_cast<const V*>(N->val), N->nnz, tn, lane);
+        cp_async_commit();
+      }
+      if (M) {
+        const uint64_t fl = spmm_flags<G>(M->tflags, t, lane / G);
+        const int64_t tr = M->tile_row[t];
+        if constexpr (kStage) {
+          cp_async_wait<1>();
+          __syncwarp();
+        }
+        spmm_tile_groups<I, V, G, 4, kVec, kStage, true>(
+            S + b, fl, tr, static_cast<const I*>(M->ci), static_cast<const V*>(M->val), static_cast<const I*>(M->rp),
+            M->rows, M->nnz, t, static_cast<const V*>(M->x), M->ldx, 4 * G, static_cast<V*>(M->y), M->ldy, alpha, beta,
+            bz, static_cast<V*>(M->tcin), static_cast<V*>(M->tosum), M->topen, lane);
+      }
+      __syncwarp();  // S[b] is filled again in the next turn
+      M = N;
+      t = tn;
+    }
+    __syncthreads();  // the next grab is in; this one's slot may be rewritten
   }
 }
 
@@ -260,13 +297,13 @@ __global__ void batch_calibrate1_kernel(const int64_t* __restrict__ cal_off, con
                      M.topen, M.tempty, M.tnempty, static_cast<V*>(M.y), alpha, beta, bz);
 }
 
-// Calibration of every tile matrix: thread g takes entry g - cal_off[i] of
-// tile matrix i (its tiles, then its empty rows).
-template <typename V, int KC>
+// Calibration of every tile matrix: entry g / L - cal_off[i] of tile matrix i
+// (its tiles, then its empty rows) by L lanes.
+template <typename V>
 __global__ void batch_calibrate_kernel(const int64_t* __restrict__ cal_off, const int32_t* __restrict__ cal_mat,
-                                       int ncal, int64_t total, const BatchMat* __restrict__ mats, V alpha, V beta,
-                                       bool bz) {
-  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+                                       int ncal, int64_t total, int L, int k, const BatchMat* __restrict__ mats,
+                                       V alpha, V beta, bool bz) {
+  const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, g = gt / L;
   if (g >= total) return;
   int lo = 0, hi = ncal;  // last i with cal_off[i] <= g
   while (hi - lo > 1) {
@@ -274,8 +311,9 @@ __global__ void batch_calibrate_kernel(const int64_t* __restrict__ cal_off, cons
     if (cal_off[mid] <= g) lo = mid; else hi = mid;
   }
   const BatchMat& M = mats[cal_mat[lo]];
-  spmm_calibrate<V, KC>(g - cal_off[lo], M.tiles, static_cast<const V*>(M.tcin), static_cast<const V*>(M.tosum),
-                        M.topen, M.tempty, M.tnempty, static_cast<V*>(M.y), M.ldy, alpha, beta, bz);
+  spmm_calibrate<V>(g - cal_off[lo], (int)(gt % L), L, k, M.tiles, static_cast<const V*>(M.tcin),
+                    static_cast<const V*>(M.tosum), M.topen, M.tempty, M.tnempty, static_cast<V*>(M.y), M.ldy, alpha,
+                    beta, bz);
 }
 
 // Single-matrix SpMM over the CSR plan (the per-matrix path of spops_spmm).
@@ -369,10 +407,10 @@ spops_status_t csr_spmm(Context* ctx, Matrix* A, double alpha, const void* X, in
                         void* Y, int64_t ldy) {
   if (A->format != SPOPS_FMT_CSR) return fail(SPOPS_ERR_UNSUPPORTED, "SpMM needs a CSR matrix");
   if (!A->plan.ready) SPOPS_TRY(csr_analyse(ctx, A));
-  // k = 8, 16, 32 with X rows at most 2k wide: register tiles on the SpMV's
-  // plan.  (Passes of 8 columns over wider rows measured slower than the
-  // segment kernel: four passes at k = 32 took 20.5 ms against 6.5 ms on the
-  // power-law matrix.)
+  // k <= 32 with X rows at most 2k wide: register tiles on the SpMV's plan.
+  // (Passes of 8 columns over wider rows measured slower than the segment
+  // kernel: four passes at k = 32 took 20.5 ms against 6.5 ms on the power-law
+  // matrix.)
   if (ctx->csr_variant == 0) {
     bool used = false;
     SPOPS_TRY(csr_tile_spmm(ctx, A, alpha, X, ldx, k, beta, Y, ldy, &used));
@@ -558,42 +596,54 @@ spops_status_t launch_tiles1(Batch* B, double alpha, double beta, cudaStream_t s
   return SPOPS_OK;
 }
 
-template <typename I, typename V, int G>
-int tile_blocks_per_sm() {
-  static int cache[kMaxDevices];
-  return blocks_per_sm(batch_tile_kernel<I, V, G>, kBatchBlock, 0, cache);
+template <typename I, typename V, int G, bool kStage>
+constexpr size_t tile_smem() {
+  return !kStage ? 0 : 2 * (kBatchBlock / 32) * sizeof(SpmmTile<I, V, G>);
 }
 
-template <typename I, typename V, int G>
+template <typename I, typename V, int G, bool kVec, bool kStage>
+int tile_blocks_per_sm() {
+  static int cache[kMaxDevices];
+  return blocks_per_sm(batch_tile_kernel<I, V, G, kVec, kStage>, kBatchBlock, tile_smem<I, V, G, kStage>(), cache);
+}
+
+template <typename I, typename V, int G, bool kVec, bool kStage>
 spops_status_t launch_tiles(Batch* B, double alpha, double beta, cudaStream_t st) {
   const bool bz = beta == 0.0;
-  const int bps = tile_blocks_per_sm<I, V, G>();
+  const int bps = tile_blocks_per_sm<I, V, G, kVec, kStage>();
   if (bps < 1) return fail(SPOPS_ERR_CUDA, "batch: kernel attributes could not be set");
   int64_t grid = (int64_t)B->ctx->num_sms * bps;
-  const int64_t need = (B->ntitems + 7) / 8;
+  const int64_t need = (B->ntitems + kBlockItems<G> - 1) / kBlockItems<G>;
   if (grid > need) grid = need;
   SPOPS_CUDA(cudaMemsetAsync(B->tqueue.p, 0, 8, st));
-  batch_tile_kernel<I, V, G><<<(unsigned)grid, kBatchBlock, 0, st>>>(B->titems.as<BatchItem>(), B->ntitems,
+  batch_tile_kernel<I, V, G, kVec, kStage><<<(unsigned)grid, kBatchBlock, tile_smem<I, V, G, kStage>(), st>>>(B->titems.as<BatchItem>(), B->ntitems,
                                                                     B->table.as<BatchMat>(), (V)alpha, (V)beta, bz,
                                                                     B->tqueue.as<unsigned long long>());
   SPOPS_LAUNCH_CHECK();
   if (B->ncal_total > 0) {
-    batch_calibrate_kernel<V, 4 * G><<<(unsigned)((B->ncal_total + 255) / 256), 256, 0, st>>>(
-        B->cal_off.as<int64_t>(), B->cal_mat.as<int32_t>(), B->ncal, B->ncal_total, B->table.as<BatchMat>(),
-        (V)alpha, (V)beta, bz);
+    const int L = spmm_cal_lanes(4 * G);
+    batch_calibrate_kernel<V><<<(unsigned)((B->ncal_total * L + 255) / 256), 256, 0, st>>>(
+        B->cal_off.as<int64_t>(), B->cal_mat.as<int32_t>(), B->ncal, B->ncal_total, L, 4 * G,
+        B->table.as<BatchMat>(), (V)alpha, (V)beta, bz);
     SPOPS_LAUNCH_CHECK();
   }
   return SPOPS_OK;
 }
+
+// k = 32: a lane per column and staged entries for FP64, vector parts for FP32
+// (spmm_tiles_k).  k = 8 and 16 are not staged: with the table's pointers live
+// too the staged form spills (k = 16: 3.27 ms against 2.70 ms).
+template <typename V>
+constexpr bool kBatchVec32 = sizeof(V) == 4;
 
 template <typename I, typename V>
 spops_status_t launch_batch(Batch* B, double alpha, double beta, cudaStream_t st) {
   const bool bz = beta == 0.0;
   if (B->ntitems > 0) {  // tile items, then their calibration
     if (B->k == 1) SPOPS_TRY((launch_tiles1<I, V>(B, alpha, beta, st)));
-    else if (B->k == 8) SPOPS_TRY((launch_tiles<I, V, 2>(B, alpha, beta, st)));
-    else if (B->k == 16) SPOPS_TRY((launch_tiles<I, V, 4>(B, alpha, beta, st)));
-    else SPOPS_TRY((launch_tiles<I, V, 8>(B, alpha, beta, st)));
+    else if (B->k == 8) SPOPS_TRY((launch_tiles<I, V, 2, true, false>(B, alpha, beta, st)));
+    else if (B->k == 16) SPOPS_TRY((launch_tiles<I, V, 4, true, false>(B, alpha, beta, st)));
+    else SPOPS_TRY((launch_tiles<I, V, 8, kBatchVec32<V>, true>(B, alpha, beta, st)));
   }
   if (B->nitems == 0) return SPOPS_OK;
   auto go = [&](auto kern, size_t smem, int bps) -> spops_status_t {
@@ -693,7 +743,8 @@ spops_status_t prepare(Batch* B) {
       if (B->t_cin[m].bytes < bytes) SPOPS_TRY(B->t_cin[m].alloc(bytes));
       if (B->t_osum[m].bytes < bytes) SPOPS_TRY(B->t_osum[m].alloc(bytes));
       B->tile_ok[m] = 1;
-    } else if (csr_tile_spmm_usable(A, h.x, h.ldx, B->k) && h.ldy >= B->k) {
+    } else if ((B->k == 8 || B->k == 16 || B->k == 32) && csr_tile_spmm_usable(A, h.x, h.ldx, B->k) &&
+               csr_spmm_vector(h.x, h.ldx, B->k, vs) && h.ldy >= B->k) {
       if (!A->plan.tiles.ready || A->plan.tiles.k != 8) SPOPS_TRY(csr_tile_analyse(B->ctx, A, 8));
       const size_t bytes = (size_t)A->plan.tiles.tiles * (size_t)B->k * vs;
       if (B->t_cin[m].bytes < bytes) SPOPS_TRY(B->t_cin[m].alloc(bytes));

@@ -193,118 +193,239 @@ __device__ __forceinline__ void spmv_calibrate1(int64_t t, int64_t tiles, const 
   }
 }
 
-// ---- multi-RHS with k = 8, 16, 32 on the SpMV's tile plan (csr_tile_spmm
-// and the batch's tile items)
-template <typename V>
-__device__ __forceinline__ void axpby_store8(V* __restrict__ y, const V (&v)[8], V alpha, V beta, bool bz) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j) axpby_store(y + j, v[j], alpha, beta, bz);
+// ---- multi-RHS with up to 32 columns on the SpMV's tile plan
+// (csr_tile_spmm and the batch's tile items)
+//
+// One warp per tile, G lanes per entry: group q (lanes qG .. qG + G - 1) takes
+// the 8G consecutive entries of the plan's lanes qG .. qG + G - 1.  A lane
+// holds J columns of the result:
+//   kVec   columns 4h .. 4h + 3 of lane h (J = 4), an X row's part in one load
+//          of 32 (FP64) or 16 (FP32) bytes: k a multiple of 4, rows aligned
+//   else   columns h, h + G, ... (one load each): any k and alignment
+// so the group's lanes gather an entry's whole X row together and a row costs
+// one L2 request per 128 bytes.  Lanes past k load and store nothing.
+//
+// kStage: the tile's columns and values come through shared memory (SpmmTile),
+// copied there asynchronously a tile ahead.  What bounds the kernel is the
+// latency of dependent loads (column, then X row) at 16 warps per SM, with no
+// unit above half its rate; staged, a warp never waits for its entries before
+// it can ask for X rows, and the copies take no registers, which leaves room
+// for eight entries' X rows per lane, four arriving while four are summed.
+// Below eight lanes per entry or so the staging's own instructions weigh more
+// than that: those forms load a lane's eight entries into registers.  Which
+// form serves which k was measured (spmm_tiles_k).
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Half an X row (4 values) for the lane-pair form: 32 bytes for FP64, 16 for
-// FP32.
-template <typename V>
-__device__ __forceinline__ void ld_xhalf(const V* __restrict__ p, V (&r)[4]) {
-  if constexpr (sizeof(V) == 8) {
-    uint32_t w[8];
-    asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
-                 : "l"(p));
-    memcpy(r, w, 32);
+// A tile's columns and values; a group's share is set 16 bytes apart from the
+// next one's, so that the groups' broadcast reads use different banks.
+template <typename I, typename V, int G>
+struct alignas(16) SpmmTile {
+  static constexpr int NG = 32 / G, E = 8 * G;  // groups, entries of each
+  static constexpr int kColB = E * (int)sizeof(I) + 16, kValB = E * (int)sizeof(V) + 16;
+  unsigned char col[NG * kColB];
+  unsigned char val[NG * kValB];
+
+  // Starts the copy of tile t by one warp (entries past nnz come as zeros).
+  __device__ __forceinline__ void fetch(const I* __restrict__ ci, const V* __restrict__ v, int64_t nnz, int64_t t,
+                                        int lane) {
+    const int64_t e0 = t * 256;
+    const int64_t left = nnz - e0;
+    constexpr int CI = 16 / (int)sizeof(I), CV = 16 / (int)sizeof(V);  // entries per 16 bytes
+    const uint32_t dc = (uint32_t)__cvta_generic_to_shared(col), dv = (uint32_t)__cvta_generic_to_shared(val);
+#pragma unroll
+    for (int q = 0; q < 256 / CI / 32; ++q) {
+      const int e = (q * 32 + lane) * CI;
+      const int64_t m = left - e;
+      const int bytes = m >= CI ? 16 : m > 0 ? (int)m * (int)sizeof(I) : 0;
+      cp_async16(dc + (e / E) * kColB + (e % E) * (int)sizeof(I), bytes ? ci + e0 + e : ci, bytes);
+    }
+#pragma unroll
+    for (int q = 0; q < 256 / CV / 32; ++q) {
+      const int e = (q * 32 + lane) * CV;
+      const int64_t m = left - e;
+      const int bytes = m >= CV ? 16 : m > 0 ? (int)m * (int)sizeof(V) : 0;
+      cp_async16(dv + (e / E) * kValB + (e % E) * (int)sizeof(V), bytes ? v + e0 + e : v, bytes);
+    }
+  }
+  // four consecutive entries of group g
+  __device__ __forceinline__ void cols4(int g, int e, I (&c)[4]) const {
+    const uint4* p = reinterpret_cast<const uint4*>(col + g * kColB + e * (int)sizeof(I));
+#pragma unroll
+    for (int q = 0; q < (int)sizeof(I) / 4; ++q) {
+      const uint4 w = p[q];
+      memcpy(reinterpret_cast<char*>(c) + 16 * q, &w, 16);
+    }
+  }
+  __device__ __forceinline__ void vals4(int g, int e, V (&a)[4]) const {
+    const uint4* p = reinterpret_cast<const uint4*>(val + g * kValB + e * (int)sizeof(V));
+#pragma unroll
+    for (int q = 0; q < (int)sizeof(V) / 4; ++q) {
+      const uint4 w = p[q];
+      memcpy(reinterpret_cast<char*>(a) + 16 * q, &w, 16);
+    }
+  }
+};
+
+// A lane's part of an X row.
+template <typename V, int G, int J, bool kVec, bool kFull>
+__device__ __forceinline__ void ld_xpart(const V* __restrict__ p, int k, int h, V (&r)[J]) {
+  if constexpr (kVec) {
+    static_assert(J == 4, "vector parts hold four columns");
+    if constexpr (sizeof(V) == 8) {
+      uint32_t w[8];
+      asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                   : "l"(p + 4 * h));
+      memcpy(r, w, 32);
+    } else {
+      uint32_t w[4];
+      asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                   : "l"(p + 4 * h));
+      memcpy(r, w, 16);
+    }
   } else {
-    uint32_t w[4];
-    asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "l"(p));
-    memcpy(r, w, 16);
+#pragma unroll
+    for (int j = 0; j < J; ++j) r[j] = kFull || h + G * j < k ? ld_gather(p + h + G * j) : V(0);
   }
 }
 
-// One tile t of a multi-RHS product with k = 4G columns, G lanes per entry:
-// group q (lanes qG .. qG + G - 1) takes the 8G consecutive entries of the
-// plan's lanes qG .. qG + G - 1, lane qG + h holding columns 4h .. 4h + 3.
-// The group's lanes gather an entry's whole X row in one instruction (32
-// bytes each for FP64), so a row costs one L2 request per 128 bytes.  The
-// group's row starts are its G lanes' flags; the heads combine over the 32/G
-// groups with the segmented scan, and the row open at the tile's end goes to
-// the k-wide calibrator.  Every column is summed in an order fixed by the
-// matrix.
-template <typename I, typename V, int G>
-__device__ __forceinline__ void spmm_tile_groups(const I* __restrict__ rp, int64_t n, int64_t nnz,
+// Row-start flags of the 8G entries of group g of tile t (bit b: entry b).
+template <int G>
+__device__ __forceinline__ uint64_t spmm_flags(const uint8_t* __restrict__ flags_all, int64_t t, int g) {
+  const uint8_t* p = flags_all + t * 32 + g * G;
+  if constexpr (G == 8) return *reinterpret_cast<const uint64_t*>(p);
+  else if constexpr (G == 4) return *reinterpret_cast<const uint32_t*>(p);
+  else if constexpr (G == 2) return *reinterpret_cast<const uint16_t*>(p);
+  else return *p;
+}
+
+// One tile t whose entries are in S.  The group's row starts are its G lanes'
+// flags; the heads combine over the 32/G groups with the segmented scan, and
+// the row open at the tile's end goes to the k-wide calibrator (carry_in and
+// open_sum hold k values per tile).  Every column is summed in an order fixed
+// by the matrix and k.
+// kFull: k == G * J, no column of any lane lies past k.
+template <typename I, typename V, int G, int J, bool kVec, bool kStage, bool kFull>
+__device__ __forceinline__ void spmm_tile_groups(const SpmmTile<I, V, G>* S, uint64_t fl, int64_t tr,
                                                  const I* __restrict__ ci, const V* __restrict__ val,
-                                                 const int64_t* __restrict__ tile_row,
-                                                 const uint8_t* __restrict__ flags_all, int64_t t,
-                                                 const V* __restrict__ X, int64_t ldx, V* __restrict__ Y, int64_t ldy,
-                                                 V alpha, V beta, bool bz, V* __restrict__ carry_in,
+                                                 const I* __restrict__ rp, int64_t n, int64_t nnz, int64_t t,
+                                                 const V* __restrict__ X, int64_t ldx, int k, V* __restrict__ Y,
+                                                 int64_t ldy, V alpha, V beta, bool bz, V* __restrict__ carry_in,
                                                  V* __restrict__ open_sum, int64_t* __restrict__ open_row, int lane) {
-  constexpr int K = 8, NG = 32 / G, KC = 4 * G;
-  static_assert(G == 2 || G == 4 || G == 8, "2, 4 or 8 lanes per entry");
+  constexpr int NG = 32 / G, E = 8 * G;
+  static_assert(G == 1 || G == 2 || G == 4 || G == 8, "1, 2, 4 or 8 lanes per entry");
   const int gq = lane / G, h = lane % G;
-  uint64_t fl = 0;  // bit b: entry b of the group's 8G starts a row
-#pragma unroll
-  for (int r = 0; r < G; ++r) fl |= (uint64_t)flags_all[t * 32 + gq * G + r] << (8 * r);
-  const int64_t tr = tile_row[t];
-  const int64_t e0 = t * (32 * K) + (int64_t)gq * G * K;
+  const bool active = kFull || (kVec ? 4 * h : h) < k;  // some column of this lane is below k
+  const int64_t e0 = t * 256 + (int64_t)gq * E;
+  const int real = nnz - e0 >= E ? E : nnz > e0 ? (int)(nnz - e0) : 0;  // entries of the group inside the matrix
   // group flags as an NG-bit mask (bit q: group q holds a row start)
   const unsigned lane_f = __ballot_sync(0xffffffffu, fl != 0 && h == 0);
   unsigned gf = 0;
+  if constexpr (G == 1) {
+    gf = lane_f;
+  } else {
 #pragma unroll
-  for (int q = 0; q < NG; ++q) gf |= ((lane_f >> (G * q)) & 1u) << q;
+    for (int q = 0; q < NG; ++q) gf |= ((lane_f >> (G * q)) & 1u) << q;
+  }
   int64_t row;
   if (tr >= 0) {
     const int cnt = __popcll(fl);
-    const unsigned below = (gq * G >= 32) ? 0xffffffffu : ((1u << (gq * G)) - 1u);  // lanes of earlier groups
+    const unsigned below = (1u << (gq * G)) - 1u;  // lanes of earlier groups
     int excl = 0;
 #pragma unroll
-    for (int bit = 0; bit < 7; ++bit)
+    for (int bit = 0; (1 << bit) <= E; ++bit)
       excl += __popc(__ballot_sync(0xffffffffu, ((cnt >> bit) & 1) && h == 0) & below) << bit;
     const int first0 = (int)(__ballot_sync(0xffffffffu, fl & 1u) & 1u);
     row = tr + excl + (int)(fl & 1u) - first0;
   } else {
     row = row_holding(rp, n, e0 < nnz ? e0 : nnz - 1);
   }
-  V acc[4], head[4];
+  auto column = [&](int j) { return kVec ? 4 * h + j : h + G * j; };
+  auto has = [&](int j) { return kFull || column(j) < k; };
+  V acc[J], head[J];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) acc[j] = head[j] = V(0);
+  for (int j = 0; j < J; ++j) acc[j] = head[j] = V(0);
   bool in_head = (fl & 1u) == 0;
-  V* Yh = Y + 4 * h;
+  // X rows of four entries (entries past nnz have column 0; they are not added)
+  auto gather = [&](const I (&c)[4], V (&x)[4][J]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (active) ld_xpart<V, G, J, kVec, kFull>(X + (int64_t)c[q] * ldx, k, h, x[q]);
+  };
+  auto add = [&](int e, const V (&a)[4], const V (&x)[4][J]) {
+    const unsigned f4 = (unsigned)(fl >> e) & 15u;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (((f4 >> q) & 1u) && e + q > 0) {
+        if (in_head) {
+#pragma unroll
+          for (int j = 0; j < J; ++j) head[j] = acc[j];
+          in_head = false;
+        } else {
+#pragma unroll
+          for (int j = 0; j < J; ++j)
+            if (has(j)) axpby_store(Y + row * ldy + column(j), acc[j], alpha, beta, bz);
+        }
+#pragma unroll
+        for (int j = 0; j < J; ++j) acc[j] = V(0);
+        ++row;
+        if (tr < 0)
+          while (row + 1 < n && rp[row] == rp[row + 1]) ++row;  // skip empty rows
+      }
+      if (e + q < real) {
+#pragma unroll
+        for (int j = 0; j < J; ++j) acc[j] += a[q] * x[q][j];
+      }
+    }
+  };
+  if constexpr (kStage) {
+    V x0[4][J], x1[4][J], a[4];
+    I c[4];
+    S->cols4(gq, 0, c);
+    gather(c, x0);
 #pragma unroll 1
-  for (int run = 0; run < G; ++run) {  // plan lanes qG, qG + 1, ...
-    I c[K];
-    V a[K];
-    tile_load<I, V, K>(ci, val, nnz, t, gq * G + run, c, a);
+    for (int e = 0; e < E; e += 8) {
+      S->cols4(gq, e + 4, c);
+      gather(c, x1);
+      S->vals4(gq, e, a);
+      add(e, a, x0);
+      if (e + 8 < E) {
+        S->cols4(gq, e + 8, c);
+        gather(c, x0);
+      }
+      S->vals4(gq, e + 4, a);
+      add(e + 4, a, x1);
+    }
+  } else {
+#pragma unroll 1
+    for (int e = 0; e < E; e += 8) {
+      I c[8], c4[4];
+      V a[8], a4[4], x[4][J];
+      tile_load<I, V, 8>(ci, val, nnz, t, gq * G + e / 8, c, a);
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      V xr[4][4];
+      for (int half = 0; half < 8; half += 4) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) ld_xhalf(X + (int64_t)c[4 * half + q] * ldx + 4 * h, xr[q]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int b = run * K + 4 * half + q;
-        if (b > 0 && ((fl >> b) & 1u)) {
-          if (in_head) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) head[j] = acc[j];
-            in_head = false;
-          } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) axpby_store(Yh + row * ldy + j, acc[j], alpha, beta, bz);
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[j] = V(0);
-          ++row;
-          if (tr < 0)
-            while (row + 1 < n && rp[row] == rp[row + 1]) ++row;  // skip empty rows
+        for (int q = 0; q < 4; ++q) {
+          c4[q] = c[half + q];
+          a4[q] = a[half + q];
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const V prod = a[4 * half + q] * xr[q][j];
-          acc[j] += prod;
-        }
+        gather(c4, x);
+        add(e + half, a4, x);
       }
     }
   }
-  V tail[4];
+  V tail[J];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < J; ++j) {
     if (in_head) head[j] = acc[j];
     tail[j] = in_head ? V(0) : acc[j];
   }
@@ -313,64 +434,71 @@ __device__ __forceinline__ void spmm_tile_groups(const I* __restrict__ rp, int64
 #pragma unroll
   for (int o = 1; o < NG; o <<= 1) {
     const unsigned span = (gq >= o) ? ((2u << gq) - 1u) & ~((2u << (gq - o)) - 1u) : 0u;
-    const bool add = gq >= o && !(starts & span);
+    const bool more = gq >= o && !(starts & span);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < J; ++j) {
       const V su = __shfl_up_sync(0xffffffffu, head[j], G * o);
-      if (add) head[j] += su;
+      if (more) head[j] += su;
     }
   }
   const unsigned later = gf & ~((2u << gq) - 1u);
   const int m = later ? __ffs(later) - 1 : NG - 1;
   const int m0 = gf ? __ffs(gf) - 1 : NG - 1;
-  V Sm[4], cin[4];
+  V Sm[J], cin[J];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < J; ++j) {
     Sm[j] = __shfl_sync(0xffffffffu, head[j], G * m + h);
     cin[j] = __shfl_sync(0xffffffffu, head[j], G * m0 + h);
   }
   if (has_flag) {
     if (later) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) axpby_store(Yh + row * ldy + j, tail[j] + Sm[j], alpha, beta, bz);
+      for (int j = 0; j < J; ++j)
+        if (has(j)) axpby_store(Y + row * ldy + column(j), tail[j] + Sm[j], alpha, beta, bz);
     } else {  // the tile's last row: may continue into the next tile
 #pragma unroll
-      for (int j = 0; j < 4; ++j) open_sum[t * KC + 4 * h + j] = tail[j] + (gq < NG - 1 ? Sm[j] : V(0));
+      for (int j = 0; j < J; ++j)
+        if (has(j)) open_sum[t * k + column(j)] = tail[j] + (gq < NG - 1 ? Sm[j] : V(0));
       if (h == 0) open_row[t] = row;
     }
   }
   if (gq == 0) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) carry_in[t * KC + 4 * h + j] = cin[j];
+    for (int j = 0; j < J; ++j)
+      if (has(j)) carry_in[t * k + column(j)] = cin[j];
     if (h == 0 && !gf) open_row[t] = -1;
   }
 }
 
+// Lanes per tile of the k-wide calibration: the power of two from k, at most a
+// warp (a lane per column: whole lines of carry_in, open_sum and Y).
+__host__ __device__ __forceinline__ int spmm_cal_lanes(int64_t k) {
+  int L = 1;
+  while (L < 32 && L < k) L <<= 1;
+  return L;
+}
+
 // Calibration of one tile t (t < tiles) or empty row (t - tiles < nempty)
-// of a product with KC columns (8 at a time).
-template <typename V, int KC>
-__device__ __forceinline__ void spmm_calibrate(int64_t t, int64_t tiles, const V* __restrict__ carry_in,
-                                               const V* __restrict__ open_sum, const int64_t* __restrict__ open_row,
+// of a product with k columns; this lane takes columns sub, sub + L, ...
+template <typename V>
+__device__ __forceinline__ void spmm_calibrate(int64_t t, int sub, int L, int k, int64_t tiles,
+                                               const V* __restrict__ carry_in, const V* __restrict__ open_sum,
+                                               const int64_t* __restrict__ open_row,
                                                const int64_t* __restrict__ empty, int64_t nempty, V* __restrict__ Y,
                                                int64_t ldy, V alpha, V beta, bool bz) {
-  V tot[8];
   if (t < tiles) {
     const int64_t r = open_row[t];
     if (r < 0) return;
-    for (int c0 = 0; c0 < KC; c0 += 8) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) tot[j] = open_sum[t * KC + c0 + j];
+    for (int c = sub; c < k; c += L) {
+      V tot = open_sum[t * k + c];
       for (int64_t u = t + 1; u < tiles; ++u) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) tot[j] += carry_in[u * KC + c0 + j];
+        tot += carry_in[u * k + c];
         if (open_row[u] >= 0) break;
       }
-      axpby_store8(Y + r * ldy + c0, tot, alpha, beta, bz);
+      axpby_store(Y + r * ldy + c, tot, alpha, beta, bz);
     }
   } else if (t - tiles < nempty) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) tot[j] = V(0);
-    for (int c0 = 0; c0 < KC; c0 += 8) axpby_store8(Y + empty[t - tiles] * ldy + c0, tot, alpha, beta, bz);
+    for (int c = sub; c < k; c += L) axpby_store(Y + empty[t - tiles] * ldy + c, V(0), alpha, beta, bz);
   }
 }
 

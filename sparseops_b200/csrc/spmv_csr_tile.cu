@@ -388,71 +388,134 @@ __global__ void csr_tile_calibrate_kernel(int64_t t_begin, int64_t tiles, const 
   }
 }
 
-// ---- multi-RHS with k = 4G on the same tile plan (csr_tile_spmm); the
+// ---- multi-RHS with k <= 32 on the same tile plan (csr_tile_spmm); the
 // per-tile work is spmm_tile_groups (csr_tile.cuh)
-template <typename I, typename V, int G>
+template <typename I, typename V, int G, int J, bool kVec, bool kStage, bool kFull>
 __global__ void __launch_bounds__(kTileBlock, 2) csr_tile_spmm_kernel(
     const I* __restrict__ rp, int64_t n, int64_t nnz, const I* __restrict__ ci, const V* __restrict__ val,
     const int64_t* __restrict__ tile_row, const uint8_t* __restrict__ flags_all, int64_t tiles,
-    const V* __restrict__ X, int64_t ldx, V* __restrict__ Y, int64_t ldy, V alpha, V beta, bool bz,
+    const V* __restrict__ X, int64_t ldx, int k, V* __restrict__ Y, int64_t ldy, V alpha, V beta, bool bz,
     V* __restrict__ carry_in, V* __restrict__ open_sum, int64_t* __restrict__ open_row) {
+  extern __shared__ __align__(16) unsigned char spmm_smem[];
+  using Tile = SpmmTile<I, V, G>;
   const int lane = threadIdx.x & 31;
+  if (kFull) k = G * J;
+  Tile* S = reinterpret_cast<Tile*>(spmm_smem) + 2 * (threadIdx.x >> 5);
   const int64_t nw = (int64_t)gridDim.x * (kTileBlock / 32);
-  for (int64_t t = blockIdx.x * (int64_t)(kTileBlock / 32) + (threadIdx.x >> 5); t < tiles; t += nw)
-    spmm_tile_groups<I, V, G>(rp, n, nnz, ci, val, tile_row, flags_all, t, X, ldx, Y, ldy, alpha, beta, bz,
-                              carry_in, open_sum, open_row, lane);
+  int64_t t = blockIdx.x * (int64_t)(kTileBlock / 32) + (threadIdx.x >> 5);
+  if (t >= tiles) return;
+  if constexpr (kStage) {
+    S[0].fetch(ci, val, nnz, t, lane);
+    cp_async_commit();
+  }
+  for (int b = 0; t < tiles; t += nw, b ^= 1) {
+    const uint64_t fl = spmm_flags<G>(flags_all, t, lane / G);
+    const int64_t tr = tile_row[t];
+    if constexpr (kStage) {
+      if (t + nw < tiles) S[b ^ 1].fetch(ci, val, nnz, t + nw, lane);
+      cp_async_commit();
+      cp_async_wait<1>();
+      __syncwarp();
+    }
+    spmm_tile_groups<I, V, G, J, kVec, kStage, kFull>(S + b, fl, tr, ci, val, rp, n, nnz, t, X, ldx, k, Y, ldy, alpha, beta, bz, carry_in,
+                                       open_sum, open_row, lane);
+    __syncwarp();  // S[b] is filled again in the next turn
+  }
 }
 
-template <typename V, int KC>
-__global__ void csr_tile_calibrate_k_kernel(int64_t tiles, const V* __restrict__ carry_in,
+template <typename V>
+__global__ void csr_tile_calibrate_k_kernel(int L, int k, int64_t tiles, const V* __restrict__ carry_in,
                                             const V* __restrict__ open_sum, const int64_t* __restrict__ open_row,
                                             const int64_t* __restrict__ empty, int64_t nempty, V* __restrict__ Y,
                                             int64_t ldy, V alpha, V beta, bool bz) {
-  spmm_calibrate<V, KC>(blockIdx.x * (int64_t)blockDim.x + threadIdx.x, tiles, carry_in, open_sum, open_row, empty,
-                        nempty, Y, ldy, alpha, beta, bz);
+  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  spmm_calibrate<V>(g / L, (int)(g % L), L, k, tiles, carry_in, open_sum, open_row, empty, nempty, Y, ldy, alpha,
+                    beta, bz);
 }
 
-template <typename I, typename V, int G>
-spops_status_t spmm_tiles_t(Context* ctx, Matrix* A, double alpha, const void* X, int64_t ldx, double beta, void* Y,
-                            int64_t ldy) {
-  constexpr int KC = 4 * G;
+template <typename I, typename V, int G, int J, bool kVec, bool kStage, bool kFull>
+spops_status_t spmm_tiles_f(Context* ctx, Matrix* A, double alpha, const void* X, int64_t ldx, int64_t k,
+                            double beta, void* Y, int64_t ldy) {
   const CsrTiles& D = A->plan.tiles;
   const bool bz = beta == 0.0;
   PoolBuf cin(ctx), osum(ctx);
   const size_t nt1 = (size_t)(D.tiles > 0 ? D.tiles : 1);
-  SPOPS_TRY(cin.alloc(nt1 * KC * sizeof(V)));
-  SPOPS_TRY(osum.alloc(nt1 * KC * sizeof(V)));
+  SPOPS_TRY(cin.alloc(nt1 * (size_t)k * sizeof(V)));
+  SPOPS_TRY(osum.alloc(nt1 * (size_t)k * sizeof(V)));
   if (D.tiles > 0) {
+    auto* kern = csr_tile_spmm_kernel<I, V, G, J, kVec, kStage, kFull>;
+    constexpr size_t smem = !kStage ? 0 : 2 * (kTileBlock / 32) * sizeof(SpmmTile<I, V, G>);
     static int blocks_per_sm = -1;  // per instantiation
     if (blocks_per_sm < 0) {
       int bps = 0;
-      SPOPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, csr_tile_spmm_kernel<I, V, G>, kTileBlock, 0));
+      SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      SPOPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, kTileBlock, smem));
       blocks_per_sm = bps > 0 ? bps : 1;
     }
     int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
     const int64_t need = (D.tiles + kTileBlock / 32 - 1) / (kTileBlock / 32);
     if (grid > need) grid = need;
-    csr_tile_spmm_kernel<I, V, G><<<(unsigned)grid, kTileBlock, 0, ctx->stream>>>(
+    kern<<<(unsigned)grid, kTileBlock, smem, ctx->stream>>>(
         A->row.as<I>(), A->rows, A->nnz, A->col.as<I>(), A->val.as<V>(), D.tile_row.as<int64_t>(),
-        D.flags.as<uint8_t>(), D.tiles, static_cast<const V*>(X), ldx, static_cast<V*>(Y), ldy, (V)alpha, (V)beta,
-        bz, cin.as<V>(), osum.as<V>(), D.open_row.as<int64_t>());
+        D.flags.as<uint8_t>(), D.tiles, static_cast<const V*>(X), ldx, (int)k, static_cast<V*>(Y), ldy, (V)alpha,
+        (V)beta, bz, cin.as<V>(), osum.as<V>(), D.open_row.as<int64_t>());
     SPOPS_LAUNCH_CHECK();
   }
   if (D.tiles + D.nempty > 0) {
-    csr_tile_calibrate_k_kernel<V, KC><<<grid_of(D.tiles + D.nempty), 256, 0, ctx->stream>>>(
-        D.tiles, cin.as<V>(), osum.as<V>(), D.open_row.as<int64_t>(), D.empty.as<int64_t>(), D.nempty,
+    const int L = spmm_cal_lanes(k);
+    csr_tile_calibrate_k_kernel<V><<<grid_of((D.tiles + D.nempty) * L), 256, 0, ctx->stream>>>(
+        L, (int)k, D.tiles, cin.as<V>(), osum.as<V>(), D.open_row.as<int64_t>(), D.empty.as<int64_t>(), D.nempty,
         static_cast<V*>(Y), ldy, (V)alpha, (V)beta, bz);
     SPOPS_LAUNCH_CHECK();
   }
   return SPOPS_OK;
 }
 
+template <typename I, typename V, int G, int J, bool kVec, bool kStage>
+spops_status_t spmm_tiles_t(Context* ctx, Matrix* A, double alpha, const void* X, int64_t ldx, int64_t k,
+                            double beta, void* Y, int64_t ldy) {
+  if (k == G * J) return spmm_tiles_f<I, V, G, J, kVec, kStage, true>(ctx, A, alpha, X, ldx, k, beta, Y, ldy);
+  return spmm_tiles_f<I, V, G, J, kVec, kStage, false>(ctx, A, alpha, X, ldx, k, beta, Y, ldy);
+}
+
+// Lanes per entry, columns per lane, vector parts and staging by k, each the
+// fastest measured on the 300,007-row power-law and a 1,000,000-row banded
+// matrix (us, FP64 | FP32; the segment kernel that served k other than 8, 16
+// and 32 took 235 | 195, 443 | 364, 679 | 530, 1031 | 700 at k = 2, 12, 24, 31
+// on the first):
+//   k = 2   2 x 1            56, 98     | 45, 83
+//   k = 3   2 x 2 staged     72, 136    | 58, 96
+//   k = 4   1 x 4 vector     68, 124    | 50, 74
+//   k = 5   2 x 3 staged     89, 167    | 71, 134   (FP32 not staged: 68, 123)
+//   k = 8   2 x 4 vector     92, 210    | 56, 105   (4 x 2 staged: 96, 211 | 69, 138)
+//   k = 12  4 x 3 staged    113, 251    | 88, 195   (FP32 vector: 76, 176)
+//   k = 16  4 x 4 vector    143, 336    | 77, 186   (FP64 staged; else staged 159, 324 | 114, 240)
+//   k = 24  8 x 3 staged    178, 414    | 144, 347  (FP32 vector staged: 129, 329)
+//   k = 32  8 x 4 staged    215, 476    | 161, 375  (FP32 vector staged: 130, 330; FP64: 246, 559)
+// A lane per column reads an FP64 row of 17 columns or more faster than a lane
+// per four: the group's eight loads are whole 64-byte pieces.
 template <typename I, typename V>
 spops_status_t spmm_tiles_k(Context* ctx, Matrix* A, double alpha, const void* X, int64_t ldx, int64_t k,
                             double beta, void* Y, int64_t ldy) {
-  if (k == 8) return spmm_tiles_t<I, V, 2>(ctx, A, alpha, X, ldx, beta, Y, ldy);
-  if (k == 16) return spmm_tiles_t<I, V, 4>(ctx, A, alpha, X, ldx, beta, Y, ldy);
-  return spmm_tiles_t<I, V, 8>(ctx, A, alpha, X, ldx, beta, Y, ldy);
+#define SPOPS_SPMM(G, J, VEC, STAGE) return spmm_tiles_t<I, V, G, J, VEC, STAGE>(ctx, A, alpha, X, ldx, k, beta, Y, ldy)
+  constexpr bool f64 = sizeof(V) == 8;
+  const bool vec = csr_spmm_vector(X, ldx, k, sizeof(V));
+  if (vec && k == 4) SPOPS_SPMM(1, 4, true, false);
+  if (vec && k == 8) SPOPS_SPMM(2, 4, true, false);
+  if (vec && k == 16) SPOPS_SPMM(4, 4, true, f64);
+  if constexpr (!f64) {
+    if (vec && k == 12) SPOPS_SPMM(4, 4, true, false);
+    if (vec && k > 16) SPOPS_SPMM(8, 4, true, true);
+  }
+  if (k <= 2) SPOPS_SPMM(2, 1, false, false);
+  if (k <= 4) SPOPS_SPMM(2, 2, false, true);
+  if (k <= 6) SPOPS_SPMM(2, 3, false, f64);
+  if (k <= 8) SPOPS_SPMM(4, 2, false, true);
+  if (k <= 12) SPOPS_SPMM(4, 3, false, true);
+  if (k <= 16) SPOPS_SPMM(4, 4, false, true);
+  if (k <= 24) SPOPS_SPMM(8, 3, false, true);
+  SPOPS_SPMM(8, 4, false, true);
+#undef SPOPS_SPMM
 }
 
 // Boundaries of `parts` tile ranges for the pipelined host SpMV: range p
@@ -488,12 +551,12 @@ spops_status_t analyse_t(Context* ctx, Matrix* A) {
   D.k = K;
   D.tiles = tiles_of<K>(nnz);
   const size_t nt1 = (size_t)(D.tiles > 0 ? D.tiles : 1);
-  SPOPS_TRY(D.tile_row.alloc(nt1 * 8));
-  SPOPS_TRY(D.flags.alloc(nt1 * 32));
-  SPOPS_TRY(D.carry_in.alloc(nt1 * 8));
-  SPOPS_TRY(D.open_sum.alloc(nt1 * 8));
-  SPOPS_TRY(D.open_row.alloc(nt1 * 8));
-  SPOPS_TRY(D.empty.alloc((size_t)(n > 0 ? n : 1) * 8));
+  SPOPS_TRY(D.tile_row.alloc_cached(ctx, nt1 * 8, kBuildCacheMax));
+  SPOPS_TRY(D.flags.alloc_cached(ctx, nt1 * 32, kBuildCacheMax));
+  SPOPS_TRY(D.carry_in.alloc_cached(ctx, nt1 * 8, kBuildCacheMax));
+  SPOPS_TRY(D.open_sum.alloc_cached(ctx, nt1 * 8, kBuildCacheMax));
+  SPOPS_TRY(D.open_row.alloc_cached(ctx, nt1 * 8, kBuildCacheMax));
+  SPOPS_TRY(D.empty.alloc_cached(ctx, (size_t)(n > 0 ? n : 1) * 8, kBuildCacheMax));
   if (D.tiles > 0 && n > 0) {
     tile_build_kernel<I, K><<<grid_of(D.tiles), 256, 0, st>>>(A->row.as<I>(), n, nnz, D.tiles,
                                                                 D.tile_row.as<int64_t>(), D.flags.as<uint8_t>());
@@ -702,17 +765,26 @@ spops_status_t csr_tile_spmv_parts(Context* ctx, Matrix* A, int parts, double al
   return spmv_parts_t<int64_t, float>(ctx, A, alpha, x, beta, y, D.part_tb, D.part_rb, done);
 }
 
+bool csr_spmm_vector(const void* X, int64_t ldx, int64_t k, size_t vs) {
+  return k % 4 == 0 && (uintptr_t)X % (4 * vs) == 0 && ldx % 4 == 0;
+}
+
 bool csr_tile_spmm_usable(const Matrix* A, const void* X, int64_t ldx, int64_t k) {
-  const size_t vs = A->vsize();
-  return (k == 8 || k == 16 || k == 32) && A->rows > 0 && A->nnz > 0 && csr_tile_usable(A, 0) &&
-         ((uintptr_t)X % 32) == 0 && ((size_t)ldx * vs) % 32 == 0 && ldx >= k && ldx <= 2 * k;
+  // X rows at most 2k wide: passes over wider rows were not measured
+  return k >= 1 && k <= 32 && A->rows > 0 && A->nnz > 0 && csr_tile_usable(A, 0) &&
+         (uintptr_t)X % A->vsize() == 0 && ldx >= k && ldx <= 2 * k;
 }
 
 spops_status_t csr_tile_spmm(Context* ctx, Matrix* A, double alpha, const void* X, int64_t ldx, int64_t k,
                              double beta, void* Y, int64_t ldy, bool* used) {
   *used = false;
   if (!csr_tile_spmm_usable(A, X, ldx, k) || ldy < k) return SPOPS_OK;
-  if (!A->plan.tiles.ready || A->plan.tiles.k != 8) SPOPS_TRY(csr_tile_analyse(ctx, A, 8));
+  if (!A->plan.tiles.ready || A->plan.tiles.k != 8) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    SPOPS_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return SPOPS_OK;  // the plan cannot be built inside a capture
+    SPOPS_TRY(csr_tile_analyse(ctx, A, 8));
+  }
   *used = true;
   const bool i32 = A->itype == SPOPS_INDEX_I32, f64 = A->vtype == SPOPS_VALUE_F64;
   if (i32 && f64) return spmm_tiles_k<int32_t, double>(ctx, A, alpha, X, ldx, k, beta, Y, ldy);

@@ -524,6 +524,8 @@ bool csr_tile_usable(const Matrix* A, int variant);
 // tile plan (k / 4 lanes per entry); *used = false (nothing done) unless the
 // matrix and X allow its vector loads and X's row stride is at most 2k.
 bool csr_tile_spmm_usable(const Matrix* A, const void* X, int64_t ldx, int64_t k);
+// X's rows can be read four columns at a time (vs: bytes of a value)
+bool csr_spmm_vector(const void* X, int64_t ldx, int64_t k, size_t vs);
 spops_status_t csr_tile_spmm(Context* ctx, Matrix* A, double alpha, const void* X, int64_t ldx, int64_t k,
                              double beta, void* Y, int64_t ldy, bool* used);
 spops_status_t csr_tile_analyse(Context* ctx, Matrix* A, int k);

@@ -244,3 +244,41 @@ def test_batch_k8_tiles_mixed_and_replayed(cuda, orc):
         X = Xd.cpu().numpy()
         ref = orc.spmm_csr(rp, ci, v, X)
         assert _err(orc, rp, ci, v, X, Y, ref, 1.0, 0.0, np.zeros_like(Y)) <= 1e-12
+
+
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 6, 7, 8, 9, 12, 13, 16, 17, 20, 24, 25, 31, 32])
+def test_spmm_every_form(cuda, orc, k, f32):
+    """SpMM at the column counts where the tile kernel changes its form, X
+    aligned, in rows of an odd stride, and one element off its allocation, on
+    empty rows, a row over several tiles and an nnz that ends inside a tile;
+    infinities in X rows that no entry reads stay out."""
+    import torch
+    from sparseops_b200 import CSR_Matrix, SpMM_csr
+    rng = np.random.default_rng(k)
+    n, cols = 700, 640
+    lens = rng.integers(0, 12, n)
+    lens[[3, 4, 5, 690, 699]] = 0
+    lens[100] = 600
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    if rp[-1] % 8 == 0:  # end inside a lane's run
+        lens[50] += 3
+        rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = np.concatenate([np.sort(rng.choice(np.arange(1, cols), m, replace=False)) for m in lens]).astype(np.int32)
+    dt = np.float32 if f32 else np.float64
+    v = rng.standard_normal(len(ci)).astype(dt)
+    A = CSR_Matrix(n, cols, *(torch.from_numpy(a).to("cuda") for a in (rp, ci, v)))
+    X = rng.uniform(-1, 1, (cols, k)).astype(dt)
+    X[0] = np.inf  # column 0 has no entry
+    Y0 = rng.standard_normal((n, k)).astype(dt)
+    Xf = np.where(np.isinf(X), 0, X).astype(np.float64)
+    ref = orc.spmm_csr(rp, ci, v.astype(np.float64), Xf, 0.8, 0.7, Y0.astype(np.float64))
+    den = 0.8 * orc.spmm_csr(rp, ci, np.abs(v).astype(np.float64), np.abs(Xf)) + 0.7 * np.abs(Y0) + 1e-300
+    for ld, off in ((k, 0), (min(k + 1, 2 * k), 0), (k, 1)):
+        buf = torch.zeros(cols * ld + 8, dtype=torch.float32 if f32 else torch.float64, device="cuda")
+        Xd = buf[off:off + cols * ld].view(cols, ld)[:, :k]
+        Xd.copy_(torch.from_numpy(X))
+        Y = torch.from_numpy(Y0).to("cuda").clone()
+        SpMM_csr(0.8, A, Xd, 0.7, Y)
+        err = np.abs(Y.cpu().numpy().astype(np.float64) - ref) / den
+        assert err.max() <= (1e-5 if f32 else 1e-12), (ld, off)
