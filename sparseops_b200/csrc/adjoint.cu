@@ -18,6 +18,7 @@
 
 #include "csr_tile.cuh"
 #include "device_util.cuh"
+#include "pdl.cuh"
 #include "spops_internal.h"
 
 namespace spops {
@@ -346,6 +347,7 @@ __global__ void __launch_bounds__(256) sddmm_tile_kernel(const I* __restrict__ r
                                                          const uint8_t* __restrict__ flags_all, int64_t tiles,
                                                          const V* __restrict__ g, const V* __restrict__ x,
                                                          V* __restrict__ out, V alpha, bool vec_out) {
+  overlap_begin();
   constexpr int K = 8;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;  // lanes below this one
@@ -420,10 +422,10 @@ spops_status_t sddmm_t(Context* ctx, Matrix* A, double alpha, const void* g, con
     const int64_t need = (D.tiles + 7) / 8;
     if (grid > need) grid = need;
     if (grid > 0) {
-      sddmm_tile_kernel<I, V><<<(unsigned)grid, 256, 0, ctx->stream>>>(
-          A->row.as<I>(), A->rows, A->nnz, A->col.as<I>(), D.tile_row.as<int64_t>(), D.flags.as<uint8_t>(), D.tiles,
+      SPOPS_CUDA(launch_overlapped(sddmm_tile_kernel<I, V>, grid, 256, 0, ctx->stream,
+        A->row.as<I>(), A->rows, A->nnz, A->col.as<I>(), D.tile_row.as<int64_t>(), D.flags.as<uint8_t>(), D.tiles,
           static_cast<const V*>(g), static_cast<const V*>(x), static_cast<V*>(out), (V)alpha,
-          ((uintptr_t)out % 32) == 0);
+          ((uintptr_t)out % 32) == 0));
       SPOPS_LAUNCH_CHECK();
     }
     return SPOPS_OK;

@@ -96,14 +96,22 @@ __device__ __forceinline__ void tile_load(const I* __restrict__ ci, const V* __r
   }
 }
 
+// What is left of a tile when its complete rows have gone to y.
+template <typename V>
+struct TileEnds {
+  bool owner;    // this lane holds the row open at the tile's end
+  bool any;      // some row starts in the tile
+  int64_t row;   // owner: that row
+  V open;        // owner: its sum so far
+  V cin;         // the entries before the tile's first row start (all lanes)
+};
+
 // Given the products p of the lane's run: rows complete inside the lane go to
-// y, the heads combine across lanes, the tile's open row and carry go to the
-// calibrator arrays.
+// y, the heads combine across lanes.
 template <typename I, typename V, int K>
-__device__ __forceinline__ void tile_finish(const I* __restrict__ rp, int64_t n, int64_t nnz, int64_t t, int lane,
-                                            uint32_t flags, int64_t tr, const V (&p)[K], V* __restrict__ y, V alpha,
-                                            V beta, bool bz, V* __restrict__ carry_in, V* __restrict__ open_sum,
-                                            int64_t* __restrict__ open_row) {
+__device__ __forceinline__ TileEnds<V> tile_sums(const I* __restrict__ rp, int64_t n, int64_t nnz, int64_t t, int lane,
+                                                 uint32_t flags, int64_t tr, const V (&p)[K], V* __restrict__ y,
+                                                 V alpha, V beta, bool bz) {
   const unsigned lt = (1u << lane) - 1u;  // lanes below this one
   const int64_t el = t * (32 * K) + (int64_t)lane * K;
   // ---- row of the lane's first entry
@@ -157,18 +165,55 @@ __device__ __forceinline__ void tile_finish(const I* __restrict__ rp, int64_t n,
   const V Sm = __shfl_sync(0xffffffffu, S, m);
   const int m0 = fmask ? __ffs(fmask) - 1 : 31;
   const V cin = __shfl_sync(0xffffffffu, S, m0);
-  if (has_flag) {
-    if (later) {
-      axpby_store(y + row, tail + Sm, alpha, beta, bz);
-    } else {  // the tile's last row: may continue into the next tile
-      open_sum[t] = tail + (lane < 31 ? Sm : V(0));
-      open_row[t] = row;
-    }
+  if (has_flag && later) axpby_store(y + row, tail + Sm, alpha, beta, bz);
+  return TileEnds<V>{has_flag && !later, fmask != 0, row, tail + (lane < 31 ? Sm : V(0)), cin};
+}
+
+// The same, the tile's open row (it may continue into the next tile) and carry
+// going to the calibrator arrays.
+template <typename I, typename V, int K>
+__device__ __forceinline__ void tile_finish(const I* __restrict__ rp, int64_t n, int64_t nnz, int64_t t, int lane,
+                                            uint32_t flags, int64_t tr, const V (&p)[K], V* __restrict__ y, V alpha,
+                                            V beta, bool bz, V* __restrict__ carry_in, V* __restrict__ open_sum,
+                                            int64_t* __restrict__ open_row) {
+  const TileEnds<V> E = tile_sums<I, V, K>(rp, n, nnz, t, lane, flags, tr, p, y, alpha, beta, bz);
+  if (E.owner) {
+    open_sum[t] = E.open;
+    open_row[t] = E.row;
   }
   if (lane == 0) {
-    carry_in[t] = cin;
-    if (!fmask) open_row[t] = -1;
+    carry_in[t] = E.cin;
+    if (!E.any) open_row[t] = -1;
   }
+}
+
+// The row open at tile t's end: its sum there and the heads of the following
+// tiles, in tile order, up to the first one that starts a row.  A long row's
+// tiles are read eight at a time (one at a time its loads were the
+// calibration's whole time: 6.4 us for a row over 20 tiles).
+template <typename V>
+__device__ __forceinline__ V chain_sum(int64_t t, int64_t tiles, const V* __restrict__ carry_in,
+                                       const V* __restrict__ open_sum, const int64_t* __restrict__ open_row) {
+  V tot = open_sum[t];
+  if (t + 1 >= tiles) return tot;
+  tot += carry_in[t + 1];
+  bool more = open_row[t + 1] < 0;
+  for (int64_t u = t + 2; more && u < tiles; u += 8) {
+    V c[8];
+    int64_t r[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const bool in = u + q < tiles;
+      c[q] = in ? carry_in[u + q] : V(0);
+      r[q] = in ? open_row[u + q] : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      if (more) tot += c[q];
+      more = more && r[q] < 0;
+    }
+  }
+  return tot;
 }
 
 // Calibration of one tile t (t < tiles) or empty row (t - tiles < nempty)
@@ -182,12 +227,7 @@ __device__ __forceinline__ void spmv_calibrate1(int64_t t, int64_t tiles, const 
   if (t < tiles) {
     const int64_t r = open_row[t];
     if (r < 0) return;
-    V tot = open_sum[t];
-    for (int64_t u = t + 1; u < tiles; ++u) {
-      tot += carry_in[u];
-      if (open_row[u] >= 0) break;
-    }
-    axpby_store(y + r, tot, alpha, beta, bz);
+    axpby_store(y + r, chain_sum<V>(t, tiles, carry_in, open_sum, open_row), alpha, beta, bz);
   } else if (t - tiles < nempty) {
     axpby_store(y + empty[t - tiles], V(0), alpha, beta, bz);
   }

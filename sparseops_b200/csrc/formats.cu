@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "device_util.cuh"
+#include "pdl.cuh"
 #include "spops_internal.h"
 #include "warp_work.cuh"
 
@@ -233,6 +234,7 @@ __global__ void __launch_bounds__(256) padded_win_kernel(
     V* __restrict__ wpartial, int* __restrict__ wcounter, int64_t npieces, const PadPiece* __restrict__ pieces,
     V* __restrict__ partial, int* __restrict__ counter, const int* __restrict__ head, const I* __restrict__ tcol,
     const V* __restrict__ tval) {
+  overlap_begin();
   const int lane = threadIdx.x & 31;
   const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   if (w >= nwin) {
@@ -998,11 +1000,11 @@ spops_status_t padded_spmv_t(Context* ctx, Matrix* A, double alpha, const void* 
       SPOPS_LAUNCH_CHECK();
       Pw.tails_fresh = true;
     }
-    padded_win_kernel<I, V><<<(unsigned)g, 256, 0, ctx->stream>>>(
+    SPOPS_CUDA(launch_overlapped(padded_win_kernel<I, V>, g, 256, 0, ctx->stream,
         A->col.as<I>(), A->val.as<V>(), P.chunk_off.as<int64_t>(), P.row_len.as<int>(), ro, n,
         static_cast<const V*>(x), static_cast<V*>(y), (V)alpha, (V)beta, beta == 0.0, P.win.as<PadWin>(), P.nwin,
         P.win_partial.as<V>(), P.win_counter.as<int>(), P.npieces, P.piece.as<PadPiece>(), P.partial.as<V>(),
-        P.counter.as<int>(), P.head.as<int>(), P.tcol.as<I>(), P.tval.as<V>());
+        P.counter.as<int>(), P.head.as<int>(), P.tcol.as<I>(), P.tval.as<V>()));
     SPOPS_LAUNCH_CHECK();
     return SPOPS_OK;
   }

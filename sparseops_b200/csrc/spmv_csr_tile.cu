@@ -31,12 +31,14 @@
 // Summation order depends only on the matrix: results are bit-reproducible.
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <functional>
 #include <vector>
 
 #include "bulk_copy.cuh"
 #include "csr_tile.cuh"
 #include "device_util.cuh"
+#include "pdl.cuh"
 #include "spops_internal.h"
 
 namespace spops {
@@ -96,6 +98,7 @@ __global__ void __launch_bounds__(kTileBlock, kMinBlocks) csr_tile_kernel(
     const int64_t* __restrict__ tile_row, const uint8_t* __restrict__ flags_all, int64_t t_begin, int64_t tiles,
     const V* __restrict__ x, V* __restrict__ y, V alpha, V beta, bool bz, V* __restrict__ carry_in,
     V* __restrict__ open_sum, int64_t* __restrict__ open_row) {
+  overlap_begin();
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (kTileBlock / 32);
   int64_t t = t_begin + blockIdx.x * (int64_t)(kTileBlock / 32) + (threadIdx.x >> 5);
@@ -127,6 +130,177 @@ __global__ void __launch_bounds__(kTileBlock, kMinBlocks) csr_tile_kernel(
     }
     tile_finish<I, V, K>(rp, n, nnz, t, lane, f, r0, p, y, alpha, beta, bz, carry_in, open_sum, open_row);
   }
+}
+
+// ---- the same in one launch
+// The row open at a tile's end is finished by the tile's own warp: it reads on
+// for the row's last entries (tail[t] of them, at most kTailMax; the first 32
+// loaded with the tile's own), and the next tile leaves the entries before its
+// first row start to it.  A row with more entries left (chain[t] > 0 further
+// tiles) is finished by whichever of its tiles arrives last: each leaves its
+// sum and adds one to the owner tile's counter (owner[t], or -1), and the last
+// one adds all of them in tile order, writes the row and clears the counter.
+// Summation order depends only on the matrix here too.
+constexpr int kTailMax = 256;
+
+// All lanes of the warp call; lane `who` has written this tile's part of the
+// chain of tile o (m tiles after it).
+template <typename V>
+__device__ __forceinline__ void chain_arrive(int lane, int who, int64_t o, int32_t m, int32_t* counter,
+                                             const V* carry_in, const V* open_sum, const int64_t* open_row, V* y,
+                                             V alpha, V beta, bool bz) {
+  int last = 0;
+  if (lane == who) {
+    __threadfence();  // the part before the count
+    last = atomicAdd(counter + o, 1) == m;
+    if (last) __threadfence();  // every part is there: read them past L1
+  }
+  if (!__shfl_sync(0xffffffffu, last, who)) return;
+  V tot = V(0);
+  for (int32_t u = lane; u < m; u += 32) tot += __ldcg(carry_in + o + 1 + u);
+  const V open = __ldcg(open_sum + o);
+  const int64_t r = __ldcg(reinterpret_cast<const long long*>(open_row + o));
+#pragma unroll
+  for (int q = 16; q > 0; q >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, q);
+  if (lane == 0) {
+    axpby_store(y + r, open + tot, alpha, beta, bz);
+    counter[o] = 0;  // for the next launch
+  }
+}
+
+template <typename I, typename V, int K, int kMinBlocks>
+__global__ void __launch_bounds__(kTileBlock, kMinBlocks) csr_tile_one_kernel(
+    const I* __restrict__ rp, int64_t n, int64_t nnz, const I* __restrict__ ci, const V* __restrict__ val,
+    const int64_t* __restrict__ tile_row, const uint8_t* __restrict__ flags_all, int64_t tiles,
+    const V* __restrict__ x, V* y, V alpha, V beta, bool bz, V* carry_in, V* open_sum, int64_t* open_row,
+    const TileTail* __restrict__ tails, int32_t* counter, const int64_t* __restrict__ empty, int64_t nempty) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = (int64_t)gridDim.x * (kTileBlock / 32);
+  int64_t t = blockIdx.x * (int64_t)(kTileBlock / 32) + (threadIdx.x >> 5);
+  I c[K], ct = I(0);
+  V a[K], at = V(0);
+  uint32_t flags;
+  int64_t tr;
+  TileTail T;
+  // the pattern and plan of a tile, then its values; the entries after it are
+  // loaded before the tail's length is known
+  auto load_pattern = [&](int64_t tt) {
+    const int64_t el = tt * (32 * K) + (int64_t)lane * K, e1 = (tt + 1) * (32 * K) + lane;
+    if (el + K <= nnz) {
+      load_run<I, K>(ci + el, c);
+    } else {
+#pragma unroll
+      for (int b = 0; b < K; ++b) c[b] = el + b < nnz ? ci[el + b] : I(0);
+    }
+    if (e1 < nnz) ct = ci[e1];
+    flags = flags_all[tt * 32 + lane];
+    tr = tile_row[tt];
+    T = tails[tt];
+  };
+  auto load_values = [&](int64_t tt) {
+    const int64_t el = tt * (32 * K) + (int64_t)lane * K, e1 = (tt + 1) * (32 * K) + lane;
+    if (el + K <= nnz) {
+      load_run<V, K>(val + el, a);
+    } else {
+#pragma unroll
+      for (int b = 0; b < K; ++b) a[b] = el + b < nnz ? val[el + b] : V(0);
+    }
+    if (e1 < nnz) at = val[e1];
+  };
+  overlap_let_next();
+  if (t < tiles) load_pattern(t);
+  overlap_wait();
+  if (t < tiles) load_values(t);
+  for (int64_t i = blockIdx.x * (int64_t)kTileBlock + threadIdx.x; i < nempty; i += (int64_t)gridDim.x * kTileBlock)
+    axpby_store(y + empty[i], V(0), alpha, beta, bz);
+  for (; t < tiles; t += nw) {
+    // lanes before the first row start: another tile's, unless they belong to a chain
+    const unsigned starts = __ballot_sync(0xffffffffu, flags != 0);
+    const bool mine = T.owner >= 0 || ((starts << (31 - lane)) != 0);
+    V p[K], ts = V(0);
+#pragma unroll
+    for (int b = 0; b < K; ++b)
+      p[b] = mine && t * (32 * K) + (int64_t)lane * K + b < nnz ? a[b] * ld_gather(x + c[b]) : V(0);
+    {
+      const V xt = ld_gather(x + ct);
+      if (lane < T.tail) ts = at * xt;
+    }
+    const uint32_t f = flags;
+    const int64_t r0 = tr;
+    const TileTail T0 = T;
+    if (T0.tail > 32) {  // the rest of a longer tail, its loads all in flight together
+      const int64_t e = (t + 1) * (32 * K) + 32 + lane;
+      const int m = T0.tail - 32 - lane;  // entry e + 32q belongs to it when 32q < m
+      V xt[kTailMax / 32 - 1];
+#pragma unroll
+      for (int q = 0; q < kTailMax / 32 - 1; ++q) xt[q] = 32 * q < m ? ld_gather(x + ci[e + 32 * q]) : V(0);
+#pragma unroll
+      for (int q = 0; q < kTailMax / 32 - 1; ++q)
+        if (32 * q < m) ts += val[e + 32 * q] * xt[q];
+    }
+    if (t + nw < tiles) {
+      load_pattern(t + nw);
+      load_values(t + nw);
+    }
+    const TileEnds<V> E = tile_sums<I, V, K>(rp, n, nnz, t, lane, f, r0, p, y, alpha, beta, bz);
+    if (T0.tail > 0) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ts += __shfl_xor_sync(0xffffffffu, ts, o);
+    }
+    if (T0.chain == 0) {
+      if (E.owner) axpby_store(y + E.row, E.open + ts, alpha, beta, bz);
+    } else {
+      if (E.owner) {
+        open_sum[t] = E.open;
+        open_row[t] = E.row;
+      }
+      chain_arrive<V>(lane, 31 - __clz(__ballot_sync(0xffffffffu, E.owner)), t, T0.chain, counter, carry_in, open_sum,
+                      open_row, y, alpha, beta, bz);
+    }
+    if (T0.owner >= 0) {
+      if (lane == 0) carry_in[t] = E.cin;
+      chain_arrive<V>(lane, 0, T0.owner, tails[T0.owner].chain, counter, carry_in, open_sum, open_row, y, alpha, beta,
+                      bz);
+    }
+  }
+}
+
+// tail, chain and owner of every tile
+template <typename I>
+__global__ void tile_tail_kernel(const I* __restrict__ rp, int64_t n, int64_t nnz, const uint8_t* __restrict__ flags,
+                                 int64_t tiles, int tile_size, TileTail* __restrict__ tails,
+                                 unsigned long long* __restrict__ nchain) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= tiles) return;
+  auto any = [&](int64_t u) {
+    const uint4* f = reinterpret_cast<const uint4*>(flags + u * 32);
+    const uint4 a = f[0], b = f[1];
+    return (a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) != 0;
+  };
+  // entries that the row open at tile u's end has after it
+  auto left = [&](int64_t u) -> int64_t {
+    const int64_t e1 = (u + 1) * tile_size;
+    return e1 >= nnz ? 0 : (int64_t)rp[row_holding(rp, n, e1 - 1) + 1] - e1;
+  };
+  TileTail T{0, 0, -1};
+  if (any(t)) {
+    const int64_t l = left(t);
+    if (l <= kTailMax) {
+      T.tail = (int32_t)l;
+    } else {
+      for (int64_t u = t + 1; u < tiles && !(flags[u * 32] & 1u); ++u) {
+        ++T.chain;
+        if (any(u)) break;
+      }
+      atomicAdd(nchain, 1ULL);
+    }
+  }
+  if (!(flags[t * 32] & 1u)) {
+    int64_t o = t - 1;
+    while (o >= 0 && !any(o)) --o;
+    if (o >= 0 && left(o) > kTailMax) T.owner = o;
+  }
+  tails[t] = T;
 }
 
 // ---- staged form (csr_variant 10): the matrix stream by bulk copies
@@ -324,6 +498,7 @@ __global__ void __launch_bounds__(kTileBlock, 3) csr_tile_indirect_kernel(
     const V* __restrict__ vsrc, const int64_t* __restrict__ tile_row, const uint8_t* __restrict__ flags_all,
     int64_t tiles, const V* __restrict__ x, V* __restrict__ y, V alpha, V beta, bool bz, V* __restrict__ carry_in,
     V* __restrict__ open_sum, int64_t* __restrict__ open_row) {
+  overlap_begin();
   constexpr int K = 8;
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (kTileBlock / 32);
@@ -373,16 +548,12 @@ __global__ void csr_tile_calibrate_kernel(int64_t t_begin, int64_t tiles, const 
                                           const V* __restrict__ open_sum, const int64_t* __restrict__ open_row,
                                           const int64_t* __restrict__ empty, int64_t nempty, V* __restrict__ y,
                                           V alpha, V beta, bool bz) {
+  overlap_begin();
   const int64_t t = t_begin + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t < tiles) {
     const int64_t r = open_row[t];
     if (r < 0) return;
-    V tot = open_sum[t];
-    for (int64_t u = t + 1; u < tiles; ++u) {
-      tot += carry_in[u];
-      if (open_row[u] >= 0) break;
-    }
-    axpby_store(y + r, tot, alpha, beta, bz);
+    axpby_store(y + r, chain_sum<V>(t, tiles, carry_in, open_sum, open_row), alpha, beta, bz);
   } else if (t - tiles < nempty) {
     axpby_store(y + empty[t - tiles], V(0), alpha, beta, bz);
   }
@@ -396,6 +567,7 @@ __global__ void __launch_bounds__(kTileBlock, 2) csr_tile_spmm_kernel(
     const int64_t* __restrict__ tile_row, const uint8_t* __restrict__ flags_all, int64_t tiles,
     const V* __restrict__ X, int64_t ldx, int k, V* __restrict__ Y, int64_t ldy, V alpha, V beta, bool bz,
     V* __restrict__ carry_in, V* __restrict__ open_sum, int64_t* __restrict__ open_row) {
+  overlap_begin();
   extern __shared__ __align__(16) unsigned char spmm_smem[];
   using Tile = SpmmTile<I, V, G>;
   const int lane = threadIdx.x & 31;
@@ -428,6 +600,7 @@ __global__ void csr_tile_calibrate_k_kernel(int L, int k, int64_t tiles, const V
                                             const V* __restrict__ open_sum, const int64_t* __restrict__ open_row,
                                             const int64_t* __restrict__ empty, int64_t nempty, V* __restrict__ Y,
                                             int64_t ldy, V alpha, V beta, bool bz) {
+  overlap_begin();
   const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   spmm_calibrate<V>(g / L, (int)(g % L), L, k, tiles, carry_in, open_sum, open_row, empty, nempty, Y, ldy, alpha,
                     beta, bz);
@@ -455,17 +628,17 @@ spops_status_t spmm_tiles_f(Context* ctx, Matrix* A, double alpha, const void* X
     int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
     const int64_t need = (D.tiles + kTileBlock / 32 - 1) / (kTileBlock / 32);
     if (grid > need) grid = need;
-    kern<<<(unsigned)grid, kTileBlock, smem, ctx->stream>>>(
+    SPOPS_CUDA(launch_overlapped(kern, grid, kTileBlock, smem, ctx->stream,
         A->row.as<I>(), A->rows, A->nnz, A->col.as<I>(), A->val.as<V>(), D.tile_row.as<int64_t>(),
         D.flags.as<uint8_t>(), D.tiles, static_cast<const V*>(X), ldx, (int)k, static_cast<V*>(Y), ldy, (V)alpha,
-        (V)beta, bz, cin.as<V>(), osum.as<V>(), D.open_row.as<int64_t>());
+        (V)beta, bz, cin.as<V>(), osum.as<V>(), D.open_row.as<int64_t>()));
     SPOPS_LAUNCH_CHECK();
   }
   if (D.tiles + D.nempty > 0) {
     const int L = spmm_cal_lanes(k);
-    csr_tile_calibrate_k_kernel<V><<<grid_of((D.tiles + D.nempty) * L), 256, 0, ctx->stream>>>(
+    SPOPS_CUDA(launch_overlapped(csr_tile_calibrate_k_kernel<V>, grid_of((D.tiles + D.nempty) * L), 256, 0, ctx->stream,
         L, (int)k, D.tiles, cin.as<V>(), osum.as<V>(), D.open_row.as<int64_t>(), D.empty.as<int64_t>(), D.nempty,
-        static_cast<V*>(Y), ldy, (V)alpha, (V)beta, bz);
+        static_cast<V*>(Y), ldy, (V)alpha, (V)beta, bz));
     SPOPS_LAUNCH_CHECK();
   }
   return SPOPS_OK;
@@ -557,22 +730,28 @@ spops_status_t analyse_t(Context* ctx, Matrix* A) {
   SPOPS_TRY(D.open_sum.alloc_cached(ctx, nt1 * 8, kBuildCacheMax));
   SPOPS_TRY(D.open_row.alloc_cached(ctx, nt1 * 8, kBuildCacheMax));
   SPOPS_TRY(D.empty.alloc_cached(ctx, (size_t)(n > 0 ? n : 1) * 8, kBuildCacheMax));
+  SPOPS_TRY(D.tails.alloc_cached(ctx, nt1 * sizeof(TileTail), kBuildCacheMax));
+  SPOPS_TRY(D.counter.alloc_cached(ctx, nt1 * 4, kBuildCacheMax));
+  SPOPS_CUDA(cudaMemsetAsync(D.counter.p, 0, nt1 * 4, st));
+  SPOPS_TRY(ctx->scratch_reserve(256));
+  unsigned long long* cnt = ctx->scratch.as<unsigned long long>();  // empty rows, chains
+  SPOPS_CUDA(cudaMemsetAsync(cnt, 0, 16, st));
   if (D.tiles > 0 && n > 0) {
     tile_build_kernel<I, K><<<grid_of(D.tiles), 256, 0, st>>>(A->row.as<I>(), n, nnz, D.tiles,
                                                                 D.tile_row.as<int64_t>(), D.flags.as<uint8_t>());
+    tile_tail_kernel<I><<<grid_of(D.tiles), 256, 0, st>>>(A->row.as<I>(), n, nnz, D.flags.as<uint8_t>(), D.tiles,
+                                                          32 * K, D.tails.as<TileTail>(), cnt + 1);
     SPOPS_LAUNCH_CHECK();
   }
-  SPOPS_TRY(ctx->scratch_reserve(256));
-  unsigned long long* cnt = ctx->scratch.as<unsigned long long>();
-  SPOPS_CUDA(cudaMemsetAsync(cnt, 0, 8, st));
   if (n > 0) {
     tile_empty_kernel<I><<<grid_of(n), 256, 0, st>>>(A->row.as<I>(), n, D.empty.as<int64_t>(), cnt);
     SPOPS_LAUNCH_CHECK();
   }
-  unsigned long long h = 0;
-  SPOPS_CUDA(cudaMemcpyAsync(&h, cnt, 8, cudaMemcpyDeviceToHost, st));
+  unsigned long long h[2] = {0, 0};
+  SPOPS_CUDA(cudaMemcpyAsync(h, cnt, 16, cudaMemcpyDeviceToHost, st));
   SPOPS_CUDA(cudaStreamSynchronize(st));
-  D.nempty = (int64_t)h;
+  D.nempty = (int64_t)h[0];
+  D.nchain = (int64_t)h[1];
   D.ready = true;
   return SPOPS_OK;
 }
@@ -594,17 +773,17 @@ spops_status_t spmv_range(Context* ctx, Matrix* A, double alpha, const void* x, 
     int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
     const int64_t need = (t1 - t0 + kTileBlock / 32 - 1) / (kTileBlock / 32);
     if (grid > need) grid = need;
-    csr_tile_kernel<I, V, K, kMinBlocks, kPipe><<<(unsigned)grid, kTileBlock, 0, ctx->stream>>>(
+    SPOPS_CUDA(launch_overlapped(csr_tile_kernel<I, V, K, kMinBlocks, kPipe>, grid, kTileBlock, 0, ctx->stream,
         A->row.as<I>(), A->rows, A->nnz, A->col.as<I>(), A->val.as<V>(), D.tile_row.as<int64_t>(),
         D.flags.as<uint8_t>(), t0, t1, static_cast<const V*>(x), static_cast<V*>(y), (V)alpha, (V)beta, bz,
-        D.carry_in.as<V>(), D.open_sum.as<V>(), D.open_row.as<int64_t>());
+        D.carry_in.as<V>(), D.open_sum.as<V>(), D.open_row.as<int64_t>()));
     SPOPS_LAUNCH_CHECK();
   }
   const int64_t ne = empty_rows ? D.nempty : 0;
   if (t1 - t0 + ne > 0) {
-    csr_tile_calibrate_kernel<V><<<grid_of(t1 - t0 + ne), 256, 0, ctx->stream>>>(
+    SPOPS_CUDA(launch_overlapped(csr_tile_calibrate_kernel<V>, grid_of(t1 - t0 + ne), 256, 0, ctx->stream,
         t0, t1, D.carry_in.as<V>(), D.open_sum.as<V>(), D.open_row.as<int64_t>(), D.empty.as<int64_t>(), ne,
-        static_cast<V*>(y), (V)alpha, (V)beta, bz);
+        static_cast<V*>(y), (V)alpha, (V)beta, bz));
     SPOPS_LAUNCH_CHECK();
   }
   return SPOPS_OK;
@@ -638,11 +817,47 @@ spops_status_t spmv_stage_t(Context* ctx, Matrix* A, double alpha, const void* x
     SPOPS_LAUNCH_CHECK();
   }
   if (tiles + D.nempty > 0) {
-    csr_tile_calibrate_kernel<V><<<grid_of(tiles + D.nempty), 256, 0, ctx->stream>>>(
+    SPOPS_CUDA(launch_overlapped(csr_tile_calibrate_kernel<V>, grid_of(tiles + D.nempty), 256, 0, ctx->stream,
         0, tiles, D.carry_in.as<V>(), D.open_sum.as<V>(), D.open_row.as<int64_t>(), D.empty.as<int64_t>(), D.nempty,
-        static_cast<V*>(y), (V)alpha, (V)beta, bz);
+        static_cast<V*>(y), (V)alpha, (V)beta, bz));
     SPOPS_LAUNCH_CHECK();
   }
+  return SPOPS_OK;
+}
+
+// One launch or two: a small matrix's call is bound by its launches, so one is
+// taken up to a tile per resident warp, or four where no row needs a chain and
+// its fences; above, reading on at every tile's end costs as much as the second
+// launch.  Calls issued back to back, two launches | one (us): power-law 20,000
+// rows 10.1 | 7.6, 60,000 rows 12.4 | 14.0; 512 x 512 Laplacian 10.2 | 7.7;
+// banded 100,000 rows 10.1 | 8.5, 1,000,000 rows 56.0 | 59.3.  (Plain launches
+// instead of overlapped ones: 11.3, 15.5, 12.4, 13.3, 58.5 in two.)
+inline bool one_launch(const Context* ctx, const Matrix* A) {
+  const CsrTiles& D = A->plan.tiles;
+  const int64_t resident = (int64_t)ctx->num_sms * 3 * (kTileBlock / 32);
+  return D.tiles <= (D.nchain > 0 ? resident : 4 * resident);
+}
+
+// All tiles in one launch (csr_tile_one_kernel).
+template <typename I, typename V>
+spops_status_t spmv_one_t(Context* ctx, Matrix* A, double alpha, const void* x, double beta, void* y) {
+  const CsrTiles& D = A->plan.tiles;
+  static int blocks_per_sm = -1;  // per instantiation
+  if (blocks_per_sm < 0) {
+    int bps = 0;
+    SPOPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, csr_tile_one_kernel<I, V, 8, 3>, kTileBlock, 0));
+    blocks_per_sm = bps > 0 ? bps : 1;
+  }
+  int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
+  const int64_t need = std::max((D.tiles + kTileBlock / 32 - 1) / (kTileBlock / 32),
+                                (D.nempty + kTileBlock - 1) / kTileBlock);
+  if (grid > need) grid = need;
+  SPOPS_CUDA(launch_overlapped(csr_tile_one_kernel<I, V, 8, 3>, grid, kTileBlock, 0, ctx->stream, A->row.as<I>(),
+                               A->rows, A->nnz, A->col.as<I>(), A->val.as<V>(), D.tile_row.as<int64_t>(),
+                               D.flags.as<uint8_t>(), D.tiles, static_cast<const V*>(x), static_cast<V*>(y), (V)alpha,
+                               (V)beta, beta == 0.0, D.carry_in.as<V>(), D.open_sum.as<V>(),
+                               D.open_row.as<int64_t>(), D.tails.as<TileTail>(), D.counter.as<int32_t>(),
+                               D.empty.as<int64_t>(), D.nempty));
   return SPOPS_OK;
 }
 
@@ -682,16 +897,16 @@ spops_status_t spmv_indirect_t(Context* ctx, Matrix* A, const int64_t* perm, con
     int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
     const int64_t need = (tiles + kTileBlock / 32 - 1) / (kTileBlock / 32);
     if (grid > need) grid = need;
-    csr_tile_indirect_kernel<I, V><<<(unsigned)grid, kTileBlock, 0, ctx->stream>>>(
+    SPOPS_CUDA(launch_overlapped(csr_tile_indirect_kernel<I, V>, grid, kTileBlock, 0, ctx->stream,
         A->row.as<I>(), A->rows, A->nnz, A->col.as<I>(), perm, static_cast<const V*>(vsrc),
         D.tile_row.as<int64_t>(), D.flags.as<uint8_t>(), tiles, static_cast<const V*>(x), static_cast<V*>(y),
-        (V)alpha, (V)beta, bz, D.carry_in.as<V>(), D.open_sum.as<V>(), D.open_row.as<int64_t>());
+        (V)alpha, (V)beta, bz, D.carry_in.as<V>(), D.open_sum.as<V>(), D.open_row.as<int64_t>()));
     SPOPS_LAUNCH_CHECK();
   }
   if (tiles + D.nempty > 0) {
-    csr_tile_calibrate_kernel<V><<<grid_of(tiles + D.nempty), 256, 0, ctx->stream>>>(
+    SPOPS_CUDA(launch_overlapped(csr_tile_calibrate_kernel<V>, grid_of(tiles + D.nempty), 256, 0, ctx->stream,
         0, tiles, D.carry_in.as<V>(), D.open_sum.as<V>(), D.open_row.as<int64_t>(), D.empty.as<int64_t>(), D.nempty,
-        static_cast<V*>(y), (V)alpha, (V)beta, bz);
+        static_cast<V*>(y), (V)alpha, (V)beta, bz));
     SPOPS_LAUNCH_CHECK();
   }
   return SPOPS_OK;
@@ -705,7 +920,10 @@ spops_status_t dispatch(Context* ctx, Matrix* A, int variant, double alpha, cons
     case 5: return spmv_t<I, V, 4, 4, false>(ctx, A, alpha, x, beta, y);
     case 6: return spmv_t<I, V, 8, 5, false>(ctx, A, alpha, x, beta, y);
     case 10: return spmv_stage_t<I, V, 2, 6>(ctx, A, alpha, x, beta, y);
-    default: return spmv_t<I, V, 8, 3, true>(ctx, A, alpha, x, beta, y);
+    default:
+      if (A->plan.tiles.tiles + A->plan.tiles.nempty == 0) return SPOPS_OK;
+      if (one_launch(ctx, A)) return spmv_one_t<I, V>(ctx, A, alpha, x, beta, y);
+      return spmv_t<I, V, 8, 3, true>(ctx, A, alpha, x, beta, y);
   }
 }
 
@@ -713,6 +931,7 @@ spops_status_t dispatch(Context* ctx, Matrix* A, int variant, double alpha, cons
 
 void CsrTiles::release() {
   tile_row.release(); flags.release(); carry_in.release(); open_sum.release(); open_row.release(); empty.release();
+  tails.release(); counter.release();
   part_tb.clear();
   part_rb.clear();
   tiles = 0;

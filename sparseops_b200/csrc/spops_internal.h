@@ -281,6 +281,14 @@ struct CsrSeg {
   int32_t chunk;
 };
 
+// How the row open at a tile's end is finished (csr_tile_one_kernel): by the
+// tile itself reading `tail` entries on, or, `chain` > 0, with the next `chain`
+// tiles; owner: the tile whose chain this tile's first entries belong to, or -1.
+struct TileTail {
+  int32_t tail, chain;
+  int64_t owner;
+};
+
 // Tile analysis of a CSR matrix for the register-sum kernel
 // (spmv_csr_tile.cu): tiles of 32*k consecutive entries, one warp each.
 struct CsrTiles {
@@ -294,6 +302,9 @@ struct CsrTiles {
   DevBuf open_sum;         // V [tiles]: partial sum of the row open at the tile's end
   DevBuf open_row;         // int64 [tiles]: that row, or -1 (no row starts in the tile)
   DevBuf empty;            // int64 [rows]: empty rows
+  DevBuf tails;            // TileTail [tiles]
+  int64_t nchain = 0;      // tiles whose open row needs a chain
+  DevBuf counter;          // int32 [tiles]: parts of the open row that are in (zero between launches)
   std::vector<int64_t> part_tb, part_rb;  // tile / row bounds of the pipelined host SpMV's ranges
   void release();
 };

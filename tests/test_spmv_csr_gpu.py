@@ -390,3 +390,38 @@ def test_host_path_queued(cuda, rows, pinned):
     call("spops_spmv", ctx.handle, dbl(1.0), h.handle, vp(xd.data_ptr()), dbl(0.0), vp(yd.data_ptr()))
     torch.cuda.synchronize()
     assert torch.equal(yh, yd.cpu())
+
+
+@pytest.mark.parametrize("itype,vtype", [(np.int32, np.float64), (np.int64, np.float32)])
+@pytest.mark.parametrize("lens", [
+    [256] * 8, [255, 1, 257, 300], [200, 88, 31, 33, 250, 6, 200, 312, 1],     # tails of 0, 1, 31 .. 33, 255, 256
+    [200, 313, 5, 200, 569, 7, 3000, 1, 600, 0, 0, 9],                         # one entry more: chains of tiles
+    [0, 5000, 0, 0, 1], [1], [0, 0, 3], [7] * 5000, [0] * 3000 + [40]
+])
+def test_one_launch_row_ends(cuda, orc, itype, vtype, lens):
+    """Small matrices run in one launch: rows that end 0 to 256 entries past
+    their tile, further, on a tile's last entry and in the partial last tile,
+    empty rows around them, twice in a row (the second call on the cleared
+    counters), bit-identical; an infinity that no entry reads stays out."""
+    import torch
+    from sparseops_b200 import CSR_Matrix, SpOps_csr
+    rng = np.random.default_rng(len(lens))
+    n, cols = len(lens), 6000
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(itype)
+    ci = np.concatenate([np.sort(rng.choice(np.arange(1, cols), m, replace=False)) for m in lens]).astype(itype)
+    v = rng.standard_normal(len(ci)).astype(vtype)
+    x = rng.uniform(-1, 1, cols).astype(vtype)
+    x[0] = np.inf
+    y0 = rng.standard_normal(n).astype(vtype)
+    xf = np.where(np.isinf(x), 0, x).astype(np.float64)
+    a64 = (rp.astype(np.int32), ci.astype(np.int32), v.astype(np.float64))
+    ref = orc.spmv_csr(*a64, xf, 0.8, 0.7, y0.astype(np.float64))
+    den = 0.8 * orc.absdot(*a64, xf) + 0.7 * np.abs(y0) + 1e-300
+    A = CSR_Matrix(n, cols, *(torch.from_numpy(a).to("cuda") for a in (rp, ci, v)))
+    out = []
+    for _ in range(2):
+        y = torch.from_numpy(y0).to("cuda")
+        SpOps_csr(0.8, A, torch.from_numpy(x).to("cuda"), 0.7, y)
+        out.append(y.cpu().numpy())
+    assert np.array_equal(out[0], out[1])
+    assert (np.abs(out[0] - ref) / den).max() <= (1e-5 if vtype == np.float32 else 1e-12)
