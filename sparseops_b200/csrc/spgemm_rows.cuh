@@ -157,40 +157,7 @@ __global__ void __launch_bounds__(32 * W)
     const int t = (w * R + s) * 32 + lane;
     key[s] = t < P ? M.key[t] : kNone;
   }
-  if (W == 1) {
-    warp_bitonic_sort<R>(key, lane);
-    __syncwarp();
-  } else {
-    // each warp its 32R keys (descending for odd warps: the complements
-    // ascending), then the merge levels above, their cross-warp stages through
-    // shared memory
-    const uint32_t flip = (w & 1) ? kNone : 0u;
-#pragma unroll
-    for (int s = 0; s < R; ++s) key[s] ^= flip;
-    warp_bitonic_sort<R>(key, lane);
-#pragma unroll
-    for (int s = 0; s < R; ++s) key[s] ^= flip;
-    __syncthreads();  // every warp has its keys in registers
-#pragma unroll 1
-    for (int kk = 2 * NW; kk <= N; kk <<= 1) {
-      const bool asc = kk >= N ? true : ((w & (kk / NW)) == 0);
-#pragma unroll 1
-      for (int jj = kk >> 1; jj >= NW; jj >>= 1) {
-        const int pw = w ^ (jj / NW);
-        const bool keep_min = ((w & (jj / NW)) == 0) == asc;
-#pragma unroll
-        for (int s = 0; s < R; ++s) M.key[w * NW + s * 32 + lane] = key[s];
-        __syncthreads();
-#pragma unroll
-        for (int s = 0; s < R; ++s) {
-          const uint32_t o = M.key[pw * NW + s * 32 + lane];
-          key[s] = keep_min ? min(key[s], o) : max(key[s], o);
-        }
-        __syncthreads();
-      }
-      warp_merge_stage<R, NW / 2>(key, lane, asc);
-    }
-  }
+  block_sort_keys<R, W>(key, M.key, w, lane);
   // ---- where columns start and end: position w*32R + lane*R + s
   const int p0 = w * NW + lane * R;
   const int nv = min(max(P - p0, 0), R);  // real keys of this lane

@@ -329,6 +329,47 @@ __device__ __forceinline__ void warp_merge_stage(uint32_t (&k)[R], int lane, boo
   if constexpr (JJ > 1) warp_merge_stage<R, JJ / 2>(k, lane, asc);
 }
 
+// Ascending sort of a block's 32*R*W keys (W warps, R keys per lane), blocked:
+// warp w, lane L, slot s then holds position w*32R + L*R + s.  Each warp sorts
+// its 32R keys (descending for odd warps: the complements ascending), then the
+// merge levels above run their cross-warp stages through xk (32*R*W keys of
+// shared memory, which every warp is done reading after the first barrier).
+template <int R, int W>
+__device__ __forceinline__ void block_sort_keys(uint32_t (&key)[R], uint32_t* xk, int w, int lane) {
+  if constexpr (W == 1) {
+    warp_bitonic_sort<R>(key, lane);
+    __syncwarp();
+  } else {
+    constexpr int NW = 32 * R, N = NW * W;
+    const uint32_t flip = (w & 1) ? 0xffffffffu : 0u;
+#pragma unroll
+    for (int s = 0; s < R; ++s) key[s] ^= flip;
+    warp_bitonic_sort<R>(key, lane);
+#pragma unroll
+    for (int s = 0; s < R; ++s) key[s] ^= flip;
+    __syncthreads();  // every warp has its keys in registers
+#pragma unroll 1
+    for (int kk = 2 * NW; kk <= N; kk <<= 1) {
+      const bool asc = kk >= N ? true : ((w & (kk / NW)) == 0);
+#pragma unroll 1
+      for (int jj = kk >> 1; jj >= NW; jj >>= 1) {  // partner: warp w ^ (jj / NW), same lane and slot
+        const int pw = w ^ (jj / NW);
+        const bool keep_min = ((w & (jj / NW)) == 0) == asc;
+#pragma unroll
+        for (int s = 0; s < R; ++s) xk[w * NW + s * 32 + lane] = key[s];
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < R; ++s) {
+          const uint32_t o = xk[pw * NW + s * 32 + lane];
+          key[s] = keep_min ? min(key[s], o) : max(key[s], o);
+        }
+        __syncthreads();
+      }
+      warp_merge_stage<R, NW / 2>(key, lane, asc);
+    }
+  }
+}
+
 template <typename I, typename V, int W>
 __global__ void __launch_bounds__(32 * W)
     sort_accum_multi_kernel(const int64_t* __restrict__ list, int64_t nlist, const int64_t* __restrict__ cptr,
@@ -417,40 +458,7 @@ __global__ void __launch_bounds__(32 * W)
     }
   }
   __syncthreads();  // operands parked
-  // sort: warp w's 512 keys in the direction the network wants at size 512
-  // (descending for odd w: sorting the complements ascending), then the
-  // merge levels 1024 .. N
-  {
-    const bool desc = (w & 1) != 0;
-    if (desc) {
-#pragma unroll
-      for (int s = 0; s < R; ++s) key[s] = ~key[s];
-    }
-    warp_bitonic_sort<R>(key, lane);
-    if (desc) {
-#pragma unroll
-      for (int s = 0; s < R; ++s) key[s] = ~key[s];
-    }
-  }
-#pragma unroll 1
-  for (int kk = 2 * NW; kk <= N; kk <<= 1) {
-    const bool asc = kk >= N ? true : ((w & (kk / NW)) == 0);
-#pragma unroll 1
-    for (int jj = kk >> 1; jj >= NW; jj >>= 1) {  // partner: warp w ^ (jj / NW), same lane and slot
-      const int pw = w ^ (jj / NW);
-      const bool keep_min = ((w & (jj / NW)) == 0) == asc;
-#pragma unroll
-      for (int s = 0; s < R; ++s) xk[w * NW + s * 32 + lane] = key[s];
-      __syncthreads();
-#pragma unroll
-      for (int s = 0; s < R; ++s) {
-        const uint32_t o = xk[pw * NW + s * 32 + lane];
-        key[s] = keep_min ? min(key[s], o) : max(key[s], o);
-      }
-      __syncthreads();
-    }
-    warp_merge_stage<R, NW / 2>(key, lane, asc);
-  }
+  block_sort_keys<R, W>(key, xk, w, lane);
   const uint32_t tmask = (1u << tbits) - 1u;
   // the key before this lane's first slot: the previous lane's last, or for
   // lane 0 the previous warp's last

@@ -23,14 +23,16 @@
 //      the first top_k kept, the diagonal excluded, by one stable segmented
 //      radix sort of a descending key with the columns in ascending order as
 //      payload.  Rows of the result are in that order, as the reference's.
-// For top_k <= 32 the counts are not materialised: each row's counts build up
-// in a hash table of its own and the best k are selected from the table (the
-// fused path below, steps 1-3 in one kernel per row size).
+// For top_k <= 32 the counts are not materialised: each row's products are
+// sorted (or counted in a hash table, the longest rows) on chip and the best k
+// selected from the distinct ones (the fused path below, steps 1-3 in one
+// kernel per row size).
 #include <cub/cub.cuh>
 
 #include <numeric>
 #include <vector>
 
+#include "spgemm_sort.cuh"
 #include "spops_internal.h"
 
 namespace spops {
@@ -120,16 +122,18 @@ __global__ void topk_write_kernel(const I* __restrict__ crp, const uint64_t* __r
 
 // (key, column) order of the ranking: key ascending (similarity descending),
 // then column ascending -- the order the stable segmented sort gives.
-__device__ __forceinline__ bool rank_less(uint64_t ka, int64_t ca, uint64_t kb, int64_t cb) {
+__device__ __forceinline__ bool rank_less(uint64_t ka, uint32_t ca, uint64_t kb, uint32_t cb) {
   return ka < kb || (ka == kb && ca < cb);
 }
 
+constexpr uint32_t kNoCol = 0xffffffffu;  // above every row number
+
 // One compare-exchange step of a warp-wide bitonic network over one
 // (key, column) per lane; `up` says whether this lane's block ascends.
-__device__ __forceinline__ void warp_cx(uint64_t& k, int64_t& c, int j, bool up) {
+__device__ __forceinline__ void warp_cx(uint64_t& k, uint32_t& c, int j, bool up) {
   const int lane = threadIdx.x & 31;
   const uint64_t pk = __shfl_xor_sync(0xffffffffu, k, j);
-  const int64_t pc = __shfl_xor_sync(0xffffffffu, c, j);
+  const uint32_t pc = __shfl_xor_sync(0xffffffffu, c, j);
   const bool keep_min = ((lane & j) == 0) == up;
   const bool take = keep_min ? rank_less(pk, pc, k, c) : rank_less(k, c, pk, pc);
   if (take) {
@@ -138,7 +142,7 @@ __device__ __forceinline__ void warp_cx(uint64_t& k, int64_t& c, int j, bool up)
   }
 }
 
-__device__ __forceinline__ void warp_sort32(uint64_t& k, int64_t& c) {
+__device__ __forceinline__ void warp_sort32(uint64_t& k, uint32_t& c) {
   const int lane = threadIdx.x & 31;
   for (int b = 2; b <= 32; b <<= 1)
     for (int j = b >> 1; j > 0; j >>= 1) warp_cx(k, c, j, (lane & b) == 0);
@@ -156,17 +160,17 @@ __device__ __forceinline__ void warp_sort32(uint64_t& k, int64_t& c) {
 // k ln(m / k) candidates, so most offers cost a ballot.
 struct WarpTop {
   uint64_t* buf_k;
-  int64_t* buf_c;
+  uint32_t* buf_c;
   int k, lane, nbuf;
   uint64_t bk, tk;  // the lane's entry of the best 32; the k-th best
-  int64_t bc, tc;
-  __device__ __forceinline__ WarpTop(uint64_t* bkey, int64_t* bcol, int k_, int lane_)
-      : buf_k(bkey), buf_c(bcol), k(k_), lane(lane_), nbuf(0), bk(kDiagKey), tk(kDiagKey), bc(INT64_MAX),
-        tc(INT64_MAX) {}  // padding sorts after every entry, the diagonal included
+  uint32_t bc, tc;
+  __device__ __forceinline__ WarpTop(uint64_t* bkey, uint32_t* bcol, int k_, int lane_)
+      : buf_k(bkey), buf_c(bcol), k(k_), lane(lane_), nbuf(0), bk(kDiagKey), tk(kDiagKey), bc(kNoCol),
+        tc(kNoCol) {}  // padding sorts after every entry, the diagonal included
   // merge 32 pairs sorted ascending across the lanes
-  __device__ __forceinline__ void merge_sorted(uint64_t ck, int64_t cc) {
+  __device__ __forceinline__ void merge_sorted(uint64_t ck, uint32_t cc) {
     const uint64_t rk = __shfl_sync(0xffffffffu, ck, 31 - lane);
-    const int64_t rc = __shfl_sync(0xffffffffu, cc, 31 - lane);
+    const uint32_t rc = __shfl_sync(0xffffffffu, cc, 31 - lane);
     if (rank_less(rk, rc, bk, bc)) {
       bk = rk;
       bc = rc;
@@ -175,11 +179,11 @@ struct WarpTop {
     tk = __shfl_sync(0xffffffffu, bk, k - 1);
     tc = __shfl_sync(0xffffffffu, bc, k - 1);
   }
-  __device__ __forceinline__ void merge(uint64_t ck, int64_t cc) {
+  __device__ __forceinline__ void merge(uint64_t ck, uint32_t cc) {
     warp_sort32(ck, cc);
     merge_sorted(ck, cc);
   }
-  __device__ __forceinline__ void offer(uint64_t key, int64_t col, bool ok) {
+  __device__ __forceinline__ void offer(uint64_t key, uint32_t col, bool ok) {
     const bool cand = ok && rank_less(key, col, tk, tc);
     const unsigned m = __ballot_sync(0xffffffffu, cand);
     if (cand) {
@@ -191,10 +195,10 @@ struct WarpTop {
     if (nbuf >= 32) {
       __syncwarp();
       const uint64_t ck = buf_k[lane];
-      const int64_t cc = buf_c[lane];
+      const uint32_t cc = buf_c[lane];
       const int rest = nbuf - 32;
       uint64_t rk = 0;
-      int64_t rc = 0;
+      uint32_t rc = 0;
       if (lane < rest) {
         rk = buf_k[32 + lane];
         rc = buf_c[32 + lane];
@@ -212,7 +216,7 @@ struct WarpTop {
     if (nbuf > 0) {
       __syncwarp();
       const uint64_t ck = lane < nbuf ? buf_k[lane] : kDiagKey;
-      const int64_t cc = lane < nbuf ? buf_c[lane] : INT64_MAX;
+      const uint32_t cc = lane < nbuf ? buf_c[lane] : kNoCol;
       nbuf = 0;
       merge(ck, cc);
     }
@@ -220,21 +224,202 @@ struct WarpTop {
 };
 
 // ---- fused top-k for k <= 32: the intersection counts are never written.
-// Row i's counts |A_i n A_j| accumulate in a hash table (one warp's, or one
-// block's of W warps; in shared memory, or in global memory for rows of more
-// than 8192 products): every pair of a column c of row i and a row j holding
-// c (row c of the pattern's transpose) adds one to j's count.  The counts are
-// integers, so the order of the additions does not matter, and the
-// transpose's rows need no order either.  Each new key also goes to a list of
-// the occupied slots; the listed slots go to WarpTop as a materialised row
-// would (warp 0 of a block merges the other warps' best 32) and are then
-// cleared, so a table is cleared in full only once per kernel.  j = i is not
-// counted; it is in C's row whenever row i has an entry, which is all the
-// exclusion of the diagonal needs.
+// The products of row i are the rows j of its columns c (row c of the
+// pattern's transpose, in any order): |A_i n A_j| is how often j occurs among
+// them.  Rows of up to 8192 products sort them (topk_sort_kernel): equal j are
+// adjacent and their number is the distance between two starts.  Longer rows
+// count in a hash table in global memory (topk_hash_global_kernel): every
+// product adds one to j's count, and each new key also goes to a list of the
+// occupied slots.  Either way the distinct j go to WarpTop (warp 0 of a block
+// merges the other warps' best 32).  j = i is left out; it is in C's row
+// whenever row i has an entry, which is all the exclusion of the diagonal needs.
 constexpr uint32_t kEmptySlot = 0xffffffffu;
-constexpr int kHashBins = 5;  // products <= 128, 512, 2048, 8192, more
+constexpr int kTopBins = 9;  // products <= 64, 128, .. 8192, more
 
-__host__ __device__ constexpr int64_t hash_bin_max(int bin) { return (int64_t)128 << (2 * bin); }
+__host__ __device__ constexpr int64_t top_bin_max(int bin) { return (int64_t)64 << bin; }
+
+// Sorted counting for one row per block: W warps, R keys per lane, up to
+// 32*R*W products.  The products are gathered and sorted as in row_sort_kernel
+// (spgemm_rows.cuh), the key being j alone, any 32-bit value.  Against hash
+// tables in shared memory (a probe and an atomic add per product, two block
+// barriers per row for more than 512 products), k = 16 on 131,072 rows of 8 to
+// 40 planted entries, fp64, int64: 128 < P <= 512 675 -> 500 us,
+// 512 < P <= 2048 1128 -> 600 us, the rest 193 -> 178 us, the whole call 2.28 ->
+// 1.48 ms.  Bound by the sort's and the gather's instructions, as
+// row_sort_kernel is; forms of 16 keys per lane because a warp's sort costs
+// about the same per key up to there and needs no barrier.
+template <int R, int W>
+struct TopSmem {
+  static constexpr int N = 32 * R * W;
+  static constexpr int kCols = W == 1 ? 32 : 64;
+  int64_t base[kCols];
+  uint64_t bkey[W][64];
+  uint32_t bcol[W][64];
+  uint32_t key[N];       // products; then the distinct j
+  int32_t off[kCols + 1];
+  uint32_t w_edge[W];
+  int32_t w_cnt[W];
+  uint16_t pos[N + 1];   // first sorted position of each distinct j, and P
+};
+
+template <typename I, typename V, int R, int W>
+__global__ void __launch_bounds__(32 * W)
+    topk_sort_kernel(const int32_t* __restrict__ rows, const I* __restrict__ arp, const I* __restrict__ aci,
+                     const I* __restrict__ trp, const I* __restrict__ tci, int k, uint64_t* __restrict__ tkey,
+                     I* __restrict__ tcol, int64_t* __restrict__ kept) {
+  using S = TopSmem<R, W>;
+  constexpr int N = S::N, NW = 32 * R, U = 4;
+  constexpr uint32_t kNone = 0xffffffffu;
+  extern __shared__ __align__(16) unsigned char top_smem[];
+  S& M = *reinterpret_cast<S*>(top_smem);
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  auto sync = [] {
+    if (W == 1) __syncwarp(); else __syncthreads();
+  };
+  const int64_t i = rows[blockIdx.x];
+  const int64_t a0 = arp[i];
+  const int64_t nj = (int64_t)arp[i + 1] - a0;
+  // ---- products
+  int P = 0;
+  for (int64_t jb = 0; jb < nj; jb += S::kCols) {
+    if (w == 0) {
+      int32_t carry = 0;
+#pragma unroll
+      for (int h = 0; h < S::kCols; h += 32) {
+        int32_t len = 0;
+        int64_t st = 0;
+        if (jb + h + lane < nj) {
+          const int64_t c = aci[a0 + jb + h + lane];
+          st = trp[c];
+          len = (int32_t)((int64_t)trp[c + 1] - st);
+        }
+        int32_t inc = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += u;
+        }
+        M.base[h + lane] = st - (carry + inc - len);
+        M.off[h + lane + 1] = carry + inc;
+        carry += __shfl_sync(0xffffffffu, inc, 31);
+      }
+      if (lane == 0) M.off[0] = 0;
+    }
+    sync();
+    const int T = M.off[S::kCols];
+    int j = 0;
+    if (W > 1) {  // the column holding this thread's first product
+      int hi = S::kCols;
+      while (hi - j > 1) {
+        const int mid = (j + hi) >> 1;
+        if (M.off[mid] <= tid) j = mid; else hi = mid;
+      }
+    }
+    for (int t0 = tid; t0 < T; t0 += 32 * W * U) {
+      int64_t q[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int t = t0 + 32 * W * u;
+        if (t < T)
+          while (M.off[j + 1] <= t) ++j;
+        q[u] = M.base[j] + t;
+      }
+      uint32_t r[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (t0 + 32 * W * u < T) r[u] = (uint32_t)tci[q[u]];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (t0 + 32 * W * u < T) M.key[P + t0 + 32 * W * u] = r[u];
+    }
+    P += T;
+    sync();
+  }
+  // ---- sort (row_sort_kernel's network)
+  uint32_t key[R];
+#pragma unroll
+  for (int s = 0; s < R; ++s) {
+    const int t = (w * R + s) * 32 + lane;
+    key[s] = t < P ? M.key[t] : kNone;
+  }
+  block_sort_keys<R, W>(key, M.key, w, lane);
+  // ---- distinct j and where each starts
+  const int p0 = w * NW + lane * R;
+  const int nv = min(max(P - p0, 0), R);  // real keys of this lane
+  uint32_t before = __shfl_up_sync(0xffffffffu, key[R - 1], 1);
+  if (W > 1) {
+    if (lane == 31) M.w_edge[w] = key[R - 1];
+    __syncthreads();
+    if (lane == 0 && w > 0) before = M.w_edge[w - 1];
+  }
+  uint32_t first = 0;
+#pragma unroll
+  for (int s = 0; s < R; ++s) first |= ((s ? key[s - 1] : before) != key[s] ? 1u : 0u) << s;
+  if (p0 == 0) first |= 1u;
+  first &= (1u << nv) - 1u;
+  const int cnt = __popc(first);
+  int incl = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  int n = __shfl_sync(0xffffffffu, incl, 31), rank = incl - cnt;
+  if (W > 1) {
+    if (lane == 31) M.w_cnt[w] = incl;
+    __syncthreads();
+    n = 0;
+#pragma unroll
+    for (int v = 0; v < W; ++v) {
+      const int q = M.w_cnt[v];
+      if (v < w) rank += q;
+      n += q;
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < R; ++s)
+    if (first >> s & 1u) {
+      M.key[rank] = key[s];
+      M.pos[rank++] = (uint16_t)(p0 + s);
+    }
+  if (tid == 0) M.pos[n] = (uint16_t)P;
+  sync();
+  // ---- the best k
+  WarpTop top(M.bkey[w], M.bcol[w], k, lane);
+  for (int q0 = w * 32; q0 < n; q0 += W * 32) {
+    const int q = q0 + lane;
+    uint64_t sim = kDiagKey;
+    uint32_t col = kNoCol;
+    bool ok = false;
+    if (q < n) {
+      col = M.key[q];
+      ok = (int64_t)col != i;
+      const V inter = (V)(M.pos[q + 1] - M.pos[q]);
+      const int64_t u = nj + ((int64_t)arp[col + 1] - (int64_t)arp[col]) - (int64_t)inter;
+      sim = desc_key(u == 0 ? V(0) : V(1) * inter / (V)u);
+    }
+    top.offer(sim, col, ok);
+  }
+  top.flush();
+  if (W > 1) {
+    if (w > 0) {  // the buffer is empty after flush: it carries this warp's best 32
+      M.bkey[w][lane] = top.bk;
+      M.bcol[w][lane] = top.bc;
+    }
+    __syncthreads();
+    if (w > 0) return;
+    for (int v = 1; v < W; ++v) {
+      const uint64_t ck = M.bkey[v][lane];
+      const uint32_t cc = M.bcol[v][lane];
+      if (__any_sync(0xffffffffu, rank_less(ck, cc, top.tk, top.tc))) top.merge_sorted(ck, cc);
+    }
+  }
+  if (lane < k) {
+    tkey[i * k + lane] = top.bk;
+    tcol[i * k + lane] = (I)(top.bc == kNoCol ? 0 : top.bc);
+  }
+  if (lane == 0) kept[i] = n - 1 < k ? n - 1 : k;  // j = i is one of the n
+}
 
 // adds one to j's count; returns the slot, plus kFreshSlot when j was not in
 // the table before, or -1 when the table is full (it has at least twice as
@@ -269,7 +454,7 @@ struct HashWarpSmem {
   int64_t st[32];
   int32_t off[33];
   uint64_t bkey[64];
-  int64_t bcol[64];
+  uint32_t bcol[64];
 };
 
 template <int W>
@@ -343,14 +528,14 @@ __device__ __forceinline__ void topk_hash_row(int64_t i, uint32_t* keys, uint32_
   for (int q0 = wg * 32; q0 < d; q0 += W * 32) {
     const int q = q0 + lane;
     uint64_t key = kDiagKey;
-    int64_t col = INT64_MAX;
+    uint32_t col = kNoCol;
     if (q < d) {
       const uint32_t h = (uint32_t)list[q];
       const uint32_t j = keys[h];
       const V inter = (V)cnts[h];
       const int64_t u = li + ((int64_t)arp[j + 1] - (int64_t)arp[j]) - (int64_t)inter;
       key = desc_key(u == 0 ? V(0) : V(1) * inter / (V)u);
-      col = (int64_t)j;
+      col = j;
     }
     top.offer(key, col, q < d);
   }
@@ -372,48 +557,19 @@ __device__ __forceinline__ void topk_hash_row(int64_t i, uint32_t* keys, uint32_
     if constexpr (W > 1) {
       for (int w = 1; w < W; ++w) {
         const uint64_t ck = ws[w].bkey[lane];
-        const int64_t cc = ws[w].bcol[lane];
+        const uint32_t cc = ws[w].bcol[lane];
         if (__any_sync(0xffffffffu, rank_less(ck, cc, top.tk, top.tc))) top.merge_sorted(ck, cc);
       }
     }
     if (lane < k) {
       tkey[i * k + lane] = top.bk;
-      tcol[i * k + lane] = (I)(top.bc == INT64_MAX ? 0 : top.bc);
+      tcol[i * k + lane] = (I)(top.bc == kNoCol ? 0 : top.bc);
     }
     if (lane == 0) kept[i] = d < k ? d : k;
   }
   group_sync<W>();  // slots cleared and the warps' lists read
   if (wg == 0 && lane == 0) *nlist = 0;
   group_sync<W>();
-}
-
-// Rows whose tables fit in shared memory: RPB groups of W warps per block,
-// each taking rows in turn over its own table of 2^LOG_S slots and its list.
-template <typename I, typename V, int W, int RPB, int LOG_S>
-__global__ void __launch_bounds__(W * RPB * 32)
-    topk_hash_kernel(const int32_t* __restrict__ rows, int64_t nrows, const I* __restrict__ arp,
-                     const I* __restrict__ aci, const I* __restrict__ trp, const I* __restrict__ tci, int k,
-                     uint64_t* __restrict__ tkey, I* __restrict__ tcol, int64_t* __restrict__ kept,
-                     int* __restrict__ err) {
-  constexpr uint32_t S = 1u << LOG_S;
-  extern __shared__ __align__(16) uint32_t hash_smem[];  // per group: keys[S], counts[S], list[S / 2] (16-bit)
-  __shared__ HashWarpSmem ws[W * RPB];
-  __shared__ int s_n[RPB];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, g = wib / W, wg = wib % W;
-  uint32_t* keys = hash_smem + (size_t)g * (2 * S + S / 4);
-  uint32_t* cnts = keys + S;
-  uint16_t* list = reinterpret_cast<uint16_t*>(cnts + S);
-  for (uint32_t q = wg * 32 + lane; q < S; q += W * 32) {
-    keys[q] = kEmptySlot;
-    cnts[q] = 0;
-  }
-  if (wg == 0 && lane == 0) s_n[g] = 0;
-  group_sync<W>();
-  // rows b = blockIdx.x * RPB + g + m * gridDim.x * RPB; a group whose rows
-  // run out leaves (RPB > 1 only with W == 1: no block-wide barrier follows)
-  for (int64_t b = blockIdx.x * (int64_t)RPB + g; b < nrows; b += (int64_t)gridDim.x * RPB)
-    topk_hash_row<I, V, W, uint16_t>(rows[b], keys, cnts, LOG_S, list, s_n + g, arp, aci, trp, tci, k, ws + g * W,
-                                     wg, lane, tkey, tcol, kept, err);
 }
 
 // The longest rows: one block of W warps per row at a time, over the first
@@ -447,29 +603,43 @@ __global__ void __launch_bounds__(W * 32)
   }
 }
 
-// Products per row (sum over its columns c of the transpose's row length) and
-// the row's bin; rows without entries keep nothing and take no bin.
+// Products per row: sum over its columns c of the transpose's row length
+// (8 lanes per row).
 template <typename I>
-__global__ void topk_bin_kernel(const I* __restrict__ arp, const I* __restrict__ aci, const I* __restrict__ trp,
-                                int64_t n, int64_t* __restrict__ prods, int32_t* __restrict__ lists,
-                                unsigned long long* __restrict__ counts, unsigned long long* __restrict__ maxp) {
-  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+__global__ void topk_prods_kernel(const I* __restrict__ arp, const I* __restrict__ aci, const I* __restrict__ trp,
+                                  int64_t n, int64_t* __restrict__ prods) {
+  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
+  const int lane = threadIdx.x & 31, sub = lane & 7;
+  const unsigned group = 0xffu << (lane - sub);
   if (i >= n) return;
   int64_t p = 0;
-  for (int64_t e = (int64_t)arp[i] + lane; e < (int64_t)arp[i + 1]; e += 32) {
+  for (int64_t e = (int64_t)arp[i] + sub; e < (int64_t)arp[i + 1]; e += 8) {
     const int64_t c = aci[e];
     p += (int64_t)trp[c + 1] - (int64_t)trp[c];
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
-  if (lane != 0 || p == 0) return;
-  prods[i] = p;
+  for (int o = 4; o > 0; o >>= 1) p += __shfl_xor_sync(group, p, o);
+  if (sub == 0) prods[i] = p;
+}
+
+// The rows' bins; rows without entries keep nothing and take no bin.  One
+// atomic per bin and warp (one per row took 92 us for 131,072 rows).
+__global__ void topk_bin_kernel(const int64_t* __restrict__ prods, int64_t n, int32_t* __restrict__ lists,
+                                unsigned long long* __restrict__ counts, unsigned long long* __restrict__ maxp) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int64_t p = i < n ? prods[i] : 0;
   int bin = 0;
-  while (bin < kHashBins - 1 && p > hash_bin_max(bin)) ++bin;
-  const unsigned long long pos = atomicAdd(counts + bin, 1ULL);
-  lists[(int64_t)bin * n + (int64_t)pos] = (int32_t)i;
-  if (bin == kHashBins - 1) atomicMax(maxp, (unsigned long long)p);
+  while (bin < kTopBins - 1 && p > top_bin_max(bin)) ++bin;
+  if (p == 0) bin = -1;
+  const unsigned same = __match_any_sync(0xffffffffu, bin);
+  const int leader = __ffs(same) - 1;
+  unsigned long long pos = 0;
+  if (bin >= 0 && lane == leader) pos = atomicAdd(counts + bin, (unsigned long long)__popc(same));
+  pos = __shfl_sync(0xffffffffu, pos, leader);
+  if (bin < 0) return;
+  lists[(int64_t)bin * n + (int64_t)pos + __popc(same & ((1u << lane) - 1u))] = (int32_t)i;
+  if (bin == kTopBins - 1) atomicMax(maxp, (unsigned long long)p);
 }
 
 // Transpose of the pattern with rows in any order: column counts, a scan, and
@@ -560,20 +730,21 @@ spops_status_t topk_fused_t(Context* ctx, Matrix* A, int k, Matrix** out, bool* 
   }
   // 2. products per row and bins
   SPOPS_TRY(prods.alloc((size_t)std::max<int64_t>(n, 1) * 8));
-  SPOPS_TRY(lists.alloc((size_t)kHashBins * std::max<int64_t>(n, 1) * 4));
-  SPOPS_TRY(bins.alloc((size_t)(kHashBins + 1) * 8));
-  SPOPS_CUDA(cudaMemsetAsync(bins.p, 0, (size_t)(kHashBins + 1) * 8, st));
+  SPOPS_TRY(lists.alloc((size_t)kTopBins * std::max<int64_t>(n, 1) * 4));
+  SPOPS_TRY(bins.alloc((size_t)(kTopBins + 1) * 8));
+  SPOPS_CUDA(cudaMemsetAsync(bins.p, 0, (size_t)(kTopBins + 1) * 8, st));
   if (n > 0) {
-    topk_bin_kernel<I><<<grid_for(n * 32), 256, 0, st>>>(A->row.as<I>(), A->col.as<I>(), trp.as<I>(), n,
-                                                         prods.as<int64_t>(), lists.as<int32_t>(),
-                                                         bins.as<unsigned long long>(),
-                                                         bins.as<unsigned long long>() + kHashBins);
+    topk_prods_kernel<I><<<grid_for(n * 8), 256, 0, st>>>(A->row.as<I>(), A->col.as<I>(), trp.as<I>(), n,
+                                                          prods.as<int64_t>());
+    topk_bin_kernel<<<grid_for(n), 256, 0, st>>>(prods.as<int64_t>(), n, lists.as<int32_t>(),
+                                                 bins.as<unsigned long long>(),
+                                                 bins.as<unsigned long long>() + kTopBins);
     SPOPS_LAUNCH_CHECK();
   }
-  unsigned long long hb[kHashBins + 1];
+  unsigned long long hb[kTopBins + 1];
   SPOPS_CUDA(cudaMemcpyAsync(hb, bins.p, sizeof(hb), cudaMemcpyDeviceToHost, st));
   SPOPS_CUDA(cudaStreamSynchronize(st));
-  const int64_t maxp = (int64_t)hb[kHashBins];
+  const int64_t maxp = (int64_t)hb[kTopBins];
   if (maxp > ((int64_t)1 << 29)) return SPOPS_OK;
   // 3. the best k of every row
   const size_t nk = (size_t)std::max<int64_t>(n * k, 1);
@@ -585,36 +756,35 @@ spops_status_t topk_fused_t(Context* ctx, Matrix* A, int k, Matrix** out, bool* 
   SPOPS_TRY(ctx->ensure_errword());
   int* err = ctx->errword.as<int>();
   const int32_t* L = lists.as<int32_t>();
-  auto launch = [&](auto kern, int bin, int warps, int rpb, int log_s) -> spops_status_t {
+  auto launch = [&](auto kern, int bin, size_t smem, int warps) -> spops_status_t {
     const int64_t cnt = (int64_t)hb[bin];
     if (cnt == 0 || k == 0) return SPOPS_OK;  // k = 0 keeps nothing
-    const size_t S = (size_t)1 << log_s;
-    const size_t smem = (size_t)rpb * (2 * S + S / 4) * 4;  // keys, counts, 16-bit list
     SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int bps = 0;
-    SPOPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, warps * rpb * 32, smem));
-    const int64_t grid = std::max<int64_t>(
-        1, std::min<int64_t>((cnt + rpb - 1) / rpb, (int64_t)ctx->num_sms * std::max(bps, 1)));
-    kern<<<(unsigned)grid, warps * rpb * 32, smem, st>>>(
-        L + (int64_t)bin * n, cnt, A->row.as<I>(), A->col.as<I>(), trp.as<I>(), tci.as<I>(), k, skey.as<uint64_t>(),
-        scol.as<I>(), kept.as<int64_t>(), err);
+    SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    kern<<<(unsigned)cnt, warps * 32, smem, st>>>(L + (int64_t)bin * n, A->row.as<I>(), A->col.as<I>(), trp.as<I>(),
+                                                  tci.as<I>(), k, skey.as<uint64_t>(), scol.as<I>(),
+                                                  kept.as<int64_t>());
     SPOPS_LAUNCH_CHECK();
     return SPOPS_OK;
   };
-  SPOPS_TRY(launch(topk_hash_kernel<I, V, 1, 4, 8>, 0, 1, 4, 8));
-  SPOPS_TRY(launch(topk_hash_kernel<I, V, 1, 4, 10>, 1, 1, 4, 10));
-  SPOPS_TRY(launch(topk_hash_kernel<I, V, 4, 1, 12>, 2, 4, 1, 12));
-  SPOPS_TRY(launch(topk_hash_kernel<I, V, 8, 1, 14>, 3, 8, 1, 14));
-  if (hb[kHashBins - 1] > 0 && k > 0) {
+  SPOPS_TRY(launch(topk_sort_kernel<I, V, 16, 16>, 7, sizeof(TopSmem<16, 16>), 16));
+  SPOPS_TRY(launch(topk_sort_kernel<I, V, 16, 8>, 6, sizeof(TopSmem<16, 8>), 8));
+  SPOPS_TRY(launch(topk_sort_kernel<I, V, 16, 4>, 5, sizeof(TopSmem<16, 4>), 4));
+  SPOPS_TRY(launch(topk_sort_kernel<I, V, 16, 2>, 4, sizeof(TopSmem<16, 2>), 2));
+  SPOPS_TRY(launch(topk_sort_kernel<I, V, 16, 1>, 3, sizeof(TopSmem<16, 1>), 1));
+  SPOPS_TRY(launch(topk_sort_kernel<I, V, 8, 1>, 2, sizeof(TopSmem<8, 1>), 1));
+  SPOPS_TRY(launch(topk_sort_kernel<I, V, 4, 1>, 1, sizeof(TopSmem<4, 1>), 1));
+  SPOPS_TRY(launch(topk_sort_kernel<I, V, 2, 1>, 0, sizeof(TopSmem<2, 1>), 1));
+  if (hb[kTopBins - 1] > 0 && k > 0) {
     int log_s = 1;
     while (((int64_t)1 << log_s) < 2 * maxp) ++log_s;
     const int64_t gslots = (int64_t)1 << log_s;
     const int64_t per_block = (2 * gslots + gslots / 2) * 4;
-    int64_t grid = std::min<int64_t>((int64_t)hb[kHashBins - 1], 2 * (int64_t)ctx->num_sms);
+    int64_t grid = std::min<int64_t>((int64_t)hb[kTopBins - 1], 2 * (int64_t)ctx->num_sms);
     grid = std::max<int64_t>(1, std::min<int64_t>(grid, ((int64_t)1 << 29) / per_block));
     SPOPS_TRY(gtab.alloc((size_t)(grid * per_block)));
     topk_hash_global_kernel<I, V, 8><<<(unsigned)grid, 256, 0, st>>>(
-        L + (int64_t)(kHashBins - 1) * n, (int64_t)hb[kHashBins - 1], prods.as<int64_t>(), A->row.as<I>(),
+        L + (int64_t)(kTopBins - 1) * n, (int64_t)hb[kTopBins - 1], prods.as<int64_t>(), A->row.as<I>(),
         A->col.as<I>(), trp.as<I>(), tci.as<I>(), k, gtab.as<uint32_t>(), gslots, skey.as<uint64_t>(), scol.as<I>(),
         kept.as<int64_t>(), err);
     SPOPS_LAUNCH_CHECK();

@@ -275,6 +275,34 @@ def test_topk_every_table_size(cuda, orc, k):
     assert default_context().check_device() == 0
 
 
+@pytest.mark.parametrize("itype,vtype,k", [(np.int64, np.float64, 32), (np.int32, np.float32, 7)])
+def test_topk_product_count_edges(cuda, orc, itype, vtype, k):
+    """Rows whose product counts are the limits between the top-k kernel forms
+    (and one past each), among rows that they share columns of 1 to 60 rows with."""
+    from sparseops_b200.spgemm import HashSpGEMMTopK
+    rng = np.random.default_rng(83)
+    counts = [1] + [c + d for c in (64, 128, 256, 512, 1024, 2048, 4096, 8192) for d in (0, 1)]
+    n, ncols = 3000, 0
+    rows = [[] for _ in range(n)]
+    for t, left in enumerate(counts):
+        while left:
+            size = min(left, int(rng.integers(1, 61)))
+            for r in [t, *rng.choice(np.arange(len(counts), n), size - 1, replace=False)]:
+                rows[r].append(ncols)
+            left -= size
+            ncols += 1
+    lens = np.array([len(r) for r in rows])
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    ci = np.concatenate(rows).astype(np.int64)
+    sizes = np.bincount(ci, minlength=ncols)
+    assert [sizes[ci[rp[t]:rp[t + 1]]].sum() for t in range(len(counts))] == counts
+    ref = orc.spgemm_topk(rp, ci, ncols, k, f32=vtype == np.float32)
+    got = HashSpGEMMTopK(_csr(rp.astype(itype), ci.astype(itype), np.ones(len(ci), vtype), ncols), k).host()
+    assert np.array_equal(got[0].astype(np.int64), ref["rp"])
+    assert np.array_equal(got[1].astype(np.int64), ref["ci"])
+    assert np.array_equal(got[2].astype(np.float64), ref["v"])
+
+
 @pytest.mark.parametrize("so", [0, 1])
 def test_vlength_pipeline_golden(cuda, golden, orc, so):
     """The reference driver's flow (test/test_spgemm_hc_lsh.cpp:230-300):
