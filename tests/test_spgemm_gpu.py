@@ -62,6 +62,34 @@ def test_spgemm_clustered_golden(cuda, golden, orc, so):
     assert C.stats["dense_clusters"] == int(g[f"sp_c{so}_dense"])
 
 
+@pytest.mark.parametrize("k,bands,constrain", [(64, 16, True), (96, 96, True), (64, 16, False), (10, 5, True),
+                                               (24, 1, True)])
+def test_lsh_bucket_and_member_edges(cuda, orc, k, bands, constrain):
+    """Buckets of 2 to 700 equal rows (both sides of the window rule's 256, and
+    member counts at the limits between the pair kernel's forms, past the last
+    one when there is no window rule), many rows without entries (one windowed
+    bucket in every band) and rows alone in their buckets, in a mixed order."""
+    from sparseops_b200.spgemm import lsh_candidate_pairs_vector, minhash_signatures_flat
+    rng = np.random.default_rng(59)
+    sizes = [2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129, 255, 256, 257, 400]
+    sizes += [512, 513] if constrain else [511, 512, 513, 600]
+    ncols, rows = 1 << 17, []
+    for s in sizes:
+        shared = rng.choice(ncols, 8, replace=False)
+        rows += [np.sort(shared)] * (s - s // 4)
+        rows += [np.unique(np.append(shared, rng.integers(0, ncols))) for _ in range(s // 4)]
+    rows += [np.zeros(0, np.int64)] * 700 + [np.unique(rng.integers(0, ncols, 6)) for _ in range(900)]
+    rows = [rows[i] for i in rng.permutation(len(rows))]
+    rp = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int64)
+    ci = np.concatenate(rows).astype(np.int64)
+    A = _csr(rp, ci, np.ones(len(ci)), ncols)
+    sig = minhash_signatures_flat(A, k, 5)
+    pairs = lsh_candidate_pairs_vector(A, k, bands, 5, constrain).host()
+    opi, opj, ops = orc.lsh_pairs(sig, bands, constrain)
+    assert len(opi) > 0
+    assert np.array_equal(pairs[0], opi) and np.array_equal(pairs[1], opj) and np.array_equal(pairs[2], ops)
+
+
 @pytest.mark.parametrize("n,ncomm", [(16384, 64), (131072, 512)])
 def test_pipeline_vs_oracle(cuda, orc, n, ncomm):
     """MinHash -> LSH -> clustering -> SpGEMM, every stage against the oracle."""
