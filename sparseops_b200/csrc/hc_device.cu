@@ -48,6 +48,7 @@
 #include <cstdio>
 #include <vector>
 
+#include "pdl.cuh"
 #include "spops_internal.h"
 
 namespace spops {
@@ -256,18 +257,20 @@ struct Comp {
   int32_t np, nr;
 };
 
-// Limits of the two block forms.  Small: one warp, 6 KB, 32 blocks per SM;
-// it holds a complete graph of 32 rows (496 pairs).  Large: the sort by 256
-// threads, 90 KB, two blocks per SM.
+// Limits of the three block forms.  Tiny: four warps of 3 KB, one component
+// each, 64 per SM.  Small: one warp, 6 KB, 32 per SM; it holds a complete graph
+// of 32 rows (496 pairs).  Large: the sort by 256 threads, 90 KB, two per SM.
+constexpr int kTinyRows = 32, kTinyPairs = 256, kTinyThreads = 32, kTinyPer = 4;
 constexpr int kSmallRows = 64, kSmallPairs = 512, kSmallThreads = 32;
 constexpr int kLargeRows = 256, kLargePairs = 8192, kLargeThreads = 256;
 
-// Components listed by the form that takes them: count[0] small, count[1]
-// large; count[2] = pairs left to the rounds.
+// Components listed by the form that takes them: count[0] small (from the back
+// of `small`, which has room for `cap`), count[1] large, count[3] tiny (from
+// the front of `small`); count[2] = pairs left to the rounds.
 __global__ void cc_class_kernel(const uint32_t* __restrict__ lab, const int64_t* __restrict__ start,
                                 const int64_t* __restrict__ cnt, const int64_t* __restrict__ ncomp,
-                                const uint32_t* __restrict__ row_lab, int64_t n, Comp* __restrict__ small,
-                                Comp* __restrict__ large, unsigned char* __restrict__ by_rounds,
+                                const uint32_t* __restrict__ row_lab, int64_t n, int64_t cap,
+                                Comp* __restrict__ small, Comp* __restrict__ large, unsigned char* __restrict__ by_rounds,
                                 unsigned long long* __restrict__ count) {
   const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (q >= *ncomp) return;
@@ -282,9 +285,9 @@ __global__ void cc_class_kernel(const uint32_t* __restrict__ lab, const int64_t*
   };
   const int64_t r0 = first_not_below(L), nr = first_not_below(L + 1) - r0, np = cnt[q];
   if (nr <= kLargeRows && np <= kLargePairs) {
-    const bool sm = nr <= kSmallRows && np <= kSmallPairs;
-    Comp* list = sm ? small : large;
-    list[atomicAdd(count + (sm ? 0 : 1), 1ULL)] = Comp{start[q], r0, (int32_t)np, (int32_t)nr};
+    const int form = nr <= kTinyRows && np <= kTinyPairs ? 3 : nr <= kSmallRows && np <= kSmallPairs ? 0 : 1;
+    const int64_t at = (int64_t)atomicAdd(count + form, 1ULL);
+    (form == 1 ? large[at] : small[form == 3 ? at : cap - 1 - at]) = Comp{start[q], r0, (int32_t)np, (int32_t)nr};
   } else {
     by_rounds[L] = 1;
     atomicAdd(count + 2, (unsigned long long)np);
@@ -326,6 +329,11 @@ __device__ __forceinline__ bool cand_above(double s, uint32_t pk, double t, uint
   return s != t ? s > t : pk > qk;
 }
 
+template <int ROWS, int PAIRS>
+__host__ __device__ constexpr size_t hc_component_smem() {
+  return ((size_t)PAIRS * 10 + (size_t)ROWS * ROWS / 8 + (size_t)ROWS * 8 + 15) / 16 * 16;
+}
+
 // The sequential loop of hc.cpp on one component, one block each.  Bound by
 // the latency of its steps (dependent shared-memory accesses, and the global
 // loads of a Jaccard score), so many components run per SM.  The candidates
@@ -337,26 +345,37 @@ __device__ __forceinline__ bool cand_above(double s, uint32_t pk, double t, uint
 // test is two loads.  Found pairs wait in the slots of consumed candidates:
 // each consumes one candidate, so they never reach the unread ones.  On
 // 16,384 groups of 32 rows (2.3M pairs, 17,080 components) clustering took
-// 7.4 ms in 110 rounds of two kernels over all components, and takes 1.2 ms
-// this way: 0.46 ms in the small form, 0.22 ms in two large blocks, the rest
-// the components (0.10 ms), the sorts by component and the final order.
-template <typename I, int ROWS, int PAIRS, int THREADS>
-__global__ void __launch_bounds__(THREADS)
-    hc_component_kernel(const Comp* __restrict__ list, const uint32_t* __restrict__ pair_id,
+// 7.4 ms in 110 rounds of two kernels over all components, and takes 1.05 ms
+// this way: 0.25 ms for the small form and the two large blocks beside it
+// (0.46 and 0.22 ms one after the other), the rest the components (0.10 ms),
+// the sorts by component and the final order.
+//
+// The forms' launches share nothing but the parent array, in which each writes
+// its own rows, so each lets the next begin at once and waits for the one
+// before it only at its end.
+template <typename I, int ROWS, int PAIRS, int THREADS, int PER>
+__global__ void __launch_bounds__(THREADS* PER)
+    hc_component_kernel(const Comp* __restrict__ list, int64_t step, int64_t ncomp,
+                        const uint32_t* __restrict__ pair_id,
                         const uint32_t* __restrict__ row_id, const int64_t* __restrict__ pi,
                         const int64_t* __restrict__ pj, const double* __restrict__ ps, int64_t cluster_size,
                         const I* __restrict__ rp, const I* __restrict__ ci, int32_t* __restrict__ parent) {
   static_assert(ROWS <= 256 && ROWS % 32 == 0, "local rows are bytes");
+  static_assert(PER == 1 || THREADS == 32, "components of one block share no barrier");
   extern __shared__ __align__(16) unsigned char comp_smem[];
-  double* sc = reinterpret_cast<double*>(comp_smem);                     // [PAIRS]
+  const int part = PER == 1 ? 0 : threadIdx.x / THREADS;
+  double* sc = reinterpret_cast<double*>(comp_smem + part * hc_component_smem<ROWS, PAIRS>());  // [PAIRS]
   uint32_t* given = reinterpret_cast<uint32_t*>(sc + PAIRS);             // [ROWS * ROWS / 32]
   uint32_t* rows = given + ROWS * ROWS / 32;                             // [ROWS]
   uint16_t* pk = reinterpret_cast<uint16_t*>(rows + ROWS);               // [PAIRS]
   uint16_t* size = pk + PAIRS;                                           // [ROWS]
   unsigned char* root = reinterpret_cast<unsigned char*>(size + ROWS);   // [ROWS]
   unsigned char* open = root + ROWS;                                     // [ROWS]
-  const Comp C = list[blockIdx.x];
-  const int tid = threadIdx.x;
+  overlap_let_next();
+  const int64_t slot = blockIdx.x * (int64_t)PER + part;
+  if (slot >= ncomp) return;  // a whole warp, and not the block's only one
+  const Comp C = list[slot * step];
+  const int tid = threadIdx.x - part * THREADS;
   auto sync = [] {
     if (THREADS == 32) __syncwarp(); else __syncthreads();
   };
@@ -501,11 +520,7 @@ __global__ void __launch_bounds__(THREADS)
     __syncwarp();
   }
   for (int r = lane; r < C.nr; r += 32) parent[rows[r]] = (int32_t)rows[root[r]];
-}
-
-template <int ROWS, int PAIRS>
-constexpr size_t hc_component_smem() {
-  return (size_t)PAIRS * 10 + (size_t)ROWS * ROWS / 8 + (size_t)ROWS * 8;
+  overlap_wait();
 }
 
 // (a, b) among the initial pairs (sorted by (i, j))
@@ -630,8 +645,8 @@ spops_status_t hc_device_t(Context* ctx, Matrix* A, const int64_t* pi, const int
   SPOPS_TRY(size.alloc(nn * 4));
   SPOPS_TRY(open.alloc(nn));
   SPOPS_TRY(res.alloc(nn * 8));
-  SPOPS_TRY(flags.alloc(64));
-  SPOPS_CUDA(cudaMemsetAsync(flags.p, 0, 64, st));
+  SPOPS_TRY(flags.alloc(128));
+  SPOPS_CUDA(cudaMemsetAsync(flags.p, 0, 128, st));
   int* err = flags.as<int>();
   unsigned long long* ntasks = reinterpret_cast<unsigned long long*>(flags.as<char>() + 8);
   // live counts: cnt[cur] of the round about to run, cnt[cur ^ 1] of the next
@@ -694,32 +709,34 @@ spops_status_t hc_device_t(Context* ctx, Matrix* A, const int64_t* pi, const int
     SPOPS_CUDA(cub::DeviceScan::ExclusiveSum(ctmp.p, c4, ucnt.as<int64_t>(), ustart.as<int64_t>(), (int64_t)nc1, st));
     cc_class_kernel<<<hc_grid((int64_t)nc1), 256, 0, st>>>(
         ulab.as<uint32_t>(), ustart.as<int64_t>(), ucnt.as<int64_t>(), ncomp, rlab.as<uint32_t>(), n,
-        small.as<Comp>(), large.as<Comp>(), by_rounds.as<unsigned char>(), count);
+        (int64_t)nc1, small.as<Comp>(), large.as<Comp>(), by_rounds.as<unsigned char>(), count);
     SPOPS_LAUNCH_CHECK();
-    unsigned long long hc[3] = {0, 0, 0};
-    SPOPS_CUDA(cudaMemcpyAsync(hc, count, 24, cudaMemcpyDeviceToHost, st));
+    unsigned long long hc[4] = {0, 0, 0, 0};
+    SPOPS_CUDA(cudaMemcpyAsync(hc, count, 32, cudaMemcpyDeviceToHost, st));
     SPOPS_CUDA(cudaStreamSynchronize(st));
     rest = (int64_t)hc[2];
-    if (hc[1] > 0) {  // first: the longest blocks
-      constexpr size_t sm = hc_component_smem<kLargeRows, kLargePairs>();
-      SPOPS_CUDA(cudaFuncSetAttribute(hc_component_kernel<I, kLargeRows, kLargePairs, kLargeThreads>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-      hc_component_kernel<I, kLargeRows, kLargePairs, kLargeThreads><<<(unsigned)hc[1], kLargeThreads, sm, st>>>(
-          large.as<Comp>(), pid.as<uint32_t>(), rid.as<uint32_t>(), pi, pj, ps, cluster_size, A->row.as<I>(),
-          A->col.as<I>(), parent.as<int32_t>());
-      SPOPS_LAUNCH_CHECK();
-    }
-    if (hc[0] > 0) {
-      constexpr size_t sm = hc_component_smem<kSmallRows, kSmallPairs>();
-      hc_component_kernel<I, kSmallRows, kSmallPairs, kSmallThreads><<<(unsigned)hc[0], kSmallThreads, sm, st>>>(
-          small.as<Comp>(), pid.as<uint32_t>(), rid.as<uint32_t>(), pi, pj, ps, cluster_size, A->row.as<I>(),
-          A->col.as<I>(), parent.as<int32_t>());
-      SPOPS_LAUNCH_CHECK();
-    }
+    auto launch = [&](auto kern, const Comp* list, int64_t step, int64_t m, int threads, int per,
+                      size_t sm) -> spops_status_t {
+      if (m <= 0) return SPOPS_OK;
+      SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm * per));
+      SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+      SPOPS_CUDA(launch_overlapped(kern, (m + per - 1) / per, threads * per, sm * per, st, list, step, m,
+                                   pid.as<uint32_t>(), rid.as<uint32_t>(), pi, pj, ps, cluster_size, A->row.as<I>(),
+                                   A->col.as<I>(), parent.as<int32_t>()));
+      return SPOPS_OK;
+    };
+    // the longest blocks first
+    SPOPS_TRY(launch(hc_component_kernel<I, kLargeRows, kLargePairs, kLargeThreads, 1>, large.as<Comp>(), 1,
+                     (int64_t)hc[1], kLargeThreads, 1, hc_component_smem<kLargeRows, kLargePairs>()));
+    SPOPS_TRY(launch(hc_component_kernel<I, kSmallRows, kSmallPairs, kSmallThreads, 1>,
+                     small.as<Comp>() + (nc1 - 1), -1, (int64_t)hc[0], kSmallThreads, 1,
+                     hc_component_smem<kSmallRows, kSmallPairs>()));
+    SPOPS_TRY(launch(hc_component_kernel<I, kTinyRows, kTinyPairs, kTinyThreads, kTinyPer>, small.as<Comp>(), 1,
+                     (int64_t)hc[3], kTinyThreads, kTinyPer, hc_component_smem<kTinyRows, kTinyPairs>()));
     if (tr.on) {
       char what[96];
-      std::snprintf(what, sizeof(what), "components: %llu small, %llu large, %lld pairs to the rounds", hc[0], hc[1],
-                    (long long)rest);
+      std::snprintf(what, sizeof(what), "components: %llu tiny, %llu small, %llu large, %lld pairs to the rounds", hc[3],
+                    hc[0], hc[1], (long long)rest);
       tr.mark(st, what);
     }
   }

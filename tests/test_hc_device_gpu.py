@@ -113,3 +113,14 @@ def test_device_hc_component_sizes(cuda, sizes, cs):
     hperm, hoffs = hierarchical_clustering_v0_fast(rp, ci, n, (pi, pj, ps), cs)
     dperm, doffs = hierarchical_clustering_device(_csr(rp, ci, n), pairs_from_arrays(pi, pj, ps), cs)
     assert np.array_equal(dperm, hperm) and np.array_equal(doffs, hoffs)
+
+
+@pytest.mark.parametrize("sizes", [
+    [(32, 256), (32, 257), (33, 256), (33, 40), (2, 1)],              # both sides of the four-warp blocks' limits
+    [(31, 200), (32, 31), (16, 120), (23, 253), (2, 1), (5, 4)] * 2,  # those blocks alone, not all warps in use
+    [(9, 20)] * 9 + [(64, 512), (256, 4000), (2, 1)],                 # all three forms at once
+])
+@pytest.mark.parametrize("cs", [2, 8, 40])
+def test_device_hc_tiny_component_sizes(cuda, sizes, cs):
+    """As test_device_hc_component_sizes, at the limits of the four-warp form."""
+    test_device_hc_component_sizes(cuda, sizes, cs)
