@@ -346,9 +346,9 @@ __host__ __device__ constexpr size_t hc_component_smem() {
 // each consumes one candidate, so they never reach the unread ones.  On
 // 16,384 groups of 32 rows (2.3M pairs, 17,080 components) clustering took
 // 7.4 ms in 110 rounds of two kernels over all components, and takes 1.05 ms
-// this way: 0.25 ms for the small form and the two large blocks beside it
-// (0.46 and 0.22 ms one after the other), the rest the components (0.10 ms),
-// the sorts by component and the final order.
+// this way: 0.53 ms for the three forms side by side (0.69 one after the
+// other, with two forms), the rest the components (0.10 ms), the sorts by
+// component and the final order.
 //
 // The forms' launches share nothing but the parent array, in which each writes
 // its own rows, so each lets the next begin at once and waits for the one

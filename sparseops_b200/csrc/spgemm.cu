@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "spops_internal.h"
+#include "spgemm_groups.cuh"
 #include "spgemm_rows.cuh"
 #include "spgemm_sort.cuh"
 
@@ -504,16 +505,24 @@ spops_status_t build_clusters(Context* ctx, const Matrix* A, const int64_t* perm
 }
 
 // ------------------------------------------------------------ flops
+// 8 lanes per cluster (524,288 rows of 19 entries: 105 us with a warp each, 53
+// with 8 lanes).
 template <typename I>
 __global__ void cluster_flops_kernel(const int64_t* __restrict__ cptr, const int32_t* __restrict__ colids, int64_t ncl,
                                      const I* __restrict__ brp, int64_t* __restrict__ flops) {
-  const int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (c >= ncl) return;
+  const int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
+  const int lane = threadIdx.x & 31, sub = lane & 7;
+  if (c >= ncl) return;  // whole groups of 8 lanes
+  const unsigned group = 0xffu << (lane - sub);
+  const int64_t end = cptr[c + 1];
   int64_t f = 0;
-  for (int64_t j = cptr[c] + lane; j < cptr[c + 1]; j += 32) f += (int64_t)brp[colids[j] + 1] - (int64_t)brp[colids[j]];
-  for (int o = 16; o > 0; o >>= 1) f += __shfl_down_sync(0xffffffffu, f, o);
-  if (lane == 0) flops[c] = f;
+  for (int64_t j = cptr[c] + sub; j < end; j += 8) {
+    const int64_t r = colids[j];
+    f += (int64_t)brp[r + 1] - (int64_t)brp[r];
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) f += __shfl_xor_sync(group, f, o);
+  if (sub == 0) flops[c] = f;
 }
 
 // get_spgemm_flop (src/spgemm.cpp:24-42): 2 x sum over A's entries of nnz(B row)
@@ -1100,22 +1109,29 @@ __global__ void classify_kernel(const int64_t* __restrict__ cptr, const int64_t*
 constexpr unsigned char kRowSettled = 2;  // settled[c] of the one-row clusters of row_sort_kernel
 
 // ------------------------------------------------------------ to CSR
+// Entries kept per row of C, for the clusters whose kernel did not count them
+// (the hash path, and clusters of more than kGroupRows rows).  A warp looks at
+// 32 clusters, since few are left (a warp per cluster took 114 us for 524,288
+// rows, nearly all counted already).
 template <typename V>
 __global__ void row_count_kernel(const int64_t* __restrict__ soff_val, const int64_t* __restrict__ nz,
                                  const int64_t* __restrict__ offsets, const int64_t* __restrict__ perm, int64_t ncl,
                                  const V* __restrict__ cval, bool keep_zeros,
                                  const unsigned char* __restrict__ settled, int64_t* __restrict__ rowcnt) {
-  // warp per cluster, lanes over its rows (csz <= 32 common) and columns
-  const int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t c0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5 << 5;
   const int lane = threadIdx.x & 31;
-  if (c >= ncl || settled[c] == kRowSettled) return;  // its kernel counted the row
-  const int64_t csz = offsets[c + 1] - offsets[c];
-  const int64_t ncol = nz[c];
-  for (int64_t l = 0; l < csz; ++l) {
-    int64_t cnt = 0;
-    for (int64_t p = lane; p < ncol; p += 32) cnt += (keep_zeros || cval[soff_val[c] + p * csz + l] != V(0)) ? 1 : 0;
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-    if (lane == 0) rowcnt[perm[offsets[c] + l]] = cnt;
+  const bool mine = c0 + lane < ncl && settled[c0 + lane] != kRowSettled &&
+                    (!settled[c0 + lane] || offsets[c0 + lane + 1] - offsets[c0 + lane] > kGroupRows);
+  for (unsigned todo = __ballot_sync(0xffffffffu, mine); todo; todo &= todo - 1) {
+    const int64_t c = c0 + __ffs(todo) - 1;
+    const int64_t csz = offsets[c + 1] - offsets[c];
+    const int64_t ncol = nz[c];
+    for (int64_t l = 0; l < csz; ++l) {
+      int64_t cnt = 0;
+      for (int64_t p = lane; p < ncol; p += 32) cnt += (keep_zeros || cval[soff_val[c] + p * csz + l] != V(0)) ? 1 : 0;
+      for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+      if (lane == 0) rowcnt[perm[offsets[c] + l]] = cnt;
+    }
   }
 }
 
@@ -1251,15 +1267,14 @@ __global__ void num_bin_kernel(const int64_t* __restrict__ nz, const int64_t* __
 
 // sort path: bin q holds the clusters with at most 32 << q products whose
 // output columns fit a 32-bit key beside the product index.  settled[c]:
-//   1            sort_accum kernels (spgemm_sort.cuh), at most kSortCols
-//                (kMultiCols) columns: bins 0-4 one warp, 2^q keys per lane;
-//                bins 5-8 2^(q-4) warps of 16 keys per lane
+//   1            group_sort_kernel (spgemm_groups.cuh), at most kGroupCols
+//                columns: bins 0-4 one warp, 2^q keys per lane; bins 5-8
+//                2^(q-4) warps of 16 keys per lane
 //   kRowSettled  row_sort_kernel (spgemm_rows.cuh), clusters of one row with
 //                more than 32 << (kRowBin0 - 1) products: bin kSortBins + q -
 //                kRowBin0.  Smaller rows fit a few keys per lane, where four
-//                rows share a block of the one-warp kernel.
+//                rows share a block of group_sort_kernel.
 constexpr int kSortBins = 9;
-constexpr int kSortOneWarpBins = 5;
 constexpr int kRowBin0 = 2;
 constexpr int kRowBins = kSortBins - kRowBin0;
 constexpr int kAllBins = kSortBins + kRowBins;
@@ -1284,7 +1299,7 @@ __global__ void sort_bin_kernel(const int64_t* __restrict__ flops, const int64_t
       if (fits && q >= kRowBin0 && offsets[c + 1] - offsets[c] == 1) {
         b = (uint32_t)(kSortBins + q - kRowBin0);
         how = kRowSettled;
-      } else if (fits && nj <= (q < kSortOneWarpBins ? kSortCols : kMultiCols)) {
+      } else if (fits && nj <= kGroupCols) {
         b = (uint32_t)q;
         how = 1;
       }
@@ -1566,7 +1581,7 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
   SPOPS_TRY(cmax.alloc((size_t)std::max<int64_t>(ncl, 1) * 8));
   SPOPS_CUDA(cudaMemsetAsync(nzd.p, 0, (size_t)(ncl + 1) * 8, st));
   if (ncl > 0) {
-    cluster_flops_kernel<I><<<grid_for(ncl * 32), 256, 0, st>>>(cptr.as<int64_t>(), colids.as<int32_t>(), ncl,
+    cluster_flops_kernel<I><<<grid_for(ncl * 8), 256, 0, st>>>(cptr.as<int64_t>(), colids.as<int32_t>(), ncl,
                                                                 B->row.as<I>(), flops.as<int64_t>());
     SPOPS_LAUNCH_CHECK();
   }
@@ -1727,8 +1742,11 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
   if (stats) stats->symbolic_ms = tm.lap(st);
   tr.mark(st, "symbolic kernels + slab offsets");
 
-  // --- sort path: columns, classification and values in one pass
-  PoolBuf drop(ctx), ndense(ctx);
+  // --- sort path: columns, classification, values and the rows' counts in one
+  // pass
+  PoolBuf drop(ctx), ndense(ctx), rowcnt(ctx);
+  SPOPS_TRY(rowcnt.alloc((nn + 1) * 8));
+  SPOPS_CUDA(cudaMemsetAsync(rowcnt.p, 0, (nn + 1) * 8, st));
   SPOPS_TRY(drop.alloc(ncl1));
   SPOPS_TRY(ndense.alloc(8));
   SPOPS_CUDA(cudaMemsetAsync(ndense.p, 0, 8, st));
@@ -1737,45 +1755,33 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
   for (int q = 0; q < kSortBins; ++q) {
     const int64_t m = tstart[q + 1] - tstart[q];
     if (m <= 0) continue;
-    const unsigned grid = (unsigned)((m + kSortWarps - 1) / kSortWarps);
     const int64_t* dl = slist.as<int64_t>() + tstart[q];
-    const int tbits = 5 + q;
-#define SPOPS_SORT_LAUNCH(RR)                                                                                    \
-  /* static + dynamic shared memory can pass 48 KB: raise the limit */                                         \
-  SPOPS_CUDA(cudaFuncSetAttribute(sort_accum_kernel<I, V, RR>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
-                                  (int)sort_accum_smem<V, RR>()));                                                \
-  sort_accum_kernel<I, V, RR><<<grid, 32 * kSortWarps, sort_accum_smem<V, RR>(), st>>>(                         \
-      dl, m, cptr.as<int64_t>(), cptr_val.as<int64_t>(), colids.as<int32_t>(), avals.as<V>(), offs.as<int64_t>(), \
-      B->row.as<I>(), B->col.as<I>(), B->val.as<V>(), tbits, b_rowdense, l2_budget, sort_output, rowwise,        \
-      soff.as<int64_t>(), soff_val.as<int64_t>(), nzd.as<int64_t>(), cmin.as<int64_t>(), cmax.as<int64_t>(),      \
-      drop.as<unsigned char>(), reinterpret_cast<unsigned long long*>(ndense.p), ccol.as<int32_t>(), cval.as<V>())
-#define SPOPS_MULTI_LAUNCH(WW)                                                                                    \
-  SPOPS_CUDA(cudaFuncSetAttribute(sort_accum_multi_kernel<I, V, WW>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                  (int)sort_multi_smem<V, WW>()));                                                \
-  sort_accum_multi_kernel<I, V, WW><<<(unsigned)m, 32 * WW, sort_multi_smem<V, WW>(), st>>>(                     \
-      dl, m, cptr.as<int64_t>(), cptr_val.as<int64_t>(), colids.as<int32_t>(), avals.as<V>(), offs.as<int64_t>(), \
-      B->row.as<I>(), B->col.as<I>(), B->val.as<V>(), tbits, b_rowdense, l2_budget, sort_output, rowwise,        \
-      soff.as<int64_t>(), soff_val.as<int64_t>(), nzd.as<int64_t>(), cmin.as<int64_t>(), cmax.as<int64_t>(),      \
-      drop.as<unsigned char>(), reinterpret_cast<unsigned long long*>(ndense.p), ccol.as<int32_t>(), cval.as<V>())
+    auto launch = [&](auto kern, size_t smem, int warps) -> spops_status_t {
+      const int per = warps == 1 ? kGroupPer : 1;
+      SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem * per));
+      SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+      kern<<<(unsigned)((m + per - 1) / per), warps * per * 32, smem * per, st>>>(
+          dl, m, cptr.as<int64_t>(), cptr_val.as<int64_t>(), colids.as<int32_t>(), avals.as<V>(), offs.as<int64_t>(),
+          perm.as<int64_t>(), B->row.as<I>(), B->col.as<I>(), B->val.as<V>(), b_rowdense, l2_budget, sort_output, rowwise,
+          soff.as<int64_t>(), soff_val.as<int64_t>(), nzd.as<int64_t>(), cmin.as<int64_t>(), cmax.as<int64_t>(),
+          drop.as<unsigned char>(), reinterpret_cast<unsigned long long*>(ndense.p), ccol.as<int32_t>(),
+          cval.as<V>(), rowcnt.as<int64_t>());
+      SPOPS_LAUNCH_CHECK();
+      return SPOPS_OK;
+    };
     switch (q) {
-      case 0: SPOPS_SORT_LAUNCH(1); break;
-      case 1: SPOPS_SORT_LAUNCH(2); break;
-      case 2: SPOPS_SORT_LAUNCH(4); break;
-      case 3: SPOPS_SORT_LAUNCH(8); break;
-      case 4: SPOPS_SORT_LAUNCH(16); break;
-      case 5: SPOPS_MULTI_LAUNCH(2); break;
-      case 6: SPOPS_MULTI_LAUNCH(4); break;
-      case 7: SPOPS_MULTI_LAUNCH(8); break;
-      default: SPOPS_MULTI_LAUNCH(16); break;
+      case 0: SPOPS_TRY(launch(group_sort_kernel<I, V, 1, 1>, sizeof(GroupSmem<V, 1, 1>), 1)); break;
+      case 1: SPOPS_TRY(launch(group_sort_kernel<I, V, 2, 1>, sizeof(GroupSmem<V, 2, 1>), 1)); break;
+      case 2: SPOPS_TRY(launch(group_sort_kernel<I, V, 4, 1>, sizeof(GroupSmem<V, 4, 1>), 1)); break;
+      case 3: SPOPS_TRY(launch(group_sort_kernel<I, V, 8, 1>, sizeof(GroupSmem<V, 8, 1>), 1)); break;
+      case 4: SPOPS_TRY(launch(group_sort_kernel<I, V, 16, 1>, sizeof(GroupSmem<V, 16, 1>), 1)); break;
+      case 5: SPOPS_TRY(launch(group_sort_kernel<I, V, 16, 2>, sizeof(GroupSmem<V, 16, 2>), 2)); break;
+      case 6: SPOPS_TRY(launch(group_sort_kernel<I, V, 16, 4>, sizeof(GroupSmem<V, 16, 4>), 4)); break;
+      case 7: SPOPS_TRY(launch(group_sort_kernel<I, V, 16, 8>, sizeof(GroupSmem<V, 16, 8>), 8)); break;
+      default: SPOPS_TRY(launch(group_sort_kernel<I, V, 16, 16>, sizeof(GroupSmem<V, 16, 16>), 16)); break;
     }
-#undef SPOPS_SORT_LAUNCH
-#undef SPOPS_MULTI_LAUNCH
-    SPOPS_LAUNCH_CHECK();
   }
-  // the same for one-row clusters, their rows counted too; largest first
-  PoolBuf rowcnt(ctx);
-  SPOPS_TRY(rowcnt.alloc((nn + 1) * 8));
-  SPOPS_CUDA(cudaMemsetAsync(rowcnt.p, 0, (nn + 1) * 8, st));
+  // the same for one-row clusters; largest first
   for (int q = kRowBins - 1; q >= 0; --q) {
     const int64_t m = tstart[kSortBins + q + 1] - tstart[kSortBins + q];
     if (m <= 0) continue;
@@ -1956,7 +1962,7 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
   PoolBuf crp(ctx);
   SPOPS_TRY(crp.alloc((nn + 1) * 8));
   if (ncl > 0) {
-    row_count_kernel<V><<<grid_for(ncl * 32), 256, 0, st>>>(soff_val.as<int64_t>(), nzd.as<int64_t>(),
+    row_count_kernel<V><<<grid_for(ncl), 256, 0, st>>>(soff_val.as<int64_t>(), nzd.as<int64_t>(),
                                                             offs.as<int64_t>(), perm.as<int64_t>(), ncl, cval.as<V>(),
                                                             rowwise, settled.as<unsigned char>(),
                                                             rowcnt.as<int64_t>());

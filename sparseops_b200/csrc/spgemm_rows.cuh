@@ -4,10 +4,9 @@
 //
 // The method is that of spgemm_sort.cuh: a product's key (output column <<
 // tbits | product index t, flat (j, k) order) is sorted by a bitonic network
-// in registers, so a column's products are adjacent and in flat order.  What
-// differs is everything around the network, which took two thirds of the
-// instructions there (3,900 a row at R = 16, of which the network about
-// 1,100):
+// in registers, so a column's products are adjacent and in flat order.
+// Around the network (two thirds of the instructions, 3,900 a row at R = 16, in
+// a kernel that built its keys slot by slot and wrote from the lanes):
 //   - products are formed in a compact loop over 32*W-product steps, kRowCols
 //     columns of A staged at a time with their values, four steps' loads in
 //     flight, keys and values parked in shared memory;

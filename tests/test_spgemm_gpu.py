@@ -547,3 +547,60 @@ def test_cluster_build_kinds(cuda, orc, itype):
     C = LeSpGEMM_clustered(_csr(*a, ncols), _csr(*b, ncols), perm, offs)
     a64, b64 = (arp.astype(np.int64), aci.astype(np.int64), av), (brp.astype(np.int64), bci.astype(np.int64), bv)
     _check_c(C, orc.spgemm(a64, b64, perm.astype(np.int64), np.array(offs, np.int64)))
+
+
+@pytest.mark.parametrize("itype,vtype,so", [(np.int64, np.float64, 0), (np.int32, np.float64, 1),
+                                            (np.int64, np.float32, 0)])
+def test_cluster_product_count_edges(cuda, itype, vtype, so):
+    """Clusters of 1 to 40 rows with product counts at the limits between the
+    kernel forms; each row but the first holds half of the cluster's columns."""
+    from sparseops_b200.spgemm import LeSpGEMM_clustered
+    rng = np.random.default_rng(91)
+    ncols, nb = 1 << 18, 2000
+    hot = np.arange(0, 300, 3)
+    brows = [np.unique(np.concatenate([rng.choice(hot, int(m)), rng.integers(0, ncols, int(m))]))
+             for m in rng.integers(1, 9, nb)]
+    brows[:200] = [b[:1] for b in brows[:200]]  # one entry each, to reach any count
+    lens = np.array([len(b) for b in brows])
+    brp, bci = np.concatenate([[0], np.cumsum(lens)]), np.concatenate(brows)
+    bv = rng.standard_normal(brp[-1])
+    sizes = [1, 2, 3, 7, 8, 32, 33, 40]
+    arows, offsets, counts = [], [0], []
+    for q in range(5, 14):
+        for P in ((1 << q) - 1, 1 << q, (1 << q) + 1):
+            csz, left, take = sizes[len(counts) % len(sizes)], P, []
+            for r in rng.permutation(np.arange(200, nb)):
+                if lens[r] <= left - 20:
+                    take.append(r)
+                    left -= lens[r]
+            take = np.sort(np.concatenate([take, rng.choice(200, left, replace=False)]).astype(np.int64))
+            assert lens[take].sum() == P
+            counts.append(P)
+            for l in range(csz):
+                arows.append(take if l == 0 else np.sort(rng.choice(take, (len(take) + 1) // 2, replace=False)))
+            offsets.append(offsets[-1] + csz)
+    arp = np.concatenate([[0], np.cumsum([len(r) for r in arows])])
+    aci, av = np.concatenate(arows), rng.standard_normal(arp[-1])
+    av, bv = av.astype(vtype), bv.astype(vtype)
+    perm = rng.permutation(len(arows))  # cluster order -> row of A
+    back = np.argsort(perm)
+    orp = np.concatenate([[0], np.cumsum(np.diff(arp)[back])])
+    oci = np.concatenate([aci[arp[b]:arp[b + 1]] for b in back])
+    ov = np.concatenate([av[arp[b]:arp[b + 1]] for b in back])
+    C = LeSpGEMM_clustered(_csr(orp.astype(itype), oci.astype(itype), ov, nb),
+                           _csr(brp.astype(itype), bci.astype(itype), bv, ncols), perm.astype(np.int64),
+                           np.array(offsets, np.int64), sort_output=bool(so))
+    rp, ci, v = C.host()
+    tol = 1e-12 if vtype == np.float64 else 1e-5
+    for r in range(len(arows)):
+        val, mag = {}, {}
+        for k in range(orp[r], orp[r + 1]):
+            for e in range(brp[oci[k]], brp[oci[k] + 1]):
+                x = float(ov[k]) * float(bv[e])
+                val[bci[e]] = val.get(bci[e], 0.0) + x
+                mag[bci[e]] = mag.get(bci[e], 0.0) + abs(x)
+        want = sorted(val)
+        assert np.array_equal(ci[rp[r]:rp[r + 1]], want)
+        got = v[rp[r]:rp[r + 1]].astype(np.float64)
+        err = np.abs(got - [val[c] for c in want]) / np.array([mag[c] for c in want])
+        assert len(err) == 0 or err.max() <= tol
