@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(THREADS* PER)
     __syncwarp();
   }
   for (int r = lane; r < C.nr; r += 32) parent[rows[r]] = (int32_t)rows[root[r]];
-  overlap_wait();
+  overlap_end();
 }
 
 // (a, b) among the initial pairs (sorted by (i, j))

@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "pdl.cuh"
 #include "spgemm_sort.cuh"
 #include "spops_internal.h"
 
@@ -346,8 +347,9 @@ __global__ void __launch_bounds__(W == 1 ? 128 : 32 * W)
   auto sync = [] {
     if (W == 1) __syncwarp(); else __syncthreads();
   };
+  overlap_let_next();
   const int64_t slot = W == 1 ? blockIdx.x * (int64_t)4 + (threadIdx.x >> 5) : blockIdx.x;
-  if (slot >= nrows) return;  // W == 1: whole warps, which share no barrier
+  if (slot >= nrows) return;  // W == 1: whole warps, which share no barrier, and not the block's first
   const int64_t i = rows[slot];
   int P = 0;
   for (int b0 = 0; b0 < bands; b0 += S::kCols) {
@@ -442,6 +444,7 @@ __global__ void __launch_bounds__(W == 1 ? 128 : 32 * W)
   for (int s = 0; s < R; ++s)
     if (first >> s & 1u) out[rank++] = (int32_t)key[s];
   if (tid == 0) cnt[i] = total;
+  overlap_end();
 }
 
 // The longest rows' pairs as keys i << 32 | j at room[i] - room of the rows
@@ -674,10 +677,9 @@ spops_status_t lsh_pairs(Context* ctx, const uint64_t* sig, int64_t n, int k, in
     const int per = warps == 1 ? 4 : 1;
     SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem * per));
     SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    kern<<<(unsigned)((c + per - 1) / per), warps * per * 32, smem * per, st>>>(
-        lists.as<int32_t>() + (int64_t)bin * n, c, rec.as<uint64_t>(), n, bands, members.as<int32_t>(), droom,
-        part.as<int32_t>(), cnt.as<int64_t>());
-    SPOPS_LAUNCH_CHECK();
+    SPOPS_CUDA(launch_overlapped(kern, (c + per - 1) / per, warps * per * 32, smem * per, st,
+                                 lists.as<int32_t>() + (int64_t)bin * n, c, rec.as<uint64_t>(), n, bands,
+                                 members.as<int32_t>(), droom, part.as<int32_t>(), cnt.as<int64_t>()));
     return SPOPS_OK;
   };
   SPOPS_TRY(launch(lsh_pair_kernel<16, 16>, 7, sizeof(PairSmem<16, 16>), 16));

@@ -19,6 +19,13 @@ namespace {
 
 __device__ __forceinline__ void overlap_let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void overlap_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// For kernels that share nothing with the launch before them: they call
+// overlap_let_next() first, and at their end overlap_end(), where the grid's
+// last block alone waits (a block that waited would keep its place on the SM),
+// so that the grid does not end before the one before it.
+__device__ __forceinline__ void overlap_end() {
+  if (blockIdx.x + 1 == gridDim.x) overlap_wait();
+}
 __device__ __forceinline__ void overlap_begin() {
   overlap_let_next();
   overlap_wait();

@@ -1752,7 +1752,9 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
   SPOPS_CUDA(cudaMemsetAsync(ndense.p, 0, 8, st));
   if (rowwise) SPOPS_CUDA(cudaMemsetAsync(drop.p, 0, ncl1, st));
   const double b_rowdense = (double)B->nnz / (double)std::max<int64_t>(B->rows, 1);
-  for (int q = 0; q < kSortBins; ++q) {
+  // (the clusters' kernels share nothing: each launch overlaps with the end of
+  // the one before it, largest first)
+  for (int q = kSortBins - 1; q >= 0; --q) {
     const int64_t m = tstart[q + 1] - tstart[q];
     if (m <= 0) continue;
     const int64_t* dl = slist.as<int64_t>() + tstart[q];
@@ -1760,13 +1762,13 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
       const int per = warps == 1 ? kGroupPer : 1;
       SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem * per));
       SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-      kern<<<(unsigned)((m + per - 1) / per), warps * per * 32, smem * per, st>>>(
-          dl, m, cptr.as<int64_t>(), cptr_val.as<int64_t>(), colids.as<int32_t>(), avals.as<V>(), offs.as<int64_t>(),
-          perm.as<int64_t>(), B->row.as<I>(), B->col.as<I>(), B->val.as<V>(), b_rowdense, l2_budget, sort_output, rowwise,
+      SPOPS_CUDA(launch_overlapped(
+          kern, (m + per - 1) / per, warps * per * 32, smem * per, st, dl, m, cptr.as<int64_t>(),
+          cptr_val.as<int64_t>(), colids.as<int32_t>(), avals.as<V>(), offs.as<int64_t>(), perm.as<int64_t>(),
+          B->row.as<I>(), B->col.as<I>(), B->val.as<V>(), b_rowdense, l2_budget, sort_output, rowwise,
           soff.as<int64_t>(), soff_val.as<int64_t>(), nzd.as<int64_t>(), cmin.as<int64_t>(), cmax.as<int64_t>(),
           drop.as<unsigned char>(), reinterpret_cast<unsigned long long*>(ndense.p), ccol.as<int32_t>(),
-          cval.as<V>(), rowcnt.as<int64_t>());
-      SPOPS_LAUNCH_CHECK();
+          cval.as<V>(), rowcnt.as<int64_t>()));
       return SPOPS_OK;
     };
     switch (q) {
@@ -1789,13 +1791,12 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
     auto launch = [&](auto kern, size_t smem, int threads) -> spops_status_t {
       SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-      kern<<<(unsigned)m, threads, smem, st>>>(
+      SPOPS_CUDA(launch_overlapped(kern, m, threads, smem, st,
           dl, cptr.as<int64_t>(), cptr_val.as<int64_t>(), colids.as<int32_t>(), avals.as<V>(), offs.as<int64_t>(),
           perm.as<int64_t>(), B->row.as<I>(), B->col.as<I>(), B->val.as<V>(), b_rowdense, l2_budget, sort_output,
           rowwise, soff.as<int64_t>(), soff_val.as<int64_t>(), nzd.as<int64_t>(), cmin.as<int64_t>(),
           cmax.as<int64_t>(), drop.as<unsigned char>(), reinterpret_cast<unsigned long long*>(ndense.p),
-          ccol.as<int32_t>(), cval.as<V>(), rowcnt.as<int64_t>());
-      SPOPS_LAUNCH_CHECK();
+          ccol.as<int32_t>(), cval.as<V>(), rowcnt.as<int64_t>()));
       return SPOPS_OK;
     };
     switch (q) {

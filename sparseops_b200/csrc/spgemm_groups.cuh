@@ -22,6 +22,7 @@
 
 #include <cstdint>
 
+#include "pdl.cuh"
 #include "spgemm_sort.cuh"
 
 namespace spops {
@@ -77,8 +78,9 @@ __global__ void __launch_bounds__(W == 1 ? 32 * kGroupPer : 32 * W)
   auto sync = [] {
     if (W == 1) __syncwarp(); else __syncthreads();
   };
+  overlap_let_next();
   const int64_t slot = W == 1 ? blockIdx.x * (int64_t)kGroupPer + (threadIdx.x >> 5) : blockIdx.x;
-  if (slot >= nlist) return;  // W == 1: whole warps, which share no barrier
+  if (slot >= nlist) return;  // W == 1: whole warps, which share no barrier, and not the block's first
   const int64_t c = list[slot];
   const int64_t j0 = cptr[c], vbase = cptr_val[c];
   const int nj = (int)(cptr[c + 1] - j0);
@@ -284,14 +286,14 @@ __global__ void __launch_bounds__(W == 1 ? 32 * kGroupPer : 32 * W)
       }
     }
   }
-  if (!count) return;
   if (csz == 1) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, o);
     if (lane == 0) atomicAdd(&M.kept[0], mine);
   }
   sync();
-  if (tid < rows) rowcnt[perm[offsets[c] + tid]] = M.kept[tid];
+  if (count && tid < rows) rowcnt[perm[offsets[c] + tid]] = M.kept[tid];
+  overlap_end();
 }
 
 }  // namespace

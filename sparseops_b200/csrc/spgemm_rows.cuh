@@ -31,6 +31,7 @@
 
 #include <cstdint>
 
+#include "pdl.cuh"
 #include "spgemm_sort.cuh"
 
 namespace spops {
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(32 * W)
   auto sync = [] {
     if (W == 1) __syncwarp(); else __syncthreads();
   };
+  overlap_let_next();
   const int64_t c = list[blockIdx.x];
   const int64_t j0 = cptr[c], vbase = cptr_val[c];
   const int nj = (int)(cptr[c + 1] - j0);
@@ -298,6 +300,7 @@ __global__ void __launch_bounds__(32 * W)
     rowcnt[perm[offsets[c]]] = kept;
     if (dense && !rowwise) atomicAdd(ndense, 1ULL);
   }
+  overlap_end();
 }
 
 }  // namespace

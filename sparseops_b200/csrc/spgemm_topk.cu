@@ -32,6 +32,7 @@
 #include <numeric>
 #include <vector>
 
+#include "pdl.cuh"
 #include "spgemm_sort.cuh"
 #include "spops_internal.h"
 
@@ -276,6 +277,7 @@ __global__ void __launch_bounds__(32 * W)
   auto sync = [] {
     if (W == 1) __syncwarp(); else __syncthreads();
   };
+  overlap_let_next();
   const int64_t i = rows[blockIdx.x];
   const int64_t a0 = arp[i];
   const int64_t nj = (int64_t)arp[i + 1] - a0;
@@ -419,6 +421,7 @@ __global__ void __launch_bounds__(32 * W)
     tcol[i * k + lane] = (I)(top.bc == kNoCol ? 0 : top.bc);
   }
   if (lane == 0) kept[i] = n - 1 < k ? n - 1 : k;  // j = i is one of the n
+  overlap_end();
 }
 
 // adds one to j's count; returns the slot, plus kFreshSlot when j was not in
@@ -761,10 +764,9 @@ spops_status_t topk_fused_t(Context* ctx, Matrix* A, int k, Matrix** out, bool* 
     if (cnt == 0 || k == 0) return SPOPS_OK;  // k = 0 keeps nothing
     SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    kern<<<(unsigned)cnt, warps * 32, smem, st>>>(L + (int64_t)bin * n, A->row.as<I>(), A->col.as<I>(), trp.as<I>(),
-                                                  tci.as<I>(), k, skey.as<uint64_t>(), scol.as<I>(),
-                                                  kept.as<int64_t>());
-    SPOPS_LAUNCH_CHECK();
+    SPOPS_CUDA(launch_overlapped(kern, cnt, warps * 32, smem, st, L + (int64_t)bin * n, A->row.as<I>(),
+                                 A->col.as<I>(), trp.as<I>(), tci.as<I>(), k, skey.as<uint64_t>(), scol.as<I>(),
+                                 kept.as<int64_t>()));
     return SPOPS_OK;
   };
   SPOPS_TRY(launch(topk_sort_kernel<I, V, 16, 16>, 7, sizeof(TopSmem<16, 16>), 16));

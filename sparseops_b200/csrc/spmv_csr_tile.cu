@@ -152,7 +152,8 @@ __device__ __forceinline__ void chain_arrive(int lane, int who, int64_t o, int32
   int last = 0;
   if (lane == who) {
     __threadfence();  // the part before the count
-    last = atomicAdd(counter + o, 1) == m;
+    // wraps to 0 for the next launch, also when two launches overlapped
+    last = atomicInc(reinterpret_cast<unsigned*>(counter + o), (unsigned)m) == (unsigned)m;
     if (last) __threadfence();  // every part is there: read them past L1
   }
   if (!__shfl_sync(0xffffffffu, last, who)) return;
@@ -162,10 +163,7 @@ __device__ __forceinline__ void chain_arrive(int lane, int who, int64_t o, int32
   const int64_t r = __ldcg(reinterpret_cast<const long long*>(open_row + o));
 #pragma unroll
   for (int q = 16; q > 0; q >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, q);
-  if (lane == 0) {
-    axpby_store(y + r, open + tot, alpha, beta, bz);
-    counter[o] = 0;  // for the next launch
-  }
+  if (lane == 0) axpby_store(y + r, open + tot, alpha, beta, bz);
 }
 
 template <typename I, typename V, int K, int kMinBlocks>
