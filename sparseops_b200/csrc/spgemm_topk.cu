@@ -245,8 +245,8 @@ __host__ __device__ constexpr int64_t top_bin_max(int bin) { return (int64_t)64 
 // tables in shared memory (a probe and an atomic add per product, two block
 // barriers per row for more than 512 products), k = 16 on 131,072 rows of 8 to
 // 40 planted entries, fp64, int64: 128 < P <= 512 675 -> 500 us,
-// 512 < P <= 2048 1128 -> 600 us, the rest 193 -> 178 us, the whole call 2.28 ->
-// 1.48 ms.  Bound by the sort's and the gather's instructions, as
+// 512 < P <= 2048 1128 -> 600 us, the rest 193 -> 178 us, the whole call 2.29 ->
+// 1.48 ms, and 1.37 with the forms' launches overlapping.  Bound by the sort's and the gather's instructions, as
 // row_sort_kernel is; forms of 16 keys per lane because a warp's sort costs
 // about the same per key up to there and needs no barrier.
 template <int R, int W>
