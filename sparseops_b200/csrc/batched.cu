@@ -30,6 +30,7 @@
 
 #include "device_util.cuh"
 #include "csr_tile.cuh"
+#include "launch_util.h"
 #include "spops_internal.h"
 #include "warp_work.cuh"
 
@@ -338,39 +339,15 @@ constexpr size_t spmm_smem(int threads) {
   return (size_t)(threads / 32) * sizeof(SpmmStage<I, V>);
 }
 
-template <typename K>
-int occupancy(K kernel, int threads, size_t smem = 0) {
-  int bps = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, threads, smem) != cudaSuccess || bps < 1) return 1;
-  return bps;
-}
-
-// Resident blocks per SM of a kernel with `smem` bytes of dynamic shared
-// memory, the attribute set once per instantiation and device; 0 when it
-// cannot be set.
-constexpr int kMaxDevices = 64;
-
-template <typename K>
-int blocks_per_sm(K kern, int threads, size_t smem, int* cache) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) dev = 0;
-  if (cache[dev] == 0) {
-    if (smem && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return 0;
-    cache[dev] = occupancy(kern, threads, smem);
-  }
-  return cache[dev];
-}
-
 template <typename I, typename V, int KT>
 int spmm_blocks_per_sm() {
-  static int cache[kMaxDevices];
+  static std::atomic<int> cache[kMaxDevices];
   return blocks_per_sm(spmm_kernel<I, V, KT>, 256, spmm_smem<I, V>(256), cache);
 }
 
 template <typename I, typename V, int KT, bool kBand = false>
 int batch_blocks_per_sm() {
-  static int cache[kMaxDevices];
+  static std::atomic<int> cache[kMaxDevices];
   return blocks_per_sm(batch_kernel<I, V, KT, kBand>, kBatchBlock, KT == 1 ? 0 : spmm_smem<I, V>(kBatchBlock), cache);
 }
 
@@ -570,7 +547,7 @@ spops_status_t build_table(Batch* B) {
 
 template <typename I, typename V>
 int tile1_blocks_per_sm() {
-  static int cache[kMaxDevices];
+  static std::atomic<int> cache[kMaxDevices];
   return blocks_per_sm(batch_tile1_kernel<I, V>, kBatchBlock, 0, cache);
 }
 
@@ -603,7 +580,7 @@ constexpr size_t tile_smem() {
 
 template <typename I, typename V, int G, bool kVec, bool kStage>
 int tile_blocks_per_sm() {
-  static int cache[kMaxDevices];
+  static std::atomic<int> cache[kMaxDevices];
   return blocks_per_sm(batch_tile_kernel<I, V, G, kVec, kStage>, kBatchBlock, tile_smem<I, V, G, kStage>(), cache);
 }
 

@@ -28,6 +28,7 @@
 #include <cub/cub.cuh>
 
 #include "device_util.cuh"
+#include "launch_util.h"
 #include "spops_internal.h"
 #include "warp_work.cuh"
 
@@ -218,14 +219,10 @@ spops_status_t analyse_t(Context* ctx, Matrix* A) {
 template <typename I, typename V, int kItems, int kMinBlocks>
 spops_status_t launch_warp(Context* ctx, Matrix* A, double alpha, const void* x, double beta, void* y) {
   const CsrPlan& P = A->plan;
-  static int blocks_per_sm = -1;  // per instantiation
-  if (blocks_per_sm < 0) {
-    int bps = 0;
-    SPOPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, csr_warp_kernel<I, V, kItems, kMinBlocks>,
-                                                             kBlock, 0));
-    blocks_per_sm = bps > 0 ? bps : 1;
-  }
-  int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
+  static std::atomic<int> cache[kMaxDevices];
+  const int bps = blocks_per_sm(csr_warp_kernel<I, V, kItems, kMinBlocks>, kBlock, 0, cache);
+  if (bps < 1) return fail(SPOPS_ERR_CUDA, "csr: kernel attributes could not be set");
+  int64_t grid = (int64_t)ctx->num_sms * bps;
   const int64_t need = (P.nblocks + kBlock / 32 - 1) / (kBlock / 32);
   if (grid > need) grid = need;
   csr_warp_kernel<I, V, kItems, kMinBlocks><<<(unsigned)grid, kBlock, 0, ctx->stream>>>(

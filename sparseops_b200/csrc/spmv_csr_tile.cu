@@ -38,6 +38,7 @@
 #include "bulk_copy.cuh"
 #include "csr_tile.cuh"
 #include "device_util.cuh"
+#include "launch_util.h"
 #include "pdl.cuh"
 #include "spops_internal.h"
 
@@ -616,14 +617,10 @@ spops_status_t spmm_tiles_f(Context* ctx, Matrix* A, double alpha, const void* X
   if (D.tiles > 0) {
     auto* kern = csr_tile_spmm_kernel<I, V, G, J, kVec, kStage, kFull>;
     constexpr size_t smem = !kStage ? 0 : 2 * (kTileBlock / 32) * sizeof(SpmmTile<I, V, G>);
-    static int blocks_per_sm = -1;  // per instantiation
-    if (blocks_per_sm < 0) {
-      int bps = 0;
-      SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      SPOPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, kTileBlock, smem));
-      blocks_per_sm = bps > 0 ? bps : 1;
-    }
-    int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
+    static std::atomic<int> cache[kMaxDevices];
+    const int bps = blocks_per_sm(kern, kTileBlock, smem, cache);
+    if (bps < 1) return fail(SPOPS_ERR_CUDA, "spmm: kernel attributes could not be set");
+    int64_t grid = (int64_t)ctx->num_sms * bps;
     const int64_t need = (D.tiles + kTileBlock / 32 - 1) / (kTileBlock / 32);
     if (grid > need) grid = need;
     SPOPS_CUDA(launch_overlapped(kern, grid, kTileBlock, smem, ctx->stream,
@@ -761,14 +758,10 @@ spops_status_t spmv_range(Context* ctx, Matrix* A, double alpha, const void* x, 
   const CsrTiles& D = A->plan.tiles;
   const bool bz = beta == 0.0;
   if (t1 > t0) {
-    static int blocks_per_sm = -1;  // per instantiation
-    if (blocks_per_sm < 0) {
-      int bps = 0;
-      SPOPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, csr_tile_kernel<I, V, K, kMinBlocks, kPipe>,
-                                                               kTileBlock, 0));
-      blocks_per_sm = bps > 0 ? bps : 1;
-    }
-    int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
+    static std::atomic<int> cache[kMaxDevices];
+    const int bps = blocks_per_sm(csr_tile_kernel<I, V, K, kMinBlocks, kPipe>, kTileBlock, 0, cache);
+    if (bps < 1) return fail(SPOPS_ERR_CUDA, "csr: kernel attributes could not be set");
+    int64_t grid = (int64_t)ctx->num_sms * bps;
     const int64_t need = (t1 - t0 + kTileBlock / 32 - 1) / (kTileBlock / 32);
     if (grid > need) grid = need;
     SPOPS_CUDA(launch_overlapped(csr_tile_kernel<I, V, K, kMinBlocks, kPipe>, grid, kTileBlock, 0, ctx->stream,
@@ -796,16 +789,10 @@ spops_status_t spmv_stage_t(Context* ctx, Matrix* A, double alpha, const void* x
   if (tiles > 0) {
     SPOPS_TRY(ctx->ensure_errword());
     constexpr size_t smem = kStageWarps * sizeof(StageRing<I, V, S>);
-    static int blocks_per_sm = -1;  // per instantiation
-    if (blocks_per_sm < 0) {
-      SPOPS_CUDA(cudaFuncSetAttribute(csr_stage_kernel<I, V, S, kMinBlocks>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      int bps = 0;
-      SPOPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, csr_stage_kernel<I, V, S, kMinBlocks>,
-                                                               kStageWarps * 32, smem));
-      blocks_per_sm = bps > 0 ? bps : 1;
-    }
-    int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
+    static std::atomic<int> cache[kMaxDevices];
+    const int bps = blocks_per_sm(csr_stage_kernel<I, V, S, kMinBlocks>, kStageWarps * 32, smem, cache);
+    if (bps < 1) return fail(SPOPS_ERR_CUDA, "csr: kernel attributes could not be set");
+    int64_t grid = (int64_t)ctx->num_sms * bps;
     const int64_t need = (tiles + kStageWarps - 1) / kStageWarps;
     if (grid > need) grid = need;
     csr_stage_kernel<I, V, S, kMinBlocks><<<(unsigned)grid, kStageWarps * 32, smem, ctx->stream>>>(
@@ -840,13 +827,10 @@ inline bool one_launch(const Context* ctx, const Matrix* A) {
 template <typename I, typename V>
 spops_status_t spmv_one_t(Context* ctx, Matrix* A, double alpha, const void* x, double beta, void* y) {
   const CsrTiles& D = A->plan.tiles;
-  static int blocks_per_sm = -1;  // per instantiation
-  if (blocks_per_sm < 0) {
-    int bps = 0;
-    SPOPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, csr_tile_one_kernel<I, V, 8, 3>, kTileBlock, 0));
-    blocks_per_sm = bps > 0 ? bps : 1;
-  }
-  int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
+  static std::atomic<int> cache[kMaxDevices];
+  const int bps = blocks_per_sm(csr_tile_one_kernel<I, V, 8, 3>, kTileBlock, 0, cache);
+  if (bps < 1) return fail(SPOPS_ERR_CUDA, "csr: kernel attributes could not be set");
+  int64_t grid = (int64_t)ctx->num_sms * bps;
   const int64_t need = std::max((D.tiles + kTileBlock / 32 - 1) / (kTileBlock / 32),
                                 (D.nempty + kTileBlock - 1) / kTileBlock);
   if (grid > need) grid = need;
@@ -886,13 +870,10 @@ spops_status_t spmv_indirect_t(Context* ctx, Matrix* A, const int64_t* perm, con
   const bool bz = beta == 0.0;
   const int64_t tiles = D.tiles;
   if (tiles > 0) {
-    static int blocks_per_sm = -1;  // per instantiation
-    if (blocks_per_sm < 0) {
-      int bps = 0;
-      SPOPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, csr_tile_indirect_kernel<I, V>, kTileBlock, 0));
-      blocks_per_sm = bps > 0 ? bps : 1;
-    }
-    int64_t grid = (int64_t)ctx->num_sms * blocks_per_sm;
+    static std::atomic<int> cache[kMaxDevices];
+    const int bps = blocks_per_sm(csr_tile_indirect_kernel<I, V>, kTileBlock, 0, cache);
+    if (bps < 1) return fail(SPOPS_ERR_CUDA, "csr: kernel attributes could not be set");
+    int64_t grid = (int64_t)ctx->num_sms * bps;
     const int64_t need = (tiles + kTileBlock / 32 - 1) / (kTileBlock / 32);
     if (grid > need) grid = need;
     SPOPS_CUDA(launch_overlapped(csr_tile_indirect_kernel<I, V>, grid, kTileBlock, 0, ctx->stream,
