@@ -715,14 +715,15 @@ spops_status_t hc_device_t(Context* ctx, Matrix* A, const int64_t* pi, const int
     SPOPS_CUDA(cudaMemcpyAsync(hc, count, 32, cudaMemcpyDeviceToHost, st));
     SPOPS_CUDA(cudaStreamSynchronize(st));
     rest = (int64_t)hc[2];
+    OverlapChain chain(st);
     auto launch = [&](auto kern, const Comp* list, int64_t step, int64_t m, int threads, int per,
                       size_t sm) -> spops_status_t {
       if (m <= 0) return SPOPS_OK;
       SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm * per));
       SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-      SPOPS_CUDA(launch_overlapped(kern, (m + per - 1) / per, threads * per, sm * per, st, list, step, m,
-                                   pid.as<uint32_t>(), rid.as<uint32_t>(), pi, pj, ps, cluster_size, A->row.as<I>(),
-                                   A->col.as<I>(), parent.as<int32_t>()));
+      SPOPS_CUDA(chain.launch(kern, (m + per - 1) / per, threads * per, sm * per, list, step, m,
+                              pid.as<uint32_t>(), rid.as<uint32_t>(), pi, pj, ps, cluster_size, A->row.as<I>(),
+                              A->col.as<I>(), parent.as<int32_t>()));
       return SPOPS_OK;
     };
     // the longest blocks first

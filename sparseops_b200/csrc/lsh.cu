@@ -671,15 +671,16 @@ spops_status_t lsh_pairs(Context* ctx, const uint64_t* sig, int64_t n, int k, in
   SPOPS_TRY(part.alloc((size_t)rooms * 4));
   tr.mark(st, "rows");
   const int64_t* droom = off.as<int64_t>();
+  OverlapChain chain(st);
   auto launch = [&](auto kern, int bin, size_t smem, int warps) -> spops_status_t {
     const int64_t c = (int64_t)hb[bin];
     if (c == 0) return SPOPS_OK;
     const int per = warps == 1 ? 4 : 1;
     SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem * per));
     SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    SPOPS_CUDA(launch_overlapped(kern, (c + per - 1) / per, warps * per * 32, smem * per, st,
-                                 lists.as<int32_t>() + (int64_t)bin * n, c, rec.as<uint64_t>(), n, bands,
-                                 members.as<int32_t>(), droom, part.as<int32_t>(), cnt.as<int64_t>()));
+    SPOPS_CUDA(chain.launch(kern, (c + per - 1) / per, warps * per * 32, smem * per,
+                            lists.as<int32_t>() + (int64_t)bin * n, c, rec.as<uint64_t>(), n, bands,
+                            members.as<int32_t>(), droom, part.as<int32_t>(), cnt.as<int64_t>()));
     return SPOPS_OK;
   };
   SPOPS_TRY(launch(lsh_pair_kernel<16, 16>, 7, sizeof(PairSmem<16, 16>), 16));

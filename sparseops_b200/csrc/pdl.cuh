@@ -19,10 +19,10 @@ namespace {
 
 __device__ __forceinline__ void overlap_let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void overlap_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// For kernels that share nothing with the launch before them: they call
-// overlap_let_next() first, and at their end overlap_end(), where the grid's
-// last block alone waits (a block that waited would keep its place on the SM),
-// so that the grid does not end before the one before it.
+// For the kernels of an OverlapChain, which share nothing with one another:
+// they call overlap_let_next() first, and at their end overlap_end(), where the
+// grid's last block alone waits (a block that waited would keep its place on the
+// SM), so that the grid does not end before the one before it.
 __device__ __forceinline__ void overlap_end() {
   if (blockIdx.x + 1 == gridDim.x) overlap_wait();
 }
@@ -31,8 +31,15 @@ __device__ __forceinline__ void overlap_begin() {
   overlap_wait();
 }
 
+template <typename... P>
+cudaError_t launch_packed(const cudaLaunchConfig_t* cfg, const void* kern, P... args) {
+  void* list[] = {(void*)&args...};
+  return cudaLaunchKernelExC(cfg, kern, list);
+}
+
 template <typename... P, typename... A>
-cudaError_t launch_overlapped(void (*kern)(P...), int64_t grid, int block, size_t smem, cudaStream_t st, A... args) {
+cudaError_t launch_with(int overlapped, void (*kern)(P...), int64_t grid, int block, size_t smem, cudaStream_t st,
+                        A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
@@ -42,9 +49,30 @@ cudaError_t launch_overlapped(void (*kern)(P...), int64_t grid, int block, size_
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  cfg.numAttrs = overlapped ? 1 : 0;
+  return launch_packed(&cfg, reinterpret_cast<const void*>(kern), static_cast<P>(args)...);
 }
+
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(void (*kern)(P...), int64_t grid, int block, size_t smem, cudaStream_t st, A... args) {
+  return launch_with(1, kern, grid, block, smem, st, args...);
+}
+
+// Launches that share nothing with one another and do not wait.  The first is
+// a plain one: it begins when all work queued before it has ended, with its
+// writes visible (the fills and copies of what the kernels read or add to), and
+// since the later ones begin after it has, the same holds for them.
+struct OverlapChain {
+  cudaStream_t st;
+  bool begun = false;
+  explicit OverlapChain(cudaStream_t s) : st(s) {}
+  template <typename... P, typename... A>
+  cudaError_t launch(void (*kern)(P...), int64_t grid, int block, size_t smem, A... args) {
+    const int overlapped = begun ? 1 : 0;
+    begun = true;
+    return launch_with(overlapped, kern, grid, block, smem, st, args...);
+  }
+};
 
 }  // namespace
 }  // namespace spops

@@ -1754,6 +1754,7 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
   const double b_rowdense = (double)B->nnz / (double)std::max<int64_t>(B->rows, 1);
   // (the clusters' kernels share nothing: each launch overlaps with the end of
   // the one before it, largest first)
+  OverlapChain chain(st);
   for (int q = kSortBins - 1; q >= 0; --q) {
     const int64_t m = tstart[q + 1] - tstart[q];
     if (m <= 0) continue;
@@ -1762,8 +1763,8 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
       const int per = warps == 1 ? kGroupPer : 1;
       SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem * per));
       SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-      SPOPS_CUDA(launch_overlapped(
-          kern, (m + per - 1) / per, warps * per * 32, smem * per, st, dl, m, cptr.as<int64_t>(),
+      SPOPS_CUDA(chain.launch(
+          kern, (m + per - 1) / per, warps * per * 32, smem * per, dl, m, cptr.as<int64_t>(),
           cptr_val.as<int64_t>(), colids.as<int32_t>(), avals.as<V>(), offs.as<int64_t>(), perm.as<int64_t>(),
           B->row.as<I>(), B->col.as<I>(), B->val.as<V>(), b_rowdense, l2_budget, sort_output, rowwise,
           soff.as<int64_t>(), soff_val.as<int64_t>(), nzd.as<int64_t>(), cmin.as<int64_t>(), cmax.as<int64_t>(),
@@ -1791,7 +1792,7 @@ spops_status_t spgemm_t(Context* ctx, Matrix* A, Matrix* B, const int64_t* perm_
     auto launch = [&](auto kern, size_t smem, int threads) -> spops_status_t {
       SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-      SPOPS_CUDA(launch_overlapped(kern, m, threads, smem, st,
+      SPOPS_CUDA(chain.launch(kern, m, threads, smem,
           dl, cptr.as<int64_t>(), cptr_val.as<int64_t>(), colids.as<int32_t>(), avals.as<V>(), offs.as<int64_t>(),
           perm.as<int64_t>(), B->row.as<I>(), B->col.as<I>(), B->val.as<V>(), b_rowdense, l2_budget, sort_output,
           rowwise, soff.as<int64_t>(), soff_val.as<int64_t>(), nzd.as<int64_t>(), cmin.as<int64_t>(),

@@ -759,14 +759,15 @@ spops_status_t topk_fused_t(Context* ctx, Matrix* A, int k, Matrix** out, bool* 
   SPOPS_TRY(ctx->ensure_errword());
   int* err = ctx->errword.as<int>();
   const int32_t* L = lists.as<int32_t>();
+  OverlapChain chain(st);
   auto launch = [&](auto kern, int bin, size_t smem, int warps) -> spops_status_t {
     const int64_t cnt = (int64_t)hb[bin];
     if (cnt == 0 || k == 0) return SPOPS_OK;  // k = 0 keeps nothing
     SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     SPOPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    SPOPS_CUDA(launch_overlapped(kern, cnt, warps * 32, smem, st, L + (int64_t)bin * n, A->row.as<I>(),
-                                 A->col.as<I>(), trp.as<I>(), tci.as<I>(), k, skey.as<uint64_t>(), scol.as<I>(),
-                                 kept.as<int64_t>()));
+    SPOPS_CUDA(chain.launch(kern, cnt, warps * 32, smem, L + (int64_t)bin * n, A->row.as<I>(),
+                            A->col.as<I>(), trp.as<I>(), tci.as<I>(), k, skey.as<uint64_t>(), scol.as<I>(),
+                            kept.as<int64_t>()));
     return SPOPS_OK;
   };
   SPOPS_TRY(launch(topk_sort_kernel<I, V, 16, 16>, 7, sizeof(TopSmem<16, 16>), 16));

@@ -1,4 +1,5 @@
-"""How kernels are launched: per-device launch attributes."""
+"""How kernels are launched: per-device launch attributes, and overlapped
+launches that begin only when they may."""
 import glob
 import os
 import re
@@ -30,6 +31,35 @@ def test_launch_helpers_against_a_fake_runtime(tmp_path):
                     os.path.join(ROOT, "tests", "cpp", "launch_test.cpp")], check=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_overlapped_launches_wait_or_belong_to_a_chain():
+    """A kernel launched by launch_overlapped waits (overlap_begin, or
+    overlap_wait after its plan's loads); one that does not wait until its end
+    (overlap_end) is launched through an OverlapChain, whose first launch is a
+    plain one."""
+    def kernels(pattern):  # names of the kernels whose body calls it
+        out = set()
+        for path in glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")):
+            if path.endswith("pdl.cuh"):
+                continue
+            text = open(path).read()
+            for m in re.finditer(pattern, text):
+                head = text[:m.start()]
+                out.add(re.findall(r"(\w+_kernel)\(", head[head.rindex("__global__"):])[0])
+        return out
+
+    late = kernels(r"overlap_end\(\)")
+    assert late
+    for path in glob.glob(os.path.join(CSRC, "*.cu")):
+        text = open(path).read()
+        for m in re.finditer(r"launch_overlapped\(\s*(\w+)", text):
+            name = m.group(1)
+            if name == "kern":  # a local: the last kernel named before it
+                name = re.findall(r"auto\*? kern = (\w+_kernel)|OverlapChain|auto kern\b", text[:m.start()])[-1]
+            assert name.endswith("_kernel") and name not in late, (os.path.basename(path), m.group(0), name)
+    waits = kernels(r"overlap_begin\(\)|overlap_wait\(\)")
+    assert not waits & late
 
 
 @pytest.mark.gpu
