@@ -262,9 +262,10 @@ __global__ void __launch_bounds__(kBatchBlock, 2) batch_tile1_kernel(const Batch
       uint32_t flags = M.tflags[t * 32 + lane];
       int64_t tr = M.tile_row[t];
       for (; t < t1; ++t) {
-        V pr[K];
+        V pr[K], xv[K];
+        gather_run<I, V, K>(x, c, M.nnz, t, lane, xv);
 #pragma unroll
-        for (int b = 0; b < K; ++b) pr[b] = a[b] * ld_gather(x + c[b]);
+        for (int b = 0; b < K; ++b) pr[b] = a[b] * xv[b];
         const uint32_t f = flags;
         const int64_t r0 = tr;
         if (t + 1 < t1) {

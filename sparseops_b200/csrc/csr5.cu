@@ -75,7 +75,7 @@ __global__ void csr5_build_kernel(const I* __restrict__ rp, const I* __restrict_
       tcol[dst] = ci[e];
       tval[dst] = v[e];
     } else {
-      tcol[dst] = 0;
+      tcol[dst] = -1;  // past the end: nothing of x is read
       tval[dst] = V(0);
     }
   }
@@ -131,7 +131,10 @@ __global__ void __launch_bounds__(256) csr5_kernel(const I* __restrict__ rp, int
   const V* tv = tval + t * kTile + lane;
   V prod[kSigma];
 #pragma unroll
-  for (int s = 0; s < kSigma; ++s) prod[s] = ld_stream(tv + s * kOmega) * ld_gather(x + ld_stream(tc + s * kOmega));
+  for (int s = 0; s < kSigma; ++s) {
+    const I c = ld_stream(tc + s * kOmega);
+    prod[s] = ld_stream(tv + s * kOmega) * (c >= 0 ? ld_gather(x + c) : V(0));  // 0 * x[0] may be NaN
+  }
 #pragma unroll
   for (int s = 0; s < kSigma; ++s) {
     if (s > 0 && (flags >> s) & 1u) {  // a new row starts at step s

@@ -119,9 +119,10 @@ __global__ void __launch_bounds__(kTileBlock, kMinBlocks) csr_tile_kernel(
       flags = flags_all[t * 32 + lane];
       tr = tile_row[t];
     }
-    V p[K];
+    V p[K], xv[K];
+    gather_run<I, V, K>(x, c, nnz, t, lane, xv);
 #pragma unroll
-    for (int b = 0; b < K; ++b) p[b] = a[b] * ld_gather(x + c[b]);
+    for (int b = 0; b < K; ++b) p[b] = a[b] * xv[b];
     const uint32_t f = flags;
     const int64_t r0 = tr;
     if (kPipe && t + nw < tiles) {
@@ -445,8 +446,7 @@ __global__ void __launch_bounds__(kStageWarps * 32, kMinBlocks) csr_stage_kernel
   int s = 0;
   if (t < full && !wait(0)) return give_up();
   columns(t, 0);
-#pragma unroll
-  for (int b = 0; b < K; ++b) xv[b] = ld_gather(x + c[b]);
+  gather_run<I, V, K>(x, c, nnz, t, lane, xv);
   while (true) {
     const int64_t tn = t + nw;
     const int sn = s + 1 == S ? 0 : s + 1;
@@ -466,8 +466,7 @@ __global__ void __launch_bounds__(kStageWarps * 32, kMinBlocks) csr_stage_kernel
     if (more) {
       if (tn < full && !wait(sn)) return give_up();
       columns(tn, sn);
-#pragma unroll
-      for (int b = 0; b < K; ++b) xn[b] = ld_gather(x + c[b]);
+      gather_run<I, V, K>(x, c, nnz, tn, lane, xn);
     }
     __syncwarp();  // every lane is done with slot s
     if (t + S * nw < tiles) {
@@ -526,12 +525,11 @@ __global__ void __launch_bounds__(kTileBlock, 3) csr_tile_indirect_kernel(
   load(t);
   for (; t < tiles; t += nw) {
     const int64_t el = t * (32 * K) + (int64_t)lane * K;
-    V p[K];
+    V p[K], a[K], xv[K];
+    gather_run<int64_t, V, K>(vsrc, pm, nnz, t, lane, a);
+    gather_run<I, V, K>(x, c, nnz, t, lane, xv);
 #pragma unroll
-    for (int b = 0; b < K; ++b) {
-      const V a = el + b < nnz ? ld_gather(vsrc + pm[b]) : V(0);
-      p[b] = a * ld_gather(x + c[b]);
-    }
+    for (int b = 0; b < K; ++b) p[b] = a[b] * xv[b];
     const uint32_t f = flags;
     const int64_t r0 = tr;
     if (t + nw < tiles) load(t + nw);
