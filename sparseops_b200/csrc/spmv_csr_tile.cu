@@ -218,9 +218,13 @@ __global__ void __launch_bounds__(kTileBlock, kMinBlocks) csr_tile_one_kernel(
     const unsigned starts = __ballot_sync(0xffffffffu, flags != 0);
     const bool mine = T.owner >= 0 || ((starts << (31 - lane)) != 0);
     V p[K], ts = V(0);
+    // (x is masked, not the product, which may then be fused into its row's sum;
+    // an infinite value of another tile's entry only reaches E.cin, unused there)
 #pragma unroll
-    for (int b = 0; b < K; ++b)
-      p[b] = mine && t * (32 * K) + (int64_t)lane * K + b < nnz ? a[b] * ld_gather(x + c[b]) : V(0);
+    for (int b = 0; b < K; ++b) {
+      const V xb = mine && t * (32 * K) + (int64_t)lane * K + b < nnz ? ld_gather(x + c[b]) : V(0);
+      p[b] = a[b] * xb;
+    }
     {
       const V xt = ld_gather(x + ct);
       if (lane < T.tail) ts = at * xt;
@@ -238,10 +242,7 @@ __global__ void __launch_bounds__(kTileBlock, kMinBlocks) csr_tile_one_kernel(
       for (int q = 0; q < kTailMax / 32 - 1; ++q)
         if (32 * q < m) ts += val[e + 32 * q] * xt[q];
     }
-    if (t + nw < tiles) {
-      load_pattern(t + nw);
-      load_values(t + nw);
-    }
+    if (t + nw < tiles) load_pattern(t + nw);
     const TileEnds<V> E = tile_sums<I, V, K>(rp, n, nnz, t, lane, f, r0, p, y, alpha, beta, bz);
     if (T0.tail > 0) {
 #pragma unroll
@@ -262,6 +263,7 @@ __global__ void __launch_bounds__(kTileBlock, kMinBlocks) csr_tile_one_kernel(
       chain_arrive<V>(lane, 0, T0.owner, tails[T0.owner].chain, counter, carry_in, open_sum, open_row, y, alpha, beta,
                       bz);
     }
+    if (t + nw < tiles) load_values(t + nw);  // beside the gathers; earlier, they and this tile's would spill
   }
 }
 
