@@ -604,3 +604,31 @@ def test_cluster_product_count_edges(cuda, itype, vtype, so):
         got = v[rp[r]:rp[r + 1]].astype(np.float64)
         err = np.abs(got - [val[c] for c in want]) / np.array([mag[c] for c in want])
         assert len(err) == 0 or err.max() <= tol
+
+
+@pytest.mark.parametrize("vtype", [np.float32, np.float64])
+@pytest.mark.parametrize("terms", [2, 3, 4, 7])
+def test_clustered_products_are_fused(cuda, vtype, terms):
+    """A cluster of several rows adds a column's products in flat order, each
+    fused into the sum: the low half of the last product survives the first
+    one's cancellation (separately rounded it is lost)."""
+    import torch
+    from sparseops_b200 import CSR_Matrix
+    from sparseops_b200.spgemm import LeSpGEMM_clustered
+    h = vtype(2) ** (-12 if vtype == np.float32 else -27)
+    a = vtype(1024) * (1 + h)
+    first, low = -(vtype(1024) ** 2) * (1 + 2 * h), (vtype(1024) * h) ** 2  # a * a = low - first
+    A = np.zeros((2, terms), vtype)
+    A[0, 0], A[0, -1], A[1] = first, a, 2
+    B = np.zeros((terms, 1), vtype)
+    B[0], B[-1] = 1, a
+    A[:, 1:-1] = 0.0
+    rp = np.array([0, terms, 2 * terms], np.int64)
+    ci = np.tile(np.arange(terms, dtype=np.int64), 2)
+    dev = lambda *x: [torch.from_numpy(np.ascontiguousarray(t)).to("cuda") for t in x]
+    MA = CSR_Matrix(2, terms, *dev(rp, ci, A.reshape(-1)))
+    MB = CSR_Matrix(terms, 1, *dev(np.arange(terms + 1, dtype=np.int64), np.zeros(terms, np.int64), B.reshape(-1)))
+    C = LeSpGEMM_clustered(MA, MB, np.arange(2), np.array([0, 2]))
+    got = C.host()
+    val = got["values"] if isinstance(got, dict) else got[2]
+    assert val[0] == low
