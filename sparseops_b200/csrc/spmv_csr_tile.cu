@@ -267,40 +267,29 @@ __global__ void __launch_bounds__(kTileBlock, kMinBlocks) csr_tile_one_kernel(
   }
 }
 
-// tail, chain and owner of every tile
+// tail, chain and owner of every tile, from the bounds of the rows that hold its
+// first and last entry (walking over a row's tiles took a time quadratic in
+// them: 77 ms for one row of 2^26 entries)
 template <typename I>
-__global__ void tile_tail_kernel(const I* __restrict__ rp, int64_t n, int64_t nnz, const uint8_t* __restrict__ flags,
-                                 int64_t tiles, int tile_size, TileTail* __restrict__ tails,
-                                 unsigned long long* __restrict__ nchain) {
+__global__ void tile_tail_kernel(const I* __restrict__ rp, int64_t n, int64_t nnz, int64_t tiles, int tile_size,
+                                 TileTail* __restrict__ tails, unsigned long long* __restrict__ nchain) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= tiles) return;
-  auto any = [&](int64_t u) {
-    const uint4* f = reinterpret_cast<const uint4*>(flags + u * 32);
-    const uint4 a = f[0], b = f[1];
-    return (a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) != 0;
-  };
-  // entries that the row open at tile u's end has after it
-  auto left = [&](int64_t u) -> int64_t {
-    const int64_t e1 = (u + 1) * tile_size;
-    return e1 >= nnz ? 0 : (int64_t)rp[row_holding(rp, n, e1 - 1) + 1] - e1;
-  };
+  const int64_t e0 = t * tile_size, e1 = e0 + tile_size < nnz ? e0 + tile_size : nnz;
   TileTail T{0, 0, -1};
-  if (any(t)) {
-    const int64_t l = left(t);
-    if (l <= kTailMax) {
-      T.tail = (int32_t)l;
+  const int64_t last = row_holding(rp, n, e1 - 1), end = rp[last + 1];
+  if ((int64_t)rp[last] >= e0) {  // a row starts here, and the one open at the end is the last that does
+    if (end - e1 <= kTailMax) {
+      T.tail = (int32_t)(end - e1);
     } else {
-      for (int64_t u = t + 1; u < tiles && !(flags[u * 32] & 1u); ++u) {
-        ++T.chain;
-        if (any(u)) break;
-      }
+      T.chain = (int32_t)((end - 1) / tile_size - t);
       atomicAdd(nchain, 1ULL);
     }
   }
-  if (!(flags[t * 32] & 1u)) {
-    int64_t o = t - 1;
-    while (o >= 0 && !any(o)) --o;
-    if (o >= 0 && left(o) > kTailMax) T.owner = o;
+  const int64_t r = row_holding(rp, n, e0), s = rp[r];
+  if (s < e0) {  // the tile's first entries belong to a row that starts in an earlier tile
+    const int64_t o = s / tile_size;
+    if ((int64_t)rp[r + 1] - (o + 1) * tile_size > kTailMax) T.owner = o;
   }
   tails[t] = T;
 }
@@ -705,6 +694,9 @@ __global__ void part_bounds_kernel(const I* __restrict__ rp, int64_t n, const ui
   rb[p] = t < tiles ? row_holding(rp, n, t * (32 * K)) : n;
 }
 
+// warps of csr_tile_one_kernel that the device holds at once
+inline int64_t resident_warps(const Context* ctx) { return (int64_t)ctx->num_sms * 3 * (kTileBlock / 32); }
+
 template <int K>
 int64_t tiles_of(int64_t nnz) {
   return (nnz + 32 * K - 1) / (32 * K);
@@ -725,17 +717,21 @@ spops_status_t analyse_t(Context* ctx, Matrix* A) {
   SPOPS_TRY(D.open_sum.alloc_cached(ctx, nt1 * 8, kBuildCacheMax));
   SPOPS_TRY(D.open_row.alloc_cached(ctx, nt1 * 8, kBuildCacheMax));
   SPOPS_TRY(D.empty.alloc_cached(ctx, (size_t)(n > 0 ? n : 1) * 8, kBuildCacheMax));
-  SPOPS_TRY(D.tails.alloc_cached(ctx, nt1 * sizeof(TileTail), kBuildCacheMax));
-  SPOPS_TRY(D.counter.alloc_cached(ctx, nt1 * 4, kBuildCacheMax));
-  SPOPS_CUDA(cudaMemsetAsync(D.counter.p, 0, nt1 * 4, st));
+  const bool one = K == 8 && D.tiles <= 4 * resident_warps(ctx);  // the one-launch form may be taken
+  if (one) {
+    SPOPS_TRY(D.tails.alloc_cached(ctx, nt1 * sizeof(TileTail), kBuildCacheMax));
+    SPOPS_TRY(D.counter.alloc_cached(ctx, nt1 * 4, kBuildCacheMax));
+    SPOPS_CUDA(cudaMemsetAsync(D.counter.p, 0, nt1 * 4, st));
+  }
   SPOPS_TRY(ctx->scratch_reserve(256));
   unsigned long long* cnt = ctx->scratch.as<unsigned long long>();  // empty rows, chains
   SPOPS_CUDA(cudaMemsetAsync(cnt, 0, 16, st));
   if (D.tiles > 0 && n > 0) {
     tile_build_kernel<I, K><<<grid_of(D.tiles), 256, 0, st>>>(A->row.as<I>(), n, nnz, D.tiles,
                                                                 D.tile_row.as<int64_t>(), D.flags.as<uint8_t>());
-    tile_tail_kernel<I><<<grid_of(D.tiles), 256, 0, st>>>(A->row.as<I>(), n, nnz, D.flags.as<uint8_t>(), D.tiles,
-                                                          32 * K, D.tails.as<TileTail>(), cnt + 1);
+    if (one)
+      tile_tail_kernel<I><<<grid_of(D.tiles), 256, 0, st>>>(A->row.as<I>(), n, nnz, D.tiles, 32 * K,
+                                                            D.tails.as<TileTail>(), cnt + 1);
     SPOPS_LAUNCH_CHECK();
   }
   if (n > 0) {
@@ -819,8 +815,7 @@ spops_status_t spmv_stage_t(Context* ctx, Matrix* A, double alpha, const void* x
 // instead of overlapped ones: 11.3, 15.5, 12.4, 13.3, 58.5 in two.)
 inline bool one_launch(const Context* ctx, const Matrix* A) {
   const CsrTiles& D = A->plan.tiles;
-  const int64_t resident = (int64_t)ctx->num_sms * 3 * (kTileBlock / 32);
-  return D.tiles <= (D.nchain > 0 ? resident : 4 * resident);
+  return D.tails.p && D.tiles <= (D.nchain > 0 ? 1 : 4) * resident_warps(ctx);
 }
 
 // All tiles in one launch (csr_tile_one_kernel).

@@ -302,9 +302,9 @@ struct CsrTiles {
   DevBuf open_sum;         // V [tiles]: partial sum of the row open at the tile's end
   DevBuf open_row;         // int64 [tiles]: that row, or -1 (no row starts in the tile)
   DevBuf empty;            // int64 [rows]: empty rows
-  DevBuf tails;            // TileTail [tiles]
+  DevBuf tails;            // TileTail [tiles]; only where the one-launch form may be taken
   int64_t nchain = 0;      // tiles whose open row needs a chain
-  DevBuf counter;          // int32 [tiles]: parts of the open row that are in (zero between launches)
+  DevBuf counter;          // int32 [tiles], with tails: parts of the open row that are in (zero between launches)
   std::vector<int64_t> part_tb, part_rb;  // tile / row bounds of the pipelined host SpMV's ranges
   void release();
 };

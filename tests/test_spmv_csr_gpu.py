@@ -455,3 +455,37 @@ def test_one_launch_error(cuda, kind, vtype):
 
     small, large = {"powerlaw": (20000, 100000), "laplacian": (40000, 1000000), "banded": (30000, 300000)}[kind]
     assert mean_error(small) <= 1.05 * mean_error(large)
+
+
+def test_analysis_of_one_long_row_is_linear(cuda):
+    """The first product on a fresh handle: one row over 131,072 tiles is
+    analysed in at most four times what rows of 64 entries take (the walk over
+    a row's tiles took 20 times)."""
+    import time
+    import torch
+    from sparseops_b200 import CSR_Matrix, SpOps_csr
+    nnz = 1 << 25
+    v = torch.ones(nnz, dtype=torch.float64, device="cuda")
+    x = torch.ones(nnz, dtype=torch.float64, device="cuda")
+    ci = torch.arange(nnz, dtype=torch.int32, device="cuda")
+
+    def analysis(rows):
+        rp = torch.arange(0, nnz + 1, nnz // rows, dtype=torch.int32, device="cuda")
+        y = torch.zeros(rows, dtype=torch.float64, device="cuda")
+        best = []
+        for _ in range(3):
+            A = CSR_Matrix(rows, nnz, rp, ci, v)
+            A.device()
+            t = []
+            for _ in range(2):
+                torch.cuda.synchronize()
+                t0 = time.perf_counter()
+                SpOps_csr(1.0, A, x, 0.0, y)
+                torch.cuda.synchronize()
+                t.append(time.perf_counter() - t0)
+            assert bool((y == nnz // rows).all())
+            best.append(t[0] - t[1])
+        return min(best)
+
+    short = analysis(nnz // 64)
+    assert analysis(1) <= 4 * max(short, 1e-3)
