@@ -244,6 +244,7 @@ __global__ void __launch_bounds__(kTileBlock, kMinBlocks) csr_tile_one_kernel(
     }
     if (t + nw < tiles) load_pattern(t + nw);
     const TileEnds<V> E = tile_sums<I, V, K>(rp, n, nnz, t, lane, f, r0, p, y, alpha, beta, bz);
+    if (t + nw < tiles) load_values(t + nw);  // any earlier, they and this tile's would spill
     if (T0.tail > 0) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) ts += __shfl_xor_sync(0xffffffffu, ts, o);
@@ -263,7 +264,6 @@ __global__ void __launch_bounds__(kTileBlock, kMinBlocks) csr_tile_one_kernel(
       chain_arrive<V>(lane, 0, T0.owner, tails[T0.owner].chain, counter, carry_in, open_sum, open_row, y, alpha, beta,
                       bz);
     }
-    if (t + nw < tiles) load_values(t + nw);  // beside the gathers; earlier, they and this tile's would spill
   }
 }
 
