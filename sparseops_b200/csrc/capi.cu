@@ -257,8 +257,8 @@ spops_status_t spops_bsr_create(spops_context_t ctx, spops_matrix_t* out, int64_
   return SPOPS_OK;
 }
 
-spops_status_t spops_matrix_array(spops_matrix_t A, spops_array_t which, const void** dev_ptr, int64_t* count,
-                                  int32_t* elem_bytes) {
+static spops_status_t find_array(const Matrix* A, spops_array_t which, const void** dev_ptr, int64_t* count,
+                                 int32_t* elem_bytes) {
   if (!A) return fail(SPOPS_ERR_INVALID, "spops_matrix_array: null matrix");
   const void* p = nullptr;
   int64_t n = 0;
@@ -304,13 +304,20 @@ spops_status_t spops_matrix_array(spops_matrix_t A, spops_array_t which, const v
   return SPOPS_OK;
 }
 
+spops_status_t spops_matrix_array(spops_matrix_t A, spops_array_t which, const void** dev_ptr, int64_t* count,
+                                  int32_t* elem_bytes) {
+  SPOPS_TRY(find_array(A, which, dev_ptr, count, elem_bytes));
+  if (dev_ptr) A->shown = true;
+  return SPOPS_OK;
+}
+
 spops_status_t spops_matrix_download(spops_context_t ctx, spops_matrix_t A, spops_array_t which, void* host_dst,
                                      int64_t count) {
   if (!ctx || !A) return fail(SPOPS_ERR_INVALID, "spops_matrix_download: null argument");
   const void* p = nullptr;
   int64_t n = 0;
   int32_t eb = 0;
-  SPOPS_TRY(spops_matrix_array(A, which, &p, &n, &eb));
+  SPOPS_TRY(find_array(A, which, &p, &n, &eb));
   if (count < 0 || count > n) return fail(SPOPS_ERR_INVALID, "spops_matrix_download: count %lld > %lld",
                                           (long long)count, (long long)n);
   if (count == 0) return SPOPS_OK;
@@ -322,9 +329,13 @@ spops_status_t spops_matrix_download(spops_context_t ctx, spops_matrix_t A, spop
 spops_status_t spops_matrix_destroy(spops_matrix_t A) {
   if (!A) return SPOPS_OK;
   DeviceGuard g(A->ctx->device);
-  // every stream that may still read the arrays: blocks that go to the
-  // context's cache are handed out again without cudaFree's own wait
-  cudaDeviceSynchronize();
+  // What may still read the arrays: the context's stream (borrowed ones may be
+  // freed by their owner next), the streams it was on before
+  // (Context::cache_block waits for those), and, where the caller has asked for
+  // an array's address, any stream.
+  BesideCaptures b;
+  if (!A->ctx->capturing()) cudaStreamSynchronize(A->ctx->stream);
+  if (A->shown) A->ctx->wait_device();
   A->release_all();
   delete A;
   return SPOPS_OK;

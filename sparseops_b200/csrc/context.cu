@@ -117,6 +117,11 @@ void Context::cache_block(void* q, size_t b, size_t keep_max) {
     cudaFree(q);
     return;
   }
+  if (capturing()) {  // an event recorded now would belong to the capture
+    cudaFree(q);
+    return;
+  }
+  if (moved) wait_device();
   while (build && (build_bytes + b > keep_max || build_blocks >= kBuildBlocks)) {
     size_t i = 0;  // the oldest of them
     while (!block_cache[i].build) ++i;
@@ -136,6 +141,24 @@ void Context::cache_block(void* q, size_t b, size_t keep_max) {
   if (build) {
     build_bytes += b;
     ++build_blocks;
+  }
+}
+
+bool Context::capturing() const {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
+void Context::wait_device() {
+  moved = false;
+  void* q = nullptr;
+  if (cudaMalloc(&q, 16) == cudaSuccess) {
+    cudaFree(q);
+  } else {
+    cudaGetLastError();
+    cudaDeviceSynchronize();
   }
 }
 
@@ -336,6 +359,7 @@ spops_status_t spops_destroy(spops_context_t c) {
 
 spops_status_t spops_set_stream(spops_context_t c, void* stream) {
   if (!c) return fail(SPOPS_ERR_INVALID, "spops_set_stream: null context");
+  if (c->stream != static_cast<cudaStream_t>(stream)) c->moved = true;
   c->stream = static_cast<cudaStream_t>(stream);
   return SPOPS_OK;
 }

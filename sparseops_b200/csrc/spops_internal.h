@@ -130,7 +130,9 @@ struct Context {
   // SpGEMM's C, for instance), kept for the next result of about the same
   // size: cudaMalloc / cudaFree of a GB-sized array cost milliseconds, and
   // their time varies.  Each block carries an event recorded on the context
-  // stream when it was released; a reuse waits for it.
+  // stream when it was released; a reuse waits for it.  The event covers the
+  // work of that stream alone, so the first release after the context has moved
+  // to another stream waits for the device, as cudaFree does.
   struct CachedBlock {
     void* p;
     size_t bytes;
@@ -145,6 +147,13 @@ struct Context {
   void cache_block(void* p, size_t bytes, size_t keep_max);
   bool take_block(size_t n, void** p, size_t* bytes);
   void drop_block_cache();
+  bool moved = false;  // to another stream, since the last wait for the device
+  // whether the context's stream is being captured: nothing queued on it now
+  // runs, and nothing that waits for it may be called
+  bool capturing() const;
+  // Waits for all work queued on the device, as cudaFree of a device array does
+  // (cudaDeviceSynchronize would end any capture under way on the device).
+  void wait_device();
   size_t arena_top = 0;       // bytes handed out
   size_t arena_over = 0;      // bytes of live pool allocations made in a scope
   size_t arena_need = 0;      // largest arena_top + arena_over seen
@@ -256,6 +265,17 @@ struct ArenaScope {
   ~ArenaScope();
   ArenaScope(const ArenaScope&) = delete;
   ArenaScope& operator=(const ArenaScope&) = delete;
+};
+
+// While it lives, calls of this thread that another stream's capture would
+// refuse (and be invalidated by) are allowed: waits for streams that are not
+// being captured, cudaMalloc and cudaFree.
+struct BesideCaptures {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  BesideCaptures(const BesideCaptures&) = delete;
+  BesideCaptures& operator=(const BesideCaptures&) = delete;
 };
 
 // RAII guard: make ctx->device current for the duration of an API call.
@@ -490,6 +510,7 @@ struct Matrix {
   spops_value_t vtype = SPOPS_VALUE_F64;
   spops_layout_t layout = SPOPS_ROW_MAJOR;
   int64_t rows = 0, cols = 0, nnz = 0;
+  bool shown = false;  // the caller has asked for an array's address (spops_matrix_array)
   // CSR / COO arrays (COO: row = row index array)
   DevBuf row, col, val;
   CsrPlan plan;
