@@ -336,6 +336,7 @@ spops_status_t spops_matrix_destroy(spops_matrix_t A) {
   BesideCaptures b;
   if (!A->ctx->capturing()) cudaStreamSynchronize(A->ctx->stream);
   if (A->shown) A->ctx->wait_device();
+  A->ctx->graph_blocks->free_dead();
   A->release_all();
   delete A;
   return SPOPS_OK;

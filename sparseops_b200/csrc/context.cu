@@ -237,6 +237,53 @@ void Context::pool_free(void* q) {
   if (q) cudaFreeAsync(q, stream);
 }
 
+void GraphBlocks::free_dead() {
+  std::lock_guard<std::mutex> lock(mutex);
+  for (void* q : dead) cudaFree(q);
+  dead.clear();
+}
+
+namespace {
+struct GraphBlock {
+  std::shared_ptr<GraphBlocks> list;
+  void* p;
+};
+void CUDART_CB graph_block_gone(void* q) {
+  GraphBlock* b = static_cast<GraphBlock*>(q);
+  {
+    std::lock_guard<std::mutex> lock(b->list->mutex);
+    b->list->dead.push_back(b->p);
+  }
+  delete b;
+}
+}  // namespace
+
+spops_status_t Context::graph_alloc(void** out, size_t bytes) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  SPOPS_CUDA(cudaStreamGetCaptureInfo_v2(stream, &status, nullptr, &graph, nullptr, nullptr));
+  if (status != cudaStreamCaptureStatusActive) return fail(SPOPS_ERR_CUDA, "no capture under way on the stream");
+  BesideCaptures beside;
+  graph_blocks->free_dead();
+  void* q = nullptr;
+  SPOPS_CUDA(cudaMalloc(&q, bytes));
+  GraphBlock* b = new GraphBlock{graph_blocks, q};
+  cudaUserObject_t object = nullptr;
+  cudaError_t e = cudaUserObjectCreate(&object, b, graph_block_gone, 1, cudaUserObjectNoDestructorSync);
+  if (e != cudaSuccess) {
+    delete b;
+    cudaFree(q);
+    return cuda_fail(e, "cudaUserObjectCreate", __FILE__, __LINE__);
+  }
+  e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+  if (e != cudaSuccess) {
+    cudaUserObjectRelease(object, 1);  // the callback takes the block
+    return cuda_fail(e, "cudaGraphRetainUserObject", __FILE__, __LINE__);
+  }
+  *out = q;
+  return SPOPS_OK;
+}
+
 ArenaScope::ArenaScope(Context* c) : ctx(c) {
   if (ctx->arena_depth++ > 0) {
     mark = ctx->arena_top;
@@ -349,6 +396,7 @@ spops_status_t spops_destroy(spops_context_t c) {
   }
   c->arena.release();
   c->drop_block_cache();
+  c->graph_blocks->free_dead();
   if (c->pool) {
     cudaStreamSynchronize(c->stream);
     cudaMemPoolDestroy(c->pool);

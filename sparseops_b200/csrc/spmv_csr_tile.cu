@@ -596,13 +596,11 @@ __global__ void csr_tile_calibrate_k_kernel(int L, int k, int64_t tiles, const V
 
 template <typename I, typename V, int G, int J, bool kVec, bool kStage, bool kFull>
 spops_status_t spmm_tiles_f(Context* ctx, Matrix* A, double alpha, const void* X, int64_t ldx, int64_t k,
-                            double beta, void* Y, int64_t ldy) {
+                            double beta, void* Y, int64_t ldy, void* scratch) {
   const CsrTiles& D = A->plan.tiles;
   const bool bz = beta == 0.0;
-  PoolBuf cin(ctx), osum(ctx);
-  const size_t nt1 = (size_t)(D.tiles > 0 ? D.tiles : 1);
-  SPOPS_TRY(cin.alloc(nt1 * (size_t)k * sizeof(V)));
-  SPOPS_TRY(osum.alloc(nt1 * (size_t)k * sizeof(V)));
+  V* cin = static_cast<V*>(scratch);  // k values per tile each
+  V* osum = cin + D.tiles * k;
   if (D.tiles > 0) {
     auto* kern = csr_tile_spmm_kernel<I, V, G, J, kVec, kStage, kFull>;
     constexpr size_t smem = !kStage ? 0 : 2 * (kTileBlock / 32) * sizeof(SpmmTile<I, V, G>);
@@ -615,13 +613,13 @@ spops_status_t spmm_tiles_f(Context* ctx, Matrix* A, double alpha, const void* X
     SPOPS_CUDA(launch_overlapped(kern, grid, kTileBlock, smem, ctx->stream,
         A->row.as<I>(), A->rows, A->nnz, A->col.as<I>(), A->val.as<V>(), D.tile_row.as<int64_t>(),
         D.flags.as<uint8_t>(), D.tiles, static_cast<const V*>(X), ldx, (int)k, static_cast<V*>(Y), ldy, (V)alpha,
-        (V)beta, bz, cin.as<V>(), osum.as<V>(), D.open_row.as<int64_t>()));
+        (V)beta, bz, cin, osum, D.open_row.as<int64_t>()));
     SPOPS_LAUNCH_CHECK();
   }
   if (D.tiles + D.nempty > 0) {
     const int L = spmm_cal_lanes(k);
     SPOPS_CUDA(launch_overlapped(csr_tile_calibrate_k_kernel<V>, grid_of((D.tiles + D.nempty) * L), 256, 0, ctx->stream,
-        L, (int)k, D.tiles, cin.as<V>(), osum.as<V>(), D.open_row.as<int64_t>(), D.empty.as<int64_t>(), D.nempty,
+        L, (int)k, D.tiles, cin, osum, D.open_row.as<int64_t>(), D.empty.as<int64_t>(), D.nempty,
         static_cast<V*>(Y), ldy, (V)alpha, (V)beta, bz));
     SPOPS_LAUNCH_CHECK();
   }
@@ -630,9 +628,9 @@ spops_status_t spmm_tiles_f(Context* ctx, Matrix* A, double alpha, const void* X
 
 template <typename I, typename V, int G, int J, bool kVec, bool kStage>
 spops_status_t spmm_tiles_t(Context* ctx, Matrix* A, double alpha, const void* X, int64_t ldx, int64_t k,
-                            double beta, void* Y, int64_t ldy) {
-  if (k == G * J) return spmm_tiles_f<I, V, G, J, kVec, kStage, true>(ctx, A, alpha, X, ldx, k, beta, Y, ldy);
-  return spmm_tiles_f<I, V, G, J, kVec, kStage, false>(ctx, A, alpha, X, ldx, k, beta, Y, ldy);
+                            double beta, void* Y, int64_t ldy, void* scratch) {
+  if (k == G * J) return spmm_tiles_f<I, V, G, J, kVec, kStage, true>(ctx, A, alpha, X, ldx, k, beta, Y, ldy, scratch);
+  return spmm_tiles_f<I, V, G, J, kVec, kStage, false>(ctx, A, alpha, X, ldx, k, beta, Y, ldy, scratch);
 }
 
 // Lanes per entry, columns per lane, vector parts and staging by k, each the
@@ -653,8 +651,8 @@ spops_status_t spmm_tiles_t(Context* ctx, Matrix* A, double alpha, const void* X
 // per four: the group's eight loads are whole 64-byte pieces.
 template <typename I, typename V>
 spops_status_t spmm_tiles_k(Context* ctx, Matrix* A, double alpha, const void* X, int64_t ldx, int64_t k,
-                            double beta, void* Y, int64_t ldy) {
-#define SPOPS_SPMM(G, J, VEC, STAGE) return spmm_tiles_t<I, V, G, J, VEC, STAGE>(ctx, A, alpha, X, ldx, k, beta, Y, ldy)
+                            double beta, void* Y, int64_t ldy, void* scratch) {
+#define SPOPS_SPMM(G, J, VEC, STAGE) return spmm_tiles_t<I, V, G, J, VEC, STAGE>(ctx, A, alpha, X, ldx, k, beta, Y, ldy, scratch)
   constexpr bool f64 = sizeof(V) == 8;
   const bool vec = csr_spmm_vector(X, ldx, k, sizeof(V));
   if (vec && k == 4) SPOPS_SPMM(1, 4, true, false);
@@ -972,18 +970,29 @@ spops_status_t csr_tile_spmm(Context* ctx, Matrix* A, double alpha, const void* 
                              double beta, void* Y, int64_t ldy, bool* used) {
   *used = false;
   if (!csr_tile_spmm_usable(A, X, ldx, k) || ldy < k) return SPOPS_OK;
+  const bool captured = ctx->capturing();
   if (!A->plan.tiles.ready || A->plan.tiles.k != 8) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    SPOPS_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
-    if (cap != cudaStreamCaptureStatusNone) return SPOPS_OK;  // the plan cannot be built inside a capture
-    SPOPS_TRY(csr_tile_analyse(ctx, A, 8));
+    if (captured) return SPOPS_OK;  // the plan cannot be built inside a capture
+    const spops_status_t s = csr_tile_analyse(ctx, A, 8);
+    if (s == SPOPS_ERR_ALLOC) {  // the segment kernel needs neither plan nor scratch
+      A->plan.tiles.release();
+      return SPOPS_OK;
+    }
+    SPOPS_TRY(s);
   }
+  PoolBuf buf(ctx);
+  void* scratch = nullptr;
+  const size_t bytes = 2 * (size_t)std::max<int64_t>(A->plan.tiles.tiles, 1) * (size_t)k * A->vsize();
+  const spops_status_t got = captured ? ctx->graph_alloc(&scratch, bytes) : buf.alloc(bytes);
+  if (got == SPOPS_ERR_ALLOC) return SPOPS_OK;
+  SPOPS_TRY(got);
+  if (!captured) scratch = buf.p;
   *used = true;
   const bool i32 = A->itype == SPOPS_INDEX_I32, f64 = A->vtype == SPOPS_VALUE_F64;
-  if (i32 && f64) return spmm_tiles_k<int32_t, double>(ctx, A, alpha, X, ldx, k, beta, Y, ldy);
-  if (i32) return spmm_tiles_k<int32_t, float>(ctx, A, alpha, X, ldx, k, beta, Y, ldy);
-  if (f64) return spmm_tiles_k<int64_t, double>(ctx, A, alpha, X, ldx, k, beta, Y, ldy);
-  return spmm_tiles_k<int64_t, float>(ctx, A, alpha, X, ldx, k, beta, Y, ldy);
+  if (i32 && f64) return spmm_tiles_k<int32_t, double>(ctx, A, alpha, X, ldx, k, beta, Y, ldy, scratch);
+  if (i32) return spmm_tiles_k<int32_t, float>(ctx, A, alpha, X, ldx, k, beta, Y, ldy, scratch);
+  if (f64) return spmm_tiles_k<int64_t, double>(ctx, A, alpha, X, ldx, k, beta, Y, ldy, scratch);
+  return spmm_tiles_k<int64_t, float>(ctx, A, alpha, X, ldx, k, beta, Y, ldy, scratch);
 }
 
 spops_status_t csr_tile_spmv_indirect(Context* ctx, Matrix* A, const int64_t* perm, const void* vsrc, double alpha,

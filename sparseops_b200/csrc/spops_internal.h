@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <string>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -65,6 +66,14 @@ struct DevBuf {
   template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
+// Device memory whose graphs are gone, left for a library call to free (the
+// callback that learns of it may not call the runtime).
+struct GraphBlocks {
+  std::mutex mutex;
+  std::vector<void*> dead;
+  void free_dead();
+};
+
 // ---------------------------------------------------------------- context
 struct Context {
   int device = 0;
@@ -118,6 +127,12 @@ struct Context {
   cudaMemPool_t pool = nullptr;
   spops_status_t pool_alloc(void** p, size_t bytes);
   void pool_free(void* p);
+  // Scratch of a call that is being captured: it belongs to the graph under
+  // capture on the context's stream (and to its copies and instances) and goes
+  // when they do, so the graph holds no allocation nodes and its replays share
+  // nothing with other calls.
+  std::shared_ptr<GraphBlocks> graph_blocks = std::make_shared<GraphBlocks>();
+  spops_status_t graph_alloc(void** p, size_t bytes);
   // arena for the temporaries of one call inside an ArenaScope: one buffer
   // kept by the context and handed out by a bump pointer, so a call whose
   // temporaries are the same sizes as the last one's maps no memory.  (The
@@ -552,9 +567,10 @@ spops_status_t csr_spmv(Context* ctx, Matrix* A, double alpha, const void* x, do
 // tile kernel (spmv_csr_tile.cu); usable when the column and value arrays are
 // aligned for the lane's vector loads
 bool csr_tile_usable(const Matrix* A, int variant);
-// Y = alpha*A*X + beta*Y with k = 8, 16 or 32 right-hand sides on the SpMV's
-// tile plan (k / 4 lanes per entry); *used = false (nothing done) unless the
-// matrix and X allow its vector loads and X's row stride is at most 2k.
+// Y = alpha*A*X + beta*Y with up to 32 right-hand sides on the SpMV's tile plan;
+// *used = false (nothing done) unless the matrix allows its vector loads, X's row
+// stride is at most 2k, and the plan and the scratch (2k values per tile) can be
+// had.
 bool csr_tile_spmm_usable(const Matrix* A, const void* X, int64_t ldx, int64_t k);
 // X's rows can be read four columns at a time (vs: bytes of a value)
 bool csr_spmm_vector(const void* X, int64_t ldx, int64_t k, size_t vs);
