@@ -1,4 +1,5 @@
 // Context, error reporting and device buffers behind the C ABI.
+#include <algorithm>
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
@@ -284,9 +285,10 @@ spops_status_t Context::graph_alloc(void** out, size_t bytes) {
   return SPOPS_OK;
 }
 
-ArenaScope::ArenaScope(Context* c) : ctx(c) {
+ArenaScope::ArenaScope(Context* c, size_t keep_bytes) : ctx(c), keep(keep_bytes) {
   if (ctx->arena_depth++ > 0) {
     mark = ctx->arena_top;
+    bound();
     return;
   }
   // the last scope's work on another stream may still read the arena
@@ -304,10 +306,28 @@ ArenaScope::ArenaScope(Context* c) : ctx(c) {
   ctx->arena_top = 0;
   ctx->arena_over = 0;
   mark = 0;
+  bound();
+}
+
+void ArenaScope::bound() {
+  if (keep == ~size_t(0)) return;
+  base = ctx->arena_top + ctx->arena_over;
+  outer_limit = ctx->arena_limit;
+  outer_peak = ctx->arena_peak;
+  ctx->arena_limit = std::min(outer_limit, base + keep);
+  ctx->arena_peak = base;
 }
 
 ArenaScope::~ArenaScope() {
   ctx->arena_top = mark;
+  if (keep != ~size_t(0)) {
+    if (ctx->arena_peak - base > keep && ctx->pool) {
+      cudaStreamSynchronize(ctx->stream);  // the frees are queued
+      cudaMemPoolTrimTo(ctx->pool, keep);
+    }
+    ctx->arena_limit = outer_limit;
+    ctx->arena_peak = std::max(outer_peak, ctx->arena_peak);
+  }
   if (--ctx->arena_depth > 0) return;
   if (!ctx->arena_done) cudaEventCreateWithFlags(&ctx->arena_done, cudaEventDisableTiming);
   if (ctx->arena_done) cudaEventRecord(ctx->arena_done, ctx->stream);

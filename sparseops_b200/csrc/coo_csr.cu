@@ -209,7 +209,7 @@ Matrix* new_csr(Context* ctx, const Matrix* like, int64_t nnz) {
 template <typename I, typename V>
 spops_status_t coo_to_csr_t(Context* ctx, Matrix* coo, bool compact, Matrix** out) {
   cudaStream_t st = ctx->stream;
-  ArenaScope scope(ctx);  // this call's temporaries come from the arena
+  ArenaScope scope(ctx, kBuildArenaMax);  // this call's temporaries come from the arena
   if (!coo->csr_view) SPOPS_TRY(coo_analyse(ctx, coo));
   const Matrix* S = coo->csr_view;  // rows sorted, file order within rows
   const int64_t n = S->rows, nz = S->nnz;

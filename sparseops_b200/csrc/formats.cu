@@ -911,7 +911,7 @@ spops_status_t padded_finish_t(Context* ctx, Matrix* M) {
   if (P.C == 32 && M->layout == SPOPS_COL_MAJOR && n > 0) {
     // heads, tails and windows of the 32-row chunks
     const int64_t nch = (n + 31) / 32;
-    ArenaScope scope(ctx);
+    ArenaScope scope(ctx, kBuildArenaMax);
     PoolBuf cnt(ctx), offs(ctx), tmp(ctx);
     SPOPS_TRY(cnt.alloc((size_t)(nch + 1) * 3 * 8));
     SPOPS_TRY(offs.alloc((size_t)(nch + 1) * 3 * 8));
@@ -1184,7 +1184,7 @@ spops_status_t coo_analyse_t(Context* ctx, Matrix* A) {
   cudaStream_t st = ctx->stream;
   const int64_t n = A->rows, nz = A->nnz;
   const size_t nzz = (size_t)(nz > 0 ? nz : 1), n1 = (size_t)n + 1;
-  ArenaScope scope(ctx);  // this call's temporaries come from the arena
+  ArenaScope scope(ctx, kBuildArenaMax);  // this call's temporaries come from the arena
   SPOPS_TRY(ctx->scratch_reserve(256));
   int* flags = ctx->scratch.as<int>();
   SPOPS_CUDA(cudaMemsetAsync(flags, 0, 4, st));

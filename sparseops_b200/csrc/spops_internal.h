@@ -47,6 +47,10 @@ constexpr size_t kBlockCacheMax = size_t(24) << 30;  // bytes a context's block 
 // blocks of a few tens to hundreds of MB, whose cudaMalloc and cudaFree cost
 // more than filling them
 constexpr size_t kBuildCacheMax = size_t(2) << 30;
+// bytes of their temporaries that a context keeps (in its arena, and as much in
+// its pool): a one-off assembly of a large matrix, about 100 bytes per entry
+// where it takes the global sorts, gives the rest back
+constexpr size_t kBuildArenaMax = size_t(1) << 30;
 
 struct DevBuf {
   void* p = nullptr;
@@ -171,7 +175,9 @@ struct Context {
   void wait_device();
   size_t arena_top = 0;       // bytes handed out
   size_t arena_over = 0;      // bytes of live pool allocations made in a scope
-  size_t arena_need = 0;      // largest arena_top + arena_over seen
+  size_t arena_need = 0;      // largest arena_top + arena_over seen, up to arena_limit
+  size_t arena_limit = ~size_t(0);  // set by an ArenaScope with a bound
+  size_t arena_peak = 0;      // largest arena_top + arena_over since such a scope opened
   int arena_depth = 0;        // open ArenaScopes
   cudaEvent_t arena_done = nullptr;    // recorded when the outermost scope ends
   cudaStream_t arena_stream = nullptr;  // the stream that event was recorded on
@@ -264,7 +270,9 @@ struct PoolBuf {
  private:
   void note_need() {
     const size_t t = ctx->arena_top + ctx->arena_over;
-    if (t > ctx->arena_need) ctx->arena_need = t;
+    if (t > ctx->arena_peak) ctx->arena_peak = t;
+    const size_t need = t < ctx->arena_limit ? t : ctx->arena_limit;
+    if (need > ctx->arena_need) ctx->arena_need = need;
   }
 };
 
@@ -272,14 +280,19 @@ struct PoolBuf {
 // the context's arena (PoolBuf).  Declare it before the call's PoolBufs.
 // Opening the outermost scope regrows the arena to what earlier scopes
 // needed (after the stream's queued work, which may still read it) and
-// orders this stream after the last scope's work on another stream.
+// orders this stream after the last scope's work on another stream.  `keep`:
+// the arena does not grow for more than that many bytes of this scope, and what
+// the scope took beyond them goes back to the device at its end.
 struct ArenaScope {
   Context* ctx;
-  size_t mark = 0;
-  explicit ArenaScope(Context* c);
+  size_t mark = 0, keep, outer_limit = 0, outer_peak = 0, base = 0;
+  explicit ArenaScope(Context* c, size_t keep_bytes = ~size_t(0));
   ~ArenaScope();
   ArenaScope(const ArenaScope&) = delete;
   ArenaScope& operator=(const ArenaScope&) = delete;
+
+ private:
+  void bound();
 };
 
 // While it lives, calls of this thread that another stream's capture would

@@ -114,3 +114,35 @@ def test_plan_rebuilt_after_a_stream_change(cuda, orc):
         ctx.set_option("csr_variant", 0)
     for y in ys:
         assert (np.abs(y.cpu().numpy() - ref) / den).max() <= 1e-12
+
+
+def test_assembly_gives_its_memory_back(cuda):
+    """A one-off assembly of 60M triplets through the global sorts (one row has
+    more than 512 entries), about 6 GB of temporaries: the context keeps at most
+    2 GB of blocks and 1 GB of temporaries in each of arena and pool (1/8 of
+    growth added), and nothing once it is closed."""
+    import torch
+    from sparseops_b200 import COO_Matrix, Context, coo_to_csr
+    n, per = 1_000_000, 60
+    rows = torch.arange(n * per, device="cuda", dtype=torch.int64)
+    cols = (rows * 48271 % n).to(torch.int32)
+    rows = (rows % n).to(torch.int32)
+    rows[:600] = 5
+    vals = torch.ones(n * per, dtype=torch.float64, device="cuda")
+    ctx = Context(0)
+
+    def held():
+        torch.cuda.synchronize()
+        return start - torch.cuda.mem_get_info()[0]
+
+    start = torch.cuda.mem_get_info()[0]
+    for _ in range(2):
+        coo = COO_Matrix(n, n, rows, cols, vals)
+        coo.device(ctx)
+        A = coo_to_csr(coo, compact=True)
+        assert A.num_nnzs > n
+        del A, coo
+        gc.collect()
+        assert held() <= 4.4 * 2 ** 30
+    ctx.close()
+    assert held() <= 64 << 20
