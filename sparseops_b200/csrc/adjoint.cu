@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(256) sddmm_tile_kernel(const I* __restrict__ r
     } else {
       row = row_holding(rp, n, el < nnz ? el : nnz - 1);
     }
-    V gi = (el < nnz && row < n) ? alpha * g[row] : V(0);
+    V gi = (el < nnz && row < n) ? alpha * ld_gather(g + row) : V(0);
     V o[K];
 #pragma unroll
     for (int b = 0; b < K; ++b) {
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(256) sddmm_tile_kernel(const I* __restrict__ r
         ++row;
         if (tr < 0)
           while (row + 1 < n && rp[row] == rp[row + 1]) ++row;  // skip empty rows
-        gi = row < n ? alpha * g[row] : V(0);
+        gi = row < n ? alpha * ld_gather(g + row) : V(0);
       }
       o[b] = gi * xv[b];
     }

@@ -6,6 +6,7 @@
 
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 
 #include "device_util.cuh"
 
@@ -23,40 +24,54 @@ __device__ __forceinline__ int64_t row_holding(const I* rp, int64_t n, int64_t e
   return lo;
 }
 
-// ---- vector loads of one lane's run (32-byte aligned for 32-byte runs)
-template <int BYTES>
+// ---- vector loads of one lane's run (32-byte aligned for 32-byte runs).
+// kFixed: of the pattern, which nothing writes while a plan is in use; else plain
+// loads, as for ld_gather (a launch before this one may have written the values)
+template <int BYTES, bool kFixed>
 struct RunLoad;
-template <>
-struct RunLoad<16> {
+template <bool kFixed>
+struct RunLoad<16, kFixed> {
   static __device__ __forceinline__ void ld(const void* p, uint32_t (&w)[4]) {
-    asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
-                 : "l"(p));
+    if constexpr (kFixed)
+      asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                   : "l"(p));
+    else
+      asm volatile("ld.global.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                   : "l"(p));
   }
 };
-template <>
-struct RunLoad<32> {
+template <bool kFixed>
+struct RunLoad<32, kFixed> {
   static __device__ __forceinline__ void ld(const void* p, uint32_t (&w)[8]) {
-    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
-                 : "l"(p));
+    if constexpr (kFixed)
+      asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                   : "l"(p));
+    else
+      asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                   : "l"(p));
   }
 };
 
-// K elements of T from p (aligned to min(32, K*sizeof(T)) bytes) into out.
+// K elements of T from p (aligned to min(32, K*sizeof(T)) bytes) into out:
+// indices are the pattern's (or a plan's), floating values are not.
 template <typename T, int K>
 __device__ __forceinline__ void load_run(const T* __restrict__ p, T (&out)[K]) {
   constexpr int BYTES = K * (int)sizeof(T);
+  constexpr bool kFixed = !std::is_floating_point<T>::value;
   static_assert(BYTES == 16 || BYTES % 32 == 0, "run must be 16 bytes or a multiple of 32");
   if constexpr (BYTES == 16) {
     uint32_t w[4];
-    RunLoad<16>::ld(p, w);
+    RunLoad<16, kFixed>::ld(p, w);
     memcpy(out, w, 16);
   } else {
 #pragma unroll
     for (int q = 0; q < BYTES / 32; ++q) {
       uint32_t w[8];
-      RunLoad<32>::ld(reinterpret_cast<const char*>(p) + 32 * q, w);
+      RunLoad<32, kFixed>::ld(reinterpret_cast<const char*>(p) + 32 * q, w);
       memcpy(reinterpret_cast<char*>(out) + 32 * q, w, 32);
     }
   }
@@ -203,13 +218,16 @@ __device__ __forceinline__ void tile_finish(const I* __restrict__ rp, int64_t n,
   }
 }
 
+// (The calibrations are set up while the tiles' sums are still being written: the
+// three arrays are not __restrict__, so that they are read by plain loads.)
+//
 // The row open at tile t's end: its sum there and the heads of the following
 // tiles, in tile order, up to the first one that starts a row.  A long row's
 // tiles are read eight at a time (one at a time its loads were the
 // calibration's whole time: 6.4 us for a row over 20 tiles).
 template <typename V>
-__device__ __forceinline__ V chain_sum(int64_t t, int64_t tiles, const V* __restrict__ carry_in,
-                                       const V* __restrict__ open_sum, const int64_t* __restrict__ open_row) {
+__device__ __forceinline__ V chain_sum(int64_t t, int64_t tiles, const V* carry_in,
+                                       const V* open_sum, const int64_t* open_row) {
   V tot = open_sum[t];
   if (t + 1 >= tiles) return tot;
   tot += carry_in[t + 1];
@@ -236,8 +254,8 @@ __device__ __forceinline__ V chain_sum(int64_t t, int64_t tiles, const V* __rest
 // of a single-vector product: the row open at tile t's end receives the heads
 // of the following tiles up to the first one that starts a row.
 template <typename V>
-__device__ __forceinline__ void spmv_calibrate1(int64_t t, int64_t tiles, const V* __restrict__ carry_in,
-                                                const V* __restrict__ open_sum, const int64_t* __restrict__ open_row,
+__device__ __forceinline__ void spmv_calibrate1(int64_t t, int64_t tiles, const V* carry_in,
+                                                const V* open_sum, const int64_t* open_row,
                                                 const int64_t* __restrict__ empty, int64_t nempty, V* __restrict__ y,
                                                 V alpha, V beta, bool bz) {
   if (t < tiles) {
@@ -337,13 +355,13 @@ __device__ __forceinline__ void ld_xpart(const V* __restrict__ p, int k, int h, 
     static_assert(J == 4, "vector parts hold four columns");
     if constexpr (sizeof(V) == 8) {
       uint32_t w[8];
-      asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                    : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
                    : "l"(p + 4 * h));
       memcpy(r, w, 32);
     } else {
       uint32_t w[4];
-      asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];"
+      asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];"
                    : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
                    : "l"(p + 4 * h));
       memcpy(r, w, 16);
@@ -538,8 +556,8 @@ __host__ __device__ __forceinline__ int spmm_cal_lanes(int64_t k) {
 // of a product with k columns; this lane takes columns sub, sub + L, ...
 template <typename V>
 __device__ __forceinline__ void spmm_calibrate(int64_t t, int sub, int L, int k, int64_t tiles,
-                                               const V* __restrict__ carry_in, const V* __restrict__ open_sum,
-                                               const int64_t* __restrict__ open_row,
+                                               const V* carry_in, const V* open_sum,
+                                               const int64_t* open_row,
                                                const int64_t* __restrict__ empty, int64_t nempty, V* __restrict__ Y,
                                                int64_t ldy, V alpha, V beta, bool bz) {
   if (t < tiles) {

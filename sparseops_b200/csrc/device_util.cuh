@@ -16,13 +16,28 @@ __device__ __forceinline__ int64_t ld_stream(const int64_t* p) {
 __device__ __forceinline__ float ld_stream(const float* p) { return __ldcs(p); }
 __device__ __forceinline__ double ld_stream(const double* p) { return __ldcs(p); }
 
-// Read-only cached load for the gathered vector.
-template <typename T>
-__device__ __forceinline__ T ld_gather(const T* p) { return __ldg(p); }
+// Cached load of what a launch before this one may have written: vectors,
+// gradients, values.  A kernel that is set up while that launch still runs
+// (pdl.cuh) reads it after its wait, and by plain loads: the non-coherent ones
+// (__ldg, or a const __restrict__ pointer) are for data that nothing writes while
+// the kernel lives.
+__device__ __forceinline__ float ld_gather(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double ld_gather(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
 
 // L2-coherent load (bypasses L1), for values written by other blocks.
 __device__ __forceinline__ float ld_cg(const float* p) { return __ldcg(p); }
 __device__ __forceinline__ double ld_cg(const double* p) { return __ldcg(p); }
+__device__ __forceinline__ int64_t ld_cg(const int64_t* p) {
+  return (int64_t)__ldcg(reinterpret_cast<const long long*>(p));
+}
 
 template <typename V>
 __device__ __forceinline__ V warp_sum(V v, int width = 32) {

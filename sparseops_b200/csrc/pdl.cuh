@@ -10,6 +10,8 @@
 // launch after such a kernel waits for its end as always.  What may be read
 // before the wait is a handle's plan and pattern alone: they were complete
 // when the plan's analysis returned and do not change while it is in use.
+// Everything else is read after it, by plain loads (ld_gather, or a pointer that
+// is not const __restrict__).
 #pragma once
 
 #include <cuda_runtime.h>

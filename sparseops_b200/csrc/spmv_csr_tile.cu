@@ -159,10 +159,11 @@ __device__ __forceinline__ void chain_arrive(int lane, int who, int64_t o, int32
     if (last) __threadfence();  // every part is there: read them past L1
   }
   if (!__shfl_sync(0xffffffffu, last, who)) return;
+  __syncwarp();  // lane `who`'s fence before the other lanes' reads (a shuffle orders no memory)
   V tot = V(0);
-  for (int32_t u = lane; u < m; u += 32) tot += __ldcg(carry_in + o + 1 + u);
-  const V open = __ldcg(open_sum + o);
-  const int64_t r = __ldcg(reinterpret_cast<const long long*>(open_row + o));
+  for (int32_t u = lane; u < m; u += 32) tot += ld_cg(carry_in + o + 1 + u);
+  const V open = ld_cg(open_sum + o);
+  const int64_t r = ld_cg(open_row + o);
 #pragma unroll
   for (int q = 16; q > 0; q >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, q);
   if (lane == 0) axpby_store(y + r, open + tot, alpha, beta, bz);
@@ -203,9 +204,9 @@ __global__ void __launch_bounds__(kTileBlock, kMinBlocks) csr_tile_one_kernel(
       load_run<V, K>(val + el, a);
     } else {
 #pragma unroll
-      for (int b = 0; b < K; ++b) a[b] = el + b < nnz ? val[el + b] : V(0);
+      for (int b = 0; b < K; ++b) a[b] = el + b < nnz ? ld_gather(val + el + b) : V(0);
     }
-    if (e1 < nnz) at = val[e1];
+    if (e1 < nnz) at = ld_gather(val + e1);
   };
   overlap_let_next();
   if (t < tiles) load_pattern(t);
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(kTileBlock, kMinBlocks) csr_tile_one_kernel(
       for (int q = 0; q < kTailMax / 32 - 1; ++q) xt[q] = 32 * q < m ? ld_gather(x + ci[e + 32 * q]) : V(0);
 #pragma unroll
       for (int q = 0; q < kTailMax / 32 - 1; ++q)
-        if (32 * q < m) ts += val[e + 32 * q] * xt[q];
+        if (32 * q < m) ts += ld_gather(val + e + 32 * q) * xt[q];
     }
     if (t + nw < tiles) load_pattern(t + nw);
     const TileEnds<V> E = tile_sums<I, V, K>(rp, n, nnz, t, lane, f, r0, p, y, alpha, beta, bz);
@@ -532,8 +533,8 @@ __global__ void __launch_bounds__(kTileBlock, 3) csr_tile_indirect_kernel(
 // first one that starts a row; empty rows get y = beta*y.  Tiles [t_begin,
 // tiles) only: a range ends where a row starts, so no chain crosses it.
 template <typename V>
-__global__ void csr_tile_calibrate_kernel(int64_t t_begin, int64_t tiles, const V* __restrict__ carry_in,
-                                          const V* __restrict__ open_sum, const int64_t* __restrict__ open_row,
+__global__ void csr_tile_calibrate_kernel(int64_t t_begin, int64_t tiles, const V* carry_in,
+                                          const V* open_sum, const int64_t* open_row,
                                           const int64_t* __restrict__ empty, int64_t nempty, V* __restrict__ y,
                                           V alpha, V beta, bool bz) {
   overlap_begin();
@@ -584,8 +585,8 @@ __global__ void __launch_bounds__(kTileBlock, 2) csr_tile_spmm_kernel(
 }
 
 template <typename V>
-__global__ void csr_tile_calibrate_k_kernel(int L, int k, int64_t tiles, const V* __restrict__ carry_in,
-                                            const V* __restrict__ open_sum, const int64_t* __restrict__ open_row,
+__global__ void csr_tile_calibrate_k_kernel(int L, int k, int64_t tiles, const V* carry_in,
+                                            const V* open_sum, const int64_t* open_row,
                                             const int64_t* __restrict__ empty, int64_t nempty, V* __restrict__ Y,
                                             int64_t ldy, V alpha, V beta, bool bz) {
   overlap_begin();
