@@ -805,13 +805,17 @@ spops_status_t spmv_stage_t(Context* ctx, Matrix* A, double alpha, const void* x
   return SPOPS_OK;
 }
 
-// One launch or two: a small matrix's call is bound by its launches, so one is
-// taken up to a tile per resident warp, or four where no row needs a chain and
-// its fences; above, reading on at every tile's end costs as much as the second
-// launch.  Calls issued back to back, two launches | one (us): power-law 20,000
-// rows 10.1 | 7.6, 60,000 rows 12.4 | 14.0; 512 x 512 Laplacian 10.2 | 7.7;
-// banded 100,000 rows 10.1 | 8.5, 1,000,000 rows 56.0 | 59.3.  (Plain launches
-// instead of overlapped ones: 11.3, 15.5, 12.4, 13.3, 58.5 in two.)
+// One launch or two: a small matrix's call is bound by issuing its launches (7.4 us
+// of host time for one, 9.6 us for two), so one is taken while it is no longer on
+// the device either: up to a tile per resident warp, or four where no row needs a
+// chain and its fences.  Above, reading on at every tile's end costs more than the
+// second launch.  Device time, two launches | one (us; FP64, int32, beta = 0), at
+// 0.5, 1, 1.5 and 2 times the limit:
+//   power-law, chains (1,770 .. 7,069 tiles)   7.4 | 6.9   8.9 | 8.8   12.4 | 13.3  13.3 | 14.7
+//   banded (6,995 .. 27,966 tiles)            10.6 | 8.7  16.3 | 15.3  22.2 | 22.4  28.4 | 30.3
+//   Laplacian (7,092 .. 28,388 tiles)          9.2 | 7.6  13.7 | 13.3  18.9 | 20.4  29.7 | 33.7
+// and the same sides with FP32 and int64.  20,000 power-law rows with beta = 0.7:
+// 10.5 | 10.1.
 inline bool one_launch(const Context* ctx, const Matrix* A) {
   const CsrTiles& D = A->plan.tiles;
   return D.tails.p && D.tiles <= (D.nchain > 0 ? 1 : 4) * resident_warps(ctx);
