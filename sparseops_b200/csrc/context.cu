@@ -239,9 +239,12 @@ void Context::pool_free(void* q) {
 }
 
 void GraphBlocks::free_dead() {
-  std::lock_guard<std::mutex> lock(mutex);
-  for (void* q : dead) cudaFree(q);
-  dead.clear();
+  std::vector<void*> gone;
+  {
+    std::lock_guard<std::mutex> lock(mutex);
+    gone.swap(dead);
+  }
+  for (void* q : gone) cudaFree(q);  // waits for the device: not under the callback's lock
 }
 
 namespace {
