@@ -163,10 +163,10 @@ __global__ void __launch_bounds__(kBatchBlock, KT == 1 ? 4 : 3) batch_kernel(con
 // turn, so the warps running together hold neighbouring rows and find the
 // X rows that a banded pattern shares in L1, while the window of matrices in
 // flight stays small enough for L2.  256 matrices, FP64: k = 32 6.03 ms with
-// items taken by single warps, 5.27 ms so, 4.43 ms with the entries staged, a
-// lane per column (csr_tile.cuh) and grabs of 4 items (8: 4.57, 16: 5.22 ms);
-// k = 16 3.06 -> 2.70 ms, k = 8 1.75 -> 1.72 ms.  Still bound by the latency of
-// the X gathers (nothing above half its rate).
+// items taken by single warps, 5.27 ms so, 4.5 ms with the entries staged, a
+// lane per column (csr_tile.cuh) and grabs of 4 items (8 and 16 items 3 and 18 %
+// more); k = 16 3.06 -> 2.70 ms, k = 8 1.75 -> 1.72 ms.  Bound by the X gathers:
+// at k = 32 L1 is at four fifths of its rate, at k = 8 and 16 their latency.
 constexpr int64_t kTilesPerItem = 4;
 template <int G>
 constexpr int kBlockItems = G == 8 ? 4 : 8;

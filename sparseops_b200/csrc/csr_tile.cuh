@@ -280,11 +280,12 @@ __device__ __forceinline__ void spmv_calibrate1(int64_t t, int64_t tiles, const 
 // one L2 request per 128 bytes.  Lanes past k load and store nothing.
 //
 // kStage: the tile's columns and values come through shared memory (SpmmTile),
-// copied there asynchronously a tile ahead.  What bounds the kernel is the
-// latency of dependent loads (column, then X row) at 16 warps per SM, with no
+// copied there asynchronously a tile ahead.  Not staged, the kernel is bound by
+// the latency of dependent loads (column, then X row) at 16 warps per SM, with no
 // unit above half its rate; staged, a warp never waits for its entries before
 // it can ask for X rows, and the copies take no registers, which leaves room
-// for eight entries' X rows per lane, four arriving while four are summed.
+// for eight entries' X rows per lane, four arriving while four are summed.  L1 is
+// then busy for four fifths of the time (k = 12 and 32).
 // Below eight lanes per entry or so the staging's own instructions weigh more
 // than that: those forms load a lane's eight entries into registers.  Which
 // form serves which k was measured (spmm_tiles_k).

@@ -94,8 +94,7 @@ __global__ void chunk_len_kernel(const int* __restrict__ cmax, int64_t nchunks, 
   elems[c] = L * C;
 }
 
-// Copy every row's entries into its padded slots (one warp per stored row).
-// Column-major chunks of 32 rows: a block per chunk, each warp a strip of 32
+// Every row's entries into its padded slots.  Column-major chunks of 32 rows: a block per chunk, each warp a strip of 32
 // slots, lane l row l.  A slot's 32 columns and values are written as whole
 // lines, padding included (column -1, value 0), so the storage needs no fill
 // pass; a lane's reads walk its own row and hit L1 after the first entry of a
@@ -127,6 +126,8 @@ __global__ void __launch_bounds__(32 * kChunkFillWarps)
   }
 }
 
+// The other layouts and chunk heights: one warp per stored row, into storage that
+// was filled with padding before.
 template <typename I, typename V, bool kColMajor>
 __global__ void pad_fill_kernel(const I* __restrict__ rp, const I* __restrict__ ci, const V* __restrict__ v,
                                 const I* __restrict__ reorder, int64_t n, int64_t C,

@@ -246,8 +246,10 @@ __host__ __device__ constexpr int64_t top_bin_max(int bin) { return (int64_t)64 
 // barriers per row for more than 512 products), k = 16 on 131,072 rows of 8 to
 // 40 planted entries, fp64, int64: 128 < P <= 512 675 -> 500 us,
 // 512 < P <= 2048 1128 -> 600 us, the rest 193 -> 178 us, the whole call 2.29 ->
-// 1.48 ms, and 1.37 with the forms' launches overlapping.  Bound by the sort's and the gather's instructions, as
-// row_sort_kernel is; forms of 16 keys per lane because a warp's sort costs
+// 1.48 ms, and 1.37 with the forms' launches overlapping.  Bound by the sort's and
+// the gather's instructions, as row_sort_kernel is: 60 % of the issue slots used,
+// the largest stall (3.7 - 5.2 cycles an instruction) the wait for instructions of
+// the unrolled network.  Forms of 16 keys per lane because a warp's sort costs
 // about the same per key up to there and needs no barrier.
 template <int R, int W>
 struct TopSmem {

@@ -636,7 +636,8 @@ spops_status_t spmm_tiles_t(Context* ctx, Matrix* A, double alpha, const void* X
 
 // Lanes per entry, columns per lane, vector parts and staging by k, each the
 // fastest measured on the 300,007-row power-law and a 1,000,000-row banded
-// matrix (us, FP64 | FP32; the segment kernel that served k other than 8, 16
+// matrix (us, FP64 | FP32, before the launches overlapped: k = 12 on the first
+// takes 102 now; the segment kernel that served k other than 8, 16
 // and 32 took 235 | 195, 443 | 364, 679 | 530, 1031 | 700 at k = 2, 12, 24, 31
 // on the first):
 //   k = 2   2 x 1            56, 98     | 45, 83
