@@ -202,6 +202,10 @@ spops_status_t spops_coo_to_csr(spops_context_t ctx, spops_matrix_t coo, int32_t
  * array of csr's index type, a permutation of 0 .. rows-1; anything else is
  * refused with SPOPS_ERR_INVALID (the reference does not check). */
 spops_status_t spops_csr_reorder_rows(spops_context_t ctx, spops_matrix_t csr, const void* perm, spops_matrix_t* out);
+/* Waits for the context's stream (unless it is being captured), and for the
+ * device where an array's address was asked for (spops_matrix_array); work on
+ * streams the context was on before is waited for before the arrays are used
+ * again.  Allowed beside captures on other streams, in any capture mode. */
 spops_status_t spops_matrix_destroy(spops_matrix_t A);
 spops_status_t spops_matrix_info(spops_matrix_t A, spops_matrix_info_t* info);
 /* Values changed in place (same pattern): drop value-derived caches. */
