@@ -94,12 +94,13 @@ __global__ void chunk_len_kernel(const int* __restrict__ cmax, int64_t nchunks, 
   elems[c] = L * C;
 }
 
-// Every row's entries into its padded slots.  Column-major chunks of 32 rows: a block per chunk, each warp a strip of 32
-// slots, lane l row l.  A slot's 32 columns and values are written as whole
-// lines, padding included (column -1, value 0), so the storage needs no fill
-// pass; a lane's reads walk its own row and hit L1 after the first entry of a
-// line.  One warp per row wrote single entries 128 and 256 bytes apart: 137 us
-// and 27 us of fills for 6.4M entries, against 44 us.
+// Every row's entries into its padded slots.  Column-major chunks of 32 rows: a
+// block per chunk, each warp a strip of 32 slots, lane l row l.  A slot's 32
+// columns and values are written as whole lines, padding included (column -1,
+// value 0), so the storage needs no fill pass; a lane's reads walk its own row and
+// hit L1 after the first entry of a line.  One warp per row wrote single entries
+// 128 and 256 bytes apart: 137 us and 27 us of fills for 6.4M entries, against
+// 44 us.
 constexpr int kChunkFillWarps = 4;
 
 template <typename I, typename V>

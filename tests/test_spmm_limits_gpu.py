@@ -125,3 +125,33 @@ def test_spmm_without_room_for_its_scratch(cuda, orc):
         out.append(Y)
     err = ((out[1] - out[0]).abs() / out[0].abs()).max()
     assert float(err) <= 1e-13  # sums of 128 positive terms in two orders
+
+
+def test_scratch_stays_while_its_graph_does(cuda):
+    """The scratch of graphs that are kept stays allocated (their instances hold
+    it, the captured graphs themselves are gone), and is given back after them."""
+    import torch
+    from sparseops_b200 import SpMM_csr
+    A, _ = _matrix(300000)
+    n, k = A.num_rows, 31
+    X = torch.rand(n, k, dtype=torch.float64, device="cuda")
+    Y = torch.zeros(n, k, dtype=torch.float64, device="cuda")
+    SpMM_csr(1.0, A, X, 0.0, Y)
+    s = torch.cuda.Stream()
+    graphs, free = [], []
+
+    def capture():
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            SpMM_csr(1.0, A, X, 0.0, Y)
+        torch.cuda.synchronize()
+        return g
+
+    for _ in range(10):  # 14 MB each
+        graphs.append(capture())
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[1] - free[-1] > 8 * (12 << 20)
+    graphs.clear()
+    torch.cuda.synchronize()
+    capture()  # a later capture frees what the graphs left
+    assert torch.cuda.mem_get_info()[0] - free[-1] > 8 * (12 << 20)
